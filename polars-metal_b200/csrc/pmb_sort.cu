@@ -12,7 +12,7 @@
 //   2. k_sort_encode — filter (the query's predicate), packed key + row index, compacted; and the
 //                      digit histograms of every pass, in the same read;
 //   3. k_sort_pass   — one stable 8-bit LSD pass per digit that is not constant (onesweep style:
-//                      warp-level ranking with __match_any_sync, per-digit decoupled look-back
+//                      warp-level ranking through shared lane masks, per-digit decoupled look-back
 //                      for the tile's global offsets, the tile reordered in shared memory so that
 //                      the writes are coalesced);
 //   4. k_seg_starts  — segment starts (key differs from its predecessor) compacted in order;
@@ -35,8 +35,8 @@
 namespace {
 
 constexpr int ST_NT = 256;              // threads of the sort kernels
-constexpr int ST_PER = 16;              // keys per thread in a pass tile
-constexpr int ST_TILE = ST_NT * ST_PER;  // 4096 keys per tile
+constexpr int ST_PER = 16;              // rows per thread in an encode or segment tile
+constexpr int ST_TILE = ST_NT * ST_PER;  // 4096 rows per tile
 constexpr int RADIX = 256;
 constexpr int MAX_PASSES = 16;
 constexpr int BIG = 256;                // rows above which a group is reduced by a whole CTA
@@ -262,136 +262,190 @@ struct PassParams {
   uint64_t cap;  // word stride of the key arrays
   int64_t n;
   int shift;
-  const unsigned int* hist;      // this pass's 256 digit counts
-  unsigned long long* lb;        // n_tiles x 256 look-back states (digit-major), zeroed
-  int64_t n_tiles;
+  const unsigned int* gstart;    // exclusive prefix sums of this pass's 256 digit counts
+  unsigned long long* lb;        // n_tiles x 256 look-back states (tile-major), zeroed
   unsigned long long* ticket;
   unsigned int* status;
   int hashed;  // digits of the key hash (partitioned strategy)
 };
 
-// One stable LSD pass over 8 bits at `shift`. Look-back states are tile-major (tile * 256 + digit),
-// so the 32 digits of a warp read one predecessor's states in one coalesced access. Per-warp digit
-// counts are 16-bit (at most 512 keys per warp), which with 4 CTAs per SM keeps the shared memory
-// of a CTA under a quarter of the SM's.
+// digit counts of every pass -> first output position of every digit (a CTA per pass)
+__global__ void __launch_bounds__(RADIX) k_digit_starts(const unsigned int* __restrict__ hist,
+                                                        unsigned int* __restrict__ gstart) {
+  __shared__ unsigned int s_scan[RADIX / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned c = hist[blockIdx.x * RADIX + tid];
+  unsigned x = c;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) s_scan[warp] = x;
+  __syncthreads();
+  for (int w = 0; w < warp; w++) x += s_scan[w];
+  gstart[blockIdx.x * RADIX + tid] = x - c;
+}
+
+// Tile shape of a pass, for W-word keys: three (two) CTAs of 12 (16) warps fit an SM's shared memory
 template <int W>
-__global__ void __launch_bounds__(ST_NT, 4) k_sort_pass(const __grid_constant__ PassParams P) {
+struct PassShape {
+  static constexpr int NT = W == 1 ? 384 : 512;
+  static constexpr int PER = W == 1 ? 10 : 6;
+  static constexpr int CTAS = W == 1 ? 3 : 2;
+  static constexpr int TILE = NT * PER, NW = NT / 32;
+  static constexpr size_t SMEM = (size_t)TILE * (8 * W + 4) + (size_t)NW * RADIX * 8;
+};
+
+// exclusive prefix of one digit over the earlier tiles: LB_W predecessor states are read per step
+// (independent loads, one L2 round trip), summed up to the nearest inclusive prefix
+constexpr int LB_W = 4;
+__device__ __forceinline__ unsigned long long digit_lookback(unsigned long long* lb, long long tile, unsigned count,
+                                                             unsigned int* st) {
+  const unsigned long long VAL = (1ULL << 62) - 1;
+  if (tile == 0) return 0;
+  unsigned long long excl = 0;
+  long long t = tile - 1;
+  uint32_t spins = 0;
+  for (;;) {
+    unsigned long long s[LB_W];
+#pragma unroll
+    for (int k = 0; k < LB_W; k++)
+      s[k] = t - k >= 0 ? *((volatile unsigned long long*)&lb[(t - k) * RADIX]) : (2ULL << 62);
+    bool done = false, miss = false;
+    int used = 0;
+#pragma unroll
+    for (int k = 0; k < LB_W; k++) {
+      if (done || miss) continue;
+      const unsigned f = (unsigned)(s[k] >> 62);
+      if (f == 0u) {
+        miss = true;
+      } else {
+        excl += s[k] & VAL;
+        used++;
+        done = f == 2u;
+      }
+    }
+    if (done) break;
+    t -= used;
+    if (miss && ++spins > PMB_SPIN_LIMIT) {
+      atomicOr(st, PMB_ST_TIMEOUT);
+      return 0;
+    }
+  }
+  *((volatile unsigned long long*)&lb[tile * RADIX]) = (2ULL << 62) | (excl + count);
+  return excl;
+}
+
+// One stable LSD pass over 8 bits at `shift` (onesweep: one read and one write of the pairs).
+// Every warp counts its keys' digits with shared atomics as soon as they are loaded, so the tile's
+// counts are published to the later tiles' look-backs before any ranking, and the counters, once
+// scanned, are the keys' running positions in the tile: a key goes straight to its place in shared
+// memory. The lanes of a round with the same digit find each other through a per-warp table of
+// lane masks (one atomicOr): __match_any_sync and eight ballots per key both cost more issue slots.
+// What bounds it: shared-memory atomics and accesses (about 50 cycles per 32 keys and SM; without
+// any output or look-back the ranking alone takes 60% of the time), not DRAM. 100M 64-bit keys:
+// 795 us (3.0 TB/s of the 6.4 a plain copy reaches); 256 threads x 16 keys with match_any, ranks
+// held to the end and a look-back of one state per step took 1020 us. 128-bit keys, 20M: 259 us,
+// against 552 us. Prefetching the next tile with bulk copies (persistent CTAs) took 900-960 us.
+template <int W>
+__global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
+    k_sort_pass(const __grid_constant__ PassParams P) {
+  constexpr int NT = PassShape<W>::NT, PER = PassShape<W>::PER, TILE = PassShape<W>::TILE, NW = PassShape<W>::NW;
   extern __shared__ __align__(16) unsigned char smem[];
-  unsigned long long* s_key = reinterpret_cast<unsigned long long*>(smem);       // W x ST_TILE
-  unsigned int* s_idx = reinterpret_cast<unsigned int*>(s_key + W * ST_TILE);   // ST_TILE
-  __shared__ unsigned short s_whist[ST_NT / 32][RADIX];
-  __shared__ unsigned int s_excl[RADIX];      // tile-local exclusive offset of each digit
-  __shared__ unsigned long long s_gbase[RADIX];
-  __shared__ unsigned int s_scan[ST_NT / 32];
+  unsigned long long* s_key = reinterpret_cast<unsigned long long*>(smem);    // W x TILE
+  unsigned int* s_idx = reinterpret_cast<unsigned int*>(s_key + W * TILE);   // TILE
+  unsigned int(*s_off)[RADIX] = reinterpret_cast<unsigned int(*)[RADIX]>(s_idx + TILE);  // NW
+  unsigned int(*s_lanes)[RADIX] = s_off + NW;                                            // NW
+  __shared__ long long s_out[RADIX];  // output position of a digit's first key, less its tile position
+  __shared__ unsigned int s_scan[RADIX / 32];
   __shared__ long long s_tile;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_tile = (long long)atomicAdd(P.ticket, 1ULL);
-  for (int i = tid; i < (ST_NT / 32) * RADIX; i += ST_NT) (&s_whist[0][0])[i] = 0;
+  for (int i = tid; i < 2 * NW * RADIX; i += NT) (&s_off[0][0])[i] = 0u;
   __syncthreads();
   const long long tile = s_tile;
-  const int64_t base = tile * ST_TILE;
+  // warp-striped items: item j of lane l of warp w is tile element w * PER * 32 + j * 32 + l
+  const int64_t e0 = (int64_t)tile * TILE + warp * (PER * 32) + lane;
   const unsigned lt = (1u << lane) - 1u;
-  // warp-striped items: warp w owns tile elements [w*512, w*512+512), item j of lane l is
-  // w*512 + j*32 + l. Only the digit and the rank stay in registers; the keys are read again (from
-  // L2) when the tile is reordered in shared memory.
-  unsigned int rank[ST_PER];
-  unsigned short dg[ST_PER];
+  PKey<W> k[PER];
+  unsigned ix[PER];
 #pragma unroll
-  for (int j = 0; j < ST_PER; j++) {
-    const int64_t e = base + warp * (ST_PER * 32) + j * 32 + lane;
-    PKey<W> k;
-    for (int i = 0; i < W; i++) k.w[i] = e < P.n ? P.kin[(uint64_t)i * P.cap + e] : 0ULL;
-    dg[j] = e < P.n ? (unsigned short)pass_digit<W>(k, P.shift, P.hashed) : (unsigned short)RADIX;
-  }
-  // ranks within the warp, in item order (stable): lanes with the same digit in one round are
-  // ordered by lane; earlier rounds come first
+  for (int j = 0; j < PER; j++)
 #pragma unroll
-  for (int j = 0; j < ST_PER; j++) {
-    const unsigned d = dg[j];
-    const unsigned peers = __match_any_sync(0xffffffffu, d);
-    const int leader = __ffs(peers) - 1;
-    unsigned old = 0;
-    if (d < RADIX && lane == leader) {
-      old = s_whist[warp][d];
-      s_whist[warp][d] = (unsigned short)(old + __popc(peers));
-    }
-    old = __shfl_sync(0xffffffffu, old, leader);
-    rank[j] = old + __popc(peers & lt);
-    __syncwarp();
-  }
+    for (int w = 0; w < W; w++) k[j].w[w] = e0 + j * 32 < P.n ? __ldcs(&P.kin[(uint64_t)w * P.cap + e0 + j * 32]) : 0ULL;
+#pragma unroll
+  for (int j = 0; j < PER; j++) ix[j] = e0 + j * 32 < P.n ? __ldcs(&P.iin[e0 + j * 32]) : 0u;
+#pragma unroll
+  for (int j = 0; j < PER; j++)
+    if (e0 + j * 32 < P.n) atomicAdd(&s_off[warp][pass_digit<W>(k[j], P.shift, P.hashed)], 1u);
   __syncthreads();
-  // per digit (thread d): warps' exclusive offsets and the tile's count
-  {
-    const int d = tid;
-    unsigned acc = 0;
-    for (int w = 0; w < ST_NT / 32; w++) {
-      unsigned c = s_whist[w][d];
-      s_whist[w][d] = (unsigned short)acc;
-      acc += c;
+  // thread d: the tile's count of digit d, published at once; then the tile-local exclusive scan
+  // over the digits, and every warp's first position of the digit
+  unsigned acc = 0, x = 0;
+  if (tid < RADIX) {
+    unsigned c[NW];
+#pragma unroll
+    for (int w = 0; w < NW; w++) c[w] = s_off[w][tid];
+#pragma unroll
+    for (int w = 0; w < NW; w++) {
+      const unsigned t = c[w];
+      c[w] = acc;
+      acc += t;
     }
-    // tile-local exclusive scan over digits (block scan of one value per thread)
-    unsigned x = acc;
+    *((volatile unsigned long long*)&P.lb[tile * RADIX + tid]) = ((tile == 0 ? 2ULL : 1ULL) << 62) | acc;
+    x = acc;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) s_scan[warp] = x;
-    __syncthreads();
-    if (tid == 0) {
-      unsigned a = 0;
-      for (int w = 0; w < ST_NT / 32; w++) {
-        unsigned c = s_scan[w];
-        s_scan[w] = a;
-        a += c;
-      }
-    }
-    __syncthreads();
-    const unsigned excl = x - acc + s_scan[warp];
-    s_excl[d] = excl;
-    // global start of this digit: the counts of the digits before it over the whole input
-    // (exclusive scan of this pass's histogram), then the earlier tiles (look-back)
-    const unsigned hd = P.hist[d];
-    unsigned y = hd;
-    for (int o = 1; o < 32; o <<= 1) {
-      unsigned z = __shfl_up_sync(0xffffffffu, y, o);
-      if (lane >= o) y += z;
-    }
-    __syncthreads();
-    if (lane == 31) s_scan[warp] = y;
-    __syncthreads();
-    if (tid == 0) {
-      unsigned a = 0;
-      for (int w = 0; w < ST_NT / 32; w++) {
-        unsigned c = s_scan[w];
-        s_scan[w] = a;
-        a += c;
-      }
-    }
-    __syncthreads();
-    const unsigned long long gstart = (unsigned long long)(y - hd + s_scan[warp]);
-    const unsigned long long pre = pmb_lookback_strided(P.lb + d, tile, RADIX, acc, P.status);
-    s_gbase[d] = gstart + pre;
-  }
-  __syncthreads();
-  // reorder the tile in shared memory by digit
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // the RADIX threads of this scan
 #pragma unroll
-  for (int j = 0; j < ST_PER; j++) {
-    const unsigned d = dg[j];
-    if (d < RADIX) {
-      const int64_t e = base + warp * (ST_PER * 32) + j * 32 + lane;
-      const unsigned lp = s_excl[d] + s_whist[warp][d] + rank[j];
-      for (int i = 0; i < W; i++) s_key[i * ST_TILE + lp] = P.kin[(uint64_t)i * P.cap + e];
-      s_idx[lp] = P.iin[e];
-    }
+    for (int w = 0; w < RADIX / 32; w++) x += w < warp ? s_scan[w] : 0u;
+    x -= acc;
+#pragma unroll
+    for (int w = 0; w < NW; w++) s_off[w][tid] = c[w] + x;
   }
   __syncthreads();
-  const int valid = (int)min((int64_t)ST_TILE, P.n - base);
-  for (int i = tid; i < valid; i += ST_NT) {
-    PKey<W> k;
-    for (int w = 0; w < W; w++) k.w[w] = s_key[w * ST_TILE + i];
-    const unsigned d = pass_digit<W>(k, P.shift, P.hashed);
-    const uint64_t g = s_gbase[d] + (uint64_t)(i - (int)s_excl[d]);
-    for (int w = 0; w < W; w++) P.kout[(uint64_t)w * P.cap + g] = k.w[w];
+  // the tile reordered by digit in shared memory, in item order (stable): the lanes of a round with
+  // the same digit are ordered by lane, earlier rounds and warps come first
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    const bool in = e0 + j * 32 < P.n;
+    const unsigned d = pass_digit<W>(k[j], P.shift, P.hashed);
+    if (in) atomicOr(&s_lanes[warp][d], 1u << lane);
+    __syncwarp();
+    const unsigned peers = s_lanes[warp][d], first = s_off[warp][d], below = __popc(peers & lt);
+    __syncwarp();
+    if (in) {
+      if (below == 0u) {
+        s_off[warp][d] = first + __popc(peers);
+        s_lanes[warp][d] = 0u;
+      }
+      const unsigned lp = first + below;
+#pragma unroll
+      for (int w = 0; w < W; w++) s_key[w * TILE + lp] = k[j].w[w];
+      s_idx[lp] = ix[j];
+    }
+    __syncwarp();
+  }
+  if (tid < RADIX) {
+    const unsigned long long pre = digit_lookback(P.lb + tid, tile, acc, P.status);
+    s_out[tid] = (long long)P.gstart[tid] + (long long)pre - (long long)x;
+  }
+  __syncthreads();
+  const int valid = (int)min((long long)TILE, (long long)P.n - tile * TILE);
+#pragma unroll
+  for (int j = 0; j < PER; j++) {
+    const int i = tid + j * NT;
+    if (i >= valid) continue;
+    PKey<W> kk;
+#pragma unroll
+    for (int w = 0; w < W; w++) kk.w[w] = s_key[w * TILE + i];
+    const uint64_t g = (uint64_t)(s_out[pass_digit<W>(kk, P.shift, P.hashed)] + i);
+#pragma unroll
+    for (int w = 0; w < W; w++) P.kout[(uint64_t)w * P.cap + g] = kk.w[w];
     P.iout[g] = s_idx[i];
   }
 }
@@ -1160,8 +1214,11 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   unsigned long long* ctr = (unsigned long long*)pmb_ws_alloc(h, 64);  // kept, ticket, n_groups, big_n
   unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
   const int64_t max_tiles = (n + ST_TILE - 1) / ST_TILE;
-  unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(h, (size_t)std::max<int64_t>(max_tiles, 1) * RADIX * 8);
-  if (!k0 || !k1 || !i0 || !i1 || !hist || !ctr || !status || !lb)
+  const int64_t max_ptiles = (n + PassShape<W>::TILE - 1) / PassShape<W>::TILE;  // pass tiles
+  unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(
+      h, (size_t)std::max<int64_t>({max_tiles, max_ptiles * RADIX, 1}) * 8);
+  unsigned int* gstart = (unsigned int*)pmb_ws_alloc(h, (size_t)MAX_PASSES * RADIX * 4);
+  if (!k0 || !k1 || !i0 || !i1 || !hist || !ctr || !status || !lb || !gstart)
     return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort buffers)");
   PMB_CUDA(h, cudaMemsetAsync(hist, 0, (size_t)MAX_PASSES * RADIX * 4, h->stream));
   PMB_CUDA(h, cudaMemsetAsync(ctr, 0, 64, h->stream));
@@ -1204,8 +1261,15 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   const int64_t m = (int64_t)kept;
   // LSD passes over the digits that are not the same for every key
   const int64_t tiles = (m + ST_TILE - 1) / ST_TILE;
-  const size_t pass_smem = (size_t)ST_TILE * (8 * W + 4);
+  const int64_t ptiles = (m + PassShape<W>::TILE - 1) / PassShape<W>::TILE;
+  constexpr size_t pass_smem = PassShape<W>::SMEM;
   PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
+  if (passes > 0 && m > 1) {
+    pmb_kernel_begin(h, "digit_starts");
+    k_digit_starts<<<passes, RADIX, 0, h->stream>>>(hist, gstart);
+    pmb_kernel_end(h);
+    PMB_CUDA(h, cudaGetLastError());
+  }
   int done = 0;
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
@@ -1220,15 +1284,14 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     P.n = m;
     P.shift = (part_groups > 0 ? 64 - pb : 0) + 8 * p;
     P.hashed = part_groups > 0;
-    P.hist = hist + (size_t)p * RADIX;
+    P.gstart = gstart + (size_t)p * RADIX;
     P.lb = lb;
-    P.n_tiles = tiles;
     P.ticket = ctr + 1;
     P.status = status;
-    PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)tiles * RADIX * 8, h->stream));
+    PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)ptiles * RADIX * 8, h->stream));
     PMB_CUDA(h, cudaMemsetAsync(ctr + 1, 0, 8, h->stream));
     pmb_kernel_begin(h, "sort_pass");
-    k_sort_pass<W><<<(unsigned)tiles, ST_NT, pass_smem, h->stream>>>(P);
+    k_sort_pass<W><<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     std::swap(k0, k1);
@@ -1426,15 +1489,22 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
   if (W != 1 && W != 2) return pmb_fail(h, PMB_E_INVALID, "sort: key of 1 or 2 words");
   if (n_passes > MAX_PASSES) return pmb_fail(h, PMB_E_INVALID, "sort: more than 16 digit passes");
   if (n <= 1 || n_passes <= 0) return PMB_OK;
-  const int64_t tiles = (n + ST_TILE - 1) / ST_TILE;
+  const int tile = W == 1 ? PassShape<1>::TILE : PassShape<2>::TILE;
+  const int64_t tiles = (n + tile - 1) / tile;
   unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(h, (size_t)tiles * RADIX * 8);
   unsigned long long* ticket = (unsigned long long*)pmb_ws_alloc(h, 64);
   unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
-  if (!lb || !ticket || !status) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
+  unsigned int* gstart = (unsigned int*)pmb_ws_alloc(h, (size_t)n_passes * RADIX * 4);
+  if (!lb || !ticket || !status || !gstart) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
   PMB_CUDA(h, cudaMemsetAsync(status, 0, 64, h->stream));
-  const size_t pass_smem = (size_t)ST_TILE * (8 * W + 4);
-  if (W == 1) PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
-  else PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
+  if (W == 1)
+    PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
+  else
+    PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<2>::SMEM));
+  pmb_kernel_begin(h, "digit_starts");
+  k_digit_starts<<<n_passes, RADIX, 0, h->stream>>>(hist_dev, gstart);
+  pmb_kernel_end(h);
+  PMB_CUDA(h, cudaGetLastError());
   for (int p = 0; p < n_passes; p++) {
     bool constant = false;
     for (int d = 0; d < RADIX; d++) constant |= hist_host[(size_t)p * RADIX + d] == (unsigned)n;
@@ -1448,16 +1518,15 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
     P.n = n;
     P.shift = 8 * p;
     P.hashed = 0;
-    P.hist = hist_dev + (size_t)p * RADIX;
+    P.gstart = gstart + (size_t)p * RADIX;
     P.lb = lb;
-    P.n_tiles = tiles;
     P.ticket = ticket;
     P.status = status;
     PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)tiles * RADIX * 8, h->stream));
     PMB_CUDA(h, cudaMemsetAsync(ticket, 0, 8, h->stream));
     pmb_kernel_begin(h, "sort_pass");
-    if (W == 1) k_sort_pass<1><<<(unsigned)tiles, ST_NT, pass_smem, h->stream>>>(P);
-    else k_sort_pass<2><<<(unsigned)tiles, ST_NT, pass_smem, h->stream>>>(P);
+    if (W == 1) k_sort_pass<1><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
+    else k_sort_pass<2><<<(unsigned)tiles, PassShape<2>::NT, PassShape<2>::SMEM, h->stream>>>(P);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     std::swap(*k, *k_alt);

@@ -1,0 +1,35 @@
+"""GPU parity at the sizes where a kernel's tiling can go wrong: tile edges, remainders, the smallest
+and largest sizes of a dispatch range. Integer results and orders are compared bit for bit with the
+oracle's; float sums as in tests/helpers.py."""
+
+import numpy as np
+import pytest
+
+from helpers import as_dict, pack
+from oracle import pyoracle
+from polars_b200 import _native as N
+from test_gpu_sort import assert_same_rows
+
+pytestmark = pytest.mark.gpu
+
+
+def _sorted_both(cols: dict, by, descending, nulls_last=False, **kw):
+    """(product, oracle) of the sort of columns given as name -> (values, bitmap or None)."""
+    got = N.sort_columns({k: N.ColumnData(d, v) for k, (d, v) in cols.items()}, by, descending, nulls_last, **kw)
+    nl = [nulls_last] * len(by)
+    want = pyoracle.sort_table(cols, by, descending, nl, kw.get("drop_nulls", False), kw.get("offset", 0),
+                               -1 if kw.get("limit") is None else kw["limit"])
+    return as_dict(got), want
+
+
+# the radix passes: tiles of 3840 keys of one word and of 3072 keys of two words; skewed digits (many
+# lanes of a warp share one) and constant ones (a skipped pass)
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("n", [11519, 11520, 11521, 12287, 12288, 12289, 46080])
+def test_radix_pass_tiles(n, wide):
+    rng = np.random.default_rng(n)
+    cols = {"a": (rng.integers(0, 3, n) * (1 << 33) + rng.integers(0, 700, n), pack(rng.random(n) > 0.1)),
+            "b": (rng.integers(-2**62, 2**62, n), None), "row": (np.arange(n, dtype=np.int32), None)}
+    by = ["a", "b"] if wide else ["a"]
+    got, want = _sorted_both(cols, by, [True, False][: len(by)])
+    assert_same_rows(got, want, f"{n} rows")
