@@ -8,7 +8,8 @@
 // (groupby.rs:2599-2833, src/aggregate_fused/emitter.rs:189-393).
 //
 // Design (one pass over the input, no row_to_group materialisation):
-//   k_sketch     — 65,536 sampled rows -> distinct / singleton counts -> group estimate
+//   k_sketch     — 65,536 sampled rows -> distinct / singleton counts -> group estimate; the
+//                  selector's features and network in the same launch
 //   k_table_init — global open-addressing table: keys = EMPTY, records = identity
 //   k_hash_agg   — persistent CTAs; each column tile arrives in shared memory by 1-D TMA bulk
 //                  copies (cp.async.bulk + mbarrier, multi-stage ring); per row: predicate in
@@ -31,31 +32,84 @@
 
 #include "pmb_groupby.h"
 #include "pmb_jit.h"
+#include "pmb_selector.cuh"
 
 // ============================================================================ sketch
 #define SK_SAMPLES 65536
-#define SK_SLOTS (1 << 18)
+#define SK_MIN_SLOTS 4096
 
 struct FxCols {
   int n;
   int col[PMB_MAX_FX];
 };
 
+// The sampling stage of a call, three launches and one read-back:
+//   k_front_init  clears the sample set and its counters; with the selector, CTAs of the same
+//                 launch also evaluate its 4096 sampled rows
+//   k_sketch      inserts 65,536 sampled rows into the sample set; with the selector, CTA 0 counts
+//                 the 4096 rows into features and runs the network meanwhile
+//   k_sketch_reduce  counts the sample set
+// Nothing here is bound by bandwidth: each launch is a few dependent round trips. As three memsets,
+// five kernels and two copies one after another the stage took 100-130 us of every call.
+struct FrontParams {
+  DQuery q;
+  int64_t m;                       // sampled rows of the sketch
+  unsigned long long* set_keys;    // `slots` keys and counts
+  unsigned int* set_cnt;
+  int slots;                       // power of two, at least 4 per sampled row
+  unsigned int* zero;              // words cleared by k_front_init (counters, histogram)
+  int zero_words;
+  FxCols fxc;
+  unsigned int* fx_expo;
+  // selector (params null: none)
+  const float* params;
+  unsigned long long* hs;          // SAMPLE key hashes and null flags
+  unsigned char* ns;
+  float* feat;                     // NF features, then NO outputs
+};
+
+constexpr int FR_NT = 256;
+__global__ void __launch_bounds__(FR_NT) k_front_init(const __grid_constant__ FrontParams F) {
+  const int i = blockIdx.x * FR_NT + threadIdx.x;
+  if (F.params && i < SAMPLE) sample_one(F.q, i, F.hs[i], F.ns[i]);
+  const int stride = gridDim.x * FR_NT;
+  ulonglong2* k = reinterpret_cast<ulonglong2*>(F.set_keys);
+  uint4* c = reinterpret_cast<uint4*>(F.set_cnt);
+  for (int s = i; s < F.slots / 2; s += stride) k[s] = make_ulonglong2(PMB_EMPTY64, PMB_EMPTY64);
+  for (int s = i; s < F.slots / 4; s += stride) c[s] = make_uint4(0u, 0u, 0u, 0u);
+  for (int s = i; s < F.zero_words; s += stride) F.zero[s] = 0u;
+}
+
 template <bool K128>
-__global__ void k_sketch(const __grid_constant__ DQuery q, int64_t m, unsigned long long* __restrict__ set_keys,
-                         unsigned int* __restrict__ set_cnt, const __grid_constant__ FxCols fxc,
-                         unsigned int* __restrict__ fx_expo) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(F_NT) k_sketch(const __grid_constant__ FrontParams F) {
+  extern __shared__ unsigned long long s_front[];  // TSLOTS words, then the network's weights
+  const DQuery& q = F.q;
+  if (F.params && blockIdx.x == 0) {
+    __shared__ float h1[NH], h2[NH];
+    float* w = reinterpret_cast<float*>(s_front + TSLOTS);
+    mlp_load(F.params, w);
+    features_body(q, F.hs, F.ns, F.feat, s_front);
+    __syncthreads();
+    mlp_run(w, F.feat, h1, h2, F.feat + NF);
+    return;
+  }
+  int64_t i = (int64_t)(blockIdx.x - (F.params ? 1 : 0)) * blockDim.x + threadIdx.x;
+  const int64_t m = F.m;
   if (i >= m) return;
   int64_t row = (m == q.n_rows) ? i : (int64_t)((double)i * (double)q.n_rows / (double)m);
   if (row >= q.n_rows) row = q.n_rows - 1;
   TileCtx t{nullptr, nullptr, nullptr, 0};
   // largest exponent of the finite values of each float-sum column (fixed-point range)
-  for (int f = 0; f < fxc.n; f++) {
-    int c = fxc.col[f];
-    if (!tc_isvalid(q, t, c, row)) continue;
-    double x = pmb_bits_to_f64(tc_bits(q, t, c, row), q.col[c].dtype);
-    if (!pmb_fx_flag(x)) atomicMax(&fx_expo[f], (unsigned)pmb_fx_expo(x));
+  for (int f = 0; f < F.fxc.n; f++) {
+    int c = F.fxc.col[f];
+    unsigned ex = 0;
+    if (tc_isvalid(q, t, c, row)) {
+      double x = pmb_bits_to_f64(tc_bits(q, t, c, row), q.col[c].dtype);
+      if (!pmb_fx_flag(x)) ex = (unsigned)pmb_fx_expo(x);
+    }
+    const unsigned am = __activemask();
+    ex = __reduce_max_sync(am, ex);
+    if (ex && (threadIdx.x & 31) == __ffs(am) - 1) atomicMax(&F.fx_expo[f], ex);
   }
   uint64_t k;
   if (K128) {
@@ -65,63 +119,82 @@ __global__ void k_sketch(const __grid_constant__ DQuery q, int64_t m, unsigned l
     k = pack_key64(q, t, row);
   }
   if (k == PMB_EMPTY64) k = PMB_EMPTY64 - 1;
-  uint32_t s = (uint32_t)(pmb_fmix64(k) & (SK_SLOTS - 1));
-  for (int p = 0; p < SK_SLOTS; p++) {
-    unsigned long long cur = set_keys[s];
+  const uint32_t mask = (uint32_t)F.slots - 1u;
+  uint32_t s = (uint32_t)pmb_fmix64(k) & mask;
+  for (int p = 0; p < F.slots; p++) {
+    unsigned long long cur = F.set_keys[s];
     if (cur == k) break;
     if (cur == PMB_EMPTY64) {
-      unsigned long long old = atomicCAS(&set_keys[s], PMB_EMPTY64, k);
+      unsigned long long old = atomicCAS(&F.set_keys[s], PMB_EMPTY64, k);
       if (old == PMB_EMPTY64 || old == k) break;
     }
-    s = (s + 1) & (SK_SLOTS - 1);
+    s = (s + 1) & mask;
   }
-  atomicAdd(&set_cnt[s], 1u);
+  atomicAdd(&F.set_cnt[s], 1u);
 }
 
-// distinct count, singletons, doubletons and the histogram of per-key sample counts
-__global__ void k_sketch_reduce(const unsigned long long* __restrict__ set_keys,
-                                const unsigned int* __restrict__ set_cnt, unsigned long long* __restrict__ out,
+// distinct count, singletons, doubletons and the histogram of per-key sample counts (its first bins
+// are the singletons and doubletons, so only keys seen more often touch it)
+__global__ void __launch_bounds__(256) k_sketch_reduce(const unsigned long long* __restrict__ set_keys,
+                                const unsigned int* __restrict__ set_cnt, int slots, unsigned long long* __restrict__ out,
                                 unsigned int* __restrict__ hist) {
-  __shared__ unsigned long long acc[3];
-  __shared__ unsigned int sh[SK_HIST];
-  if (threadIdx.x < 3) acc[threadIdx.x] = 0;
-  for (int i = threadIdx.x; i < SK_HIST; i += blockDim.x) sh[i] = 0;
-  __syncthreads();
-  unsigned long long d = 0, f1 = 0, f2 = 0;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < SK_SLOTS; s += gridDim.x * blockDim.x) {
-    if (set_keys[s] != PMB_EMPTY64) {
+  unsigned d = 0, f1 = 0, f2 = 0;
+  const ulonglong2* keys = reinterpret_cast<const ulonglong2*>(set_keys);
+  const uint2* cnts = reinterpret_cast<const uint2*>(set_cnt);
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < slots / 2; s += gridDim.x * blockDim.x) {
+    const ulonglong2 k = keys[s];
+    const uint2 c = cnts[s];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const unsigned long long key = j ? k.y : k.x;
+      const unsigned n = j ? c.y : c.x;
+      if (key == PMB_EMPTY64) continue;
       d++;
-      unsigned int c = set_cnt[s];
-      f1 += c == 1;
-      f2 += c == 2;
-      atomicAdd(&sh[c < SK_HIST ? c : SK_HIST - 1], 1u);
+      f1 += n == 1;
+      f2 += n == 2;
+      if (n > 2) atomicAdd(&hist[n < SK_HIST ? n : SK_HIST - 1], 1u);
     }
   }
-  atomicAdd(&acc[0], d);
-  atomicAdd(&acc[1], f1);
-  atomicAdd(&acc[2], f2);
+  __shared__ unsigned s_acc[3];
+  if (threadIdx.x < 3) s_acc[threadIdx.x] = 0u;
   __syncthreads();
-  if (threadIdx.x < 3) atomicAdd(&out[threadIdx.x], acc[threadIdx.x]);
-  for (int i = threadIdx.x; i < SK_HIST; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  d = __reduce_add_sync(0xffffffffu, d);
+  f1 = __reduce_add_sync(0xffffffffu, f1);
+  f2 = __reduce_add_sync(0xffffffffu, f2);
+  if ((threadIdx.x & 31) == 0 && d) {
+    atomicAdd(&s_acc[0], d);
+    atomicAdd(&s_acc[1], f1);
+    atomicAdd(&s_acc[2], f2);
+  }
+  __syncthreads();
+  if (threadIdx.x < 3 && s_acc[threadIdx.x]) {
+    atomicAdd(&out[threadIdx.x], (unsigned long long)s_acc[threadIdx.x]);
+    if (threadIdx.x) atomicAdd(&hist[threadIdx.x], s_acc[threadIdx.x]);
+  }
 }
 
 // keys of the sample with count >= t1 -> hot list, t2 <= count < t1 -> warm list
-__global__ void k_sketch_select(const unsigned long long* __restrict__ set_keys, const unsigned int* __restrict__ set_cnt,
-                                unsigned int t1, unsigned int t2, unsigned long long* __restrict__ hot,
+__global__ void __launch_bounds__(256) k_sketch_select(const unsigned long long* __restrict__ set_keys, const unsigned int* __restrict__ set_cnt,
+                                int slots, unsigned int t1, unsigned int t2, unsigned long long* __restrict__ hot,
                                 unsigned int* __restrict__ hot_n, unsigned int hot_cap,
                                 unsigned long long* __restrict__ warm, unsigned int* __restrict__ warm_n,
                                 unsigned int warm_cap) {
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < SK_SLOTS; s += gridDim.x * blockDim.x) {
-    unsigned long long k = set_keys[s];
-    if (k == PMB_EMPTY64) continue;
-    unsigned int c = set_cnt[s];
-    if (c >= t1) {
-      unsigned int i = atomicAdd(hot_n, 1u);
-      if (i < hot_cap) hot[i] = k;
-    } else if (c >= t2) {
-      unsigned int i = atomicAdd(warm_n, 1u);
-      if (i < warm_cap) warm[i] = k;
+  // counts first: most slots are below both thresholds and their keys are not read
+  const uint4* cnts = reinterpret_cast<const uint4*>(set_cnt);
+  for (int s4 = blockIdx.x * blockDim.x + threadIdx.x; s4 < slots / 4; s4 += gridDim.x * blockDim.x) {
+    const uint4 c4 = cnts[s4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const unsigned int c = j == 0 ? c4.x : j == 1 ? c4.y : j == 2 ? c4.z : c4.w;
+      if (c < t2 || c == 0u) continue;
+      const unsigned long long k = set_keys[4 * s4 + j];
+      if (c >= t1) {
+        unsigned int i = atomicAdd(hot_n, 1u);
+        if (i < hot_cap) hot[i] = k;
+      } else {
+        unsigned int i = atomicAdd(warm_n, 1u);
+        if (i < warm_cap) warm[i] = k;
+      }
     }
   }
 }
@@ -737,7 +810,7 @@ static int launch_finalize(pmb_handle* h, const FinParams& F, int64_t nslots) {
   return PMB_OK;
 }
 
-int pmb_groupby_sketch(pmb_handle* h, const CompiledQuery& cq, SketchOut* out) {
+int pmb_groupby_sketch(pmb_handle* h, const CompiledQuery& cq, SketchOut* out, bool select) {
   const DQuery& q = cq.dq;
   int64_t m = std::min<int64_t>(q.n_rows, SK_SAMPLES);
   out->samples = m;
@@ -746,41 +819,73 @@ int pmb_groupby_sketch(pmb_handle* h, const CompiledQuery& cq, SketchOut* out) {
   memset(out->fx_expo, 0, sizeof(out->fx_expo));
   out->set_keys = nullptr;
   out->set_cnt = nullptr;
+  out->set_slots = 0;
+  out->key_counts = nullptr;
   if (m == 0) return PMB_OK;
-  unsigned long long* keys = (unsigned long long*)pmb_ws_alloc(h, sizeof(unsigned long long) * SK_SLOTS);
-  unsigned int* cnt = (unsigned int*)pmb_ws_alloc(h, sizeof(unsigned int) * SK_SLOTS);
-  unsigned long long* res = (unsigned long long*)pmb_ws_alloc(h, 64 + 4 * SK_HIST);
-  if (!keys || !cnt || !res) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sketch)");
-  unsigned int* hist = (unsigned int*)(res + 8);
-  unsigned int* fx_expo = (unsigned int*)(res + 4);  // res[4..7]: 8 x u32
-  FxCols fxc;
-  memset(&fxc, 0, sizeof(fxc));
-  fxc.n = (int)cq.fx_cols.size();
-  for (int f = 0; f < fxc.n; f++) fxc.col[f] = cq.fx_cols[f];
-  PMB_CUDA(h, cudaMemsetAsync(keys, 0xFF, sizeof(unsigned long long) * SK_SLOTS, h->stream));
-  PMB_CUDA(h, cudaMemsetAsync(cnt, 0, sizeof(unsigned int) * SK_SLOTS, h->stream));
-  PMB_CUDA(h, cudaMemsetAsync(res, 0, 64 + 4 * SK_HIST, h->stream));
+  int slots = SK_MIN_SLOTS;
+  while (slots < 4 * m) slots *= 2;
+  // counters, one read-back: distinct, singletons, doubletons (3 x u64), key list counts (2 x u32),
+  // exponents (8 x u32), the selector's features and outputs, the histogram
+  constexpr size_t OFF_COUNTS = 24, OFF_EXPO = 32, OFF_FEAT = 64, OFF_HIST = 64 + 4 * 32;
+  constexpr size_t RES_BYTES = OFF_HIST + 4 * SK_HIST;
+  static_assert(NF + NO <= 32 && PMB_MAX_FX <= 8 && RES_BYTES <= PMB_SEL_PINNED_OFF, "sketch read-back");
+  unsigned long long* keys = (unsigned long long*)pmb_ws_alloc(h, sizeof(unsigned long long) * slots);
+  unsigned int* cnt = (unsigned int*)pmb_ws_alloc(h, sizeof(unsigned int) * slots);
+  uint8_t* res = (uint8_t*)pmb_ws_alloc(h, RES_BYTES);
+  unsigned long long* hs = select ? (unsigned long long*)pmb_ws_alloc(h, (size_t)SAMPLE * 9) : nullptr;
+  if (!keys || !cnt || !res || (select && !hs)) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sketch)");
+  unsigned int* hist = (unsigned int*)(res + OFF_HIST);
+  FrontParams F;
+  memset(&F, 0, sizeof(F));
+  F.q = q;
+  F.m = m;
+  F.set_keys = keys;
+  F.set_cnt = cnt;
+  F.slots = slots;
+  F.zero = (unsigned int*)res;
+  F.zero_words = (int)(RES_BYTES / 4);
+  F.fxc.n = (int)cq.fx_cols.size();
+  for (int f = 0; f < F.fxc.n; f++) F.fxc.col[f] = cq.fx_cols[f];
+  F.fx_expo = (unsigned int*)(res + OFF_EXPO);
+  if (select) {
+    F.params = h->selector;
+    F.hs = hs;
+    F.ns = reinterpret_cast<unsigned char*>(hs + SAMPLE);
+    F.feat = (float*)(res + OFF_FEAT);
+  }
+  pmb_kernel_begin(h, "front_init");
+  k_front_init<<<std::min(h->sm_count * 4, slots / 512 + SAMPLE / FR_NT), FR_NT, 0, h->stream>>>(F);
+  pmb_kernel_end(h);
+  PMB_CUDA(h, cudaGetLastError());
+  const int smem = select ? TSLOTS * 8 + MLP_WORDS * 4 : 0;
+  const unsigned blocks = (unsigned)((m + F_NT - 1) / F_NT) + (select ? 1u : 0u);
   pmb_kernel_begin(h, "sketch");
-  if (q.key_bits > 64)
-    k_sketch<true><<<(unsigned)((m + 255) / 256), 256, 0, h->stream>>>(q, m, keys, cnt, fxc, fx_expo);
-  else
-    k_sketch<false><<<(unsigned)((m + 255) / 256), 256, 0, h->stream>>>(q, m, keys, cnt, fxc, fx_expo);
+  if (q.key_bits > 64) {
+    PMB_CUDA(h, cudaFuncSetAttribute(k_sketch<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_sketch<true><<<blocks, F_NT, smem, h->stream>>>(F);
+  } else {
+    PMB_CUDA(h, cudaFuncSetAttribute(k_sketch<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_sketch<false><<<blocks, F_NT, smem, h->stream>>>(F);
+  }
   pmb_kernel_end(h);
   PMB_CUDA(h, cudaGetLastError());
   pmb_kernel_begin(h, "sketch_reduce");
-  k_sketch_reduce<<<64, 256, 0, h->stream>>>(keys, cnt, res, hist);
+  k_sketch_reduce<<<std::min(h->sm_count, slots / 512), 256, 0, h->stream>>>(keys, cnt, slots, (unsigned long long*)res, hist);
   pmb_kernel_end(h);
   PMB_CUDA(h, cudaGetLastError());
-  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, res, 64 + 4 * SK_HIST, cudaMemcpyDeviceToHost, h->stream));
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, res, RES_BYTES, cudaMemcpyDeviceToHost, h->stream));
   PMB_CUDA(h, cudaStreamSynchronize(h->stream));
   const unsigned long long* r = (const unsigned long long*)h->pinned;
   out->distinct = (int64_t)r[0];
   out->singletons = (int64_t)r[1];
   out->doubletons = (int64_t)r[2];
-  memcpy(out->fx_expo, h->pinned + 32, 4 * PMB_MAX_FX);
-  memcpy(out->hist, h->pinned + 64, 4 * SK_HIST);
+  memcpy(out->fx_expo, h->pinned + OFF_EXPO, 4 * PMB_MAX_FX);
+  memcpy(out->hist, h->pinned + OFF_HIST, 4 * SK_HIST);
+  if (select) memcpy(h->pinned + PMB_SEL_PINNED_OFF, h->pinned + OFF_FEAT + 4 * NF, 4 * NO);
   out->set_keys = keys;
   out->set_cnt = cnt;
+  out->set_slots = slots;
+  out->key_counts = (unsigned int*)(res + OFF_COUNTS);
   return PMB_OK;
 }
 
@@ -927,11 +1032,11 @@ int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int 
         }
       unsigned long long* lists = (unsigned long long*)pmb_ws_alloc(h, 8 * ((size_t)hot_cap + warm_cap) + 64);
       if (!lists) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (hot keys)");
-      unsigned int* counts = (unsigned int*)(lists + hot_cap + warm_cap);
-      PMB_CUDA(h, cudaMemsetAsync(counts, 0, 16, h->stream));
+      unsigned int* counts = sk->key_counts;
       pmb_kernel_begin(h, "sketch_select");
-      k_sketch_select<<<64, 256, 0, h->stream>>>(sk->set_keys, sk->set_cnt, t1, t2, lists, counts, (unsigned)hot_cap,
-                                                 lists + hot_cap, counts + 1, warm_cap);
+      k_sketch_select<<<std::min(h->sm_count, sk->set_slots / 1024), 256, 0, h->stream>>>(
+          sk->set_keys, sk->set_cnt, sk->set_slots, t1, t2, lists, counts, (unsigned)hot_cap, lists + hot_cap, counts + 1,
+          warm_cap);
       pmb_kernel_end(h);
       PMB_CUDA(h, cudaGetLastError());
       P.hot_keys = hot_cap ? lists : nullptr;
@@ -1170,9 +1275,8 @@ extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* 
     bool est_learned = false;
     static thread_local SketchOut sk;  // large (histogram); one per host thread
     bool have_sk = true;
-    // the selector's kernels go in before the sketch's readback, whose synchronisation serves both
-    const bool sel = strategy == PMB_STRATEGY_AUTO && pmb_selector_launch(h, cq);
-    rc = pmb_groupby_sketch(h, cq, &sk);
+    const bool sel = strategy == PMB_STRATEGY_AUTO && h->selector;
+    rc = pmb_groupby_sketch(h, cq, &sk, sel);
     if (rc) return bail(rc);
     pmb_phase(h, "sketch");
     // fixed-point range of the float sums: sample maximum with 8x headroom; partial sums of a

@@ -71,9 +71,13 @@ struct SketchOut {
   // device-resident sample set (valid until the next workspace reset)
   const unsigned long long* set_keys;
   const unsigned int* set_cnt;
+  int set_slots;                     // its slots
+  unsigned int* key_counts;          // two zeroed counters for the hot and warm key lists
 };
 
-int pmb_groupby_sketch(pmb_handle* h, const CompiledQuery& cq, SketchOut* out);
+// the sample sketch of a query and, with `select`, the installed selector's outputs (see
+// pmb_selector_read); synchronises the stream
+int pmb_groupby_sketch(pmb_handle* h, const CompiledQuery& cq, SketchOut* out, bool select = false);
 int64_t pmb_estimate_groups(const SketchOut& s, int64_t n_rows);
 int pmb_choose_strategy(pmb_handle* h, const CompiledQuery& cq, const SketchOut& sk, int64_t est);
 // AUTO's switch from a chosen global-table or sort strategy to the partitioned strategy
@@ -108,11 +112,9 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
 // learned selector (pmb_learned.cu): strategy and group count for AUTO; false when no selector is
 // installed or its output is unusable
 bool pmb_selector_pick(pmb_handle* h, const CompiledQuery& cq, int* strategy, int64_t* groups);
-// the same in two halves: the launch queues the selector's kernels and the copy of its outputs into
-// the pinned staging at PMB_SEL_PINNED_OFF (false: no selector); the read decodes them after the
-// caller's next stream synchronisation
+// the outputs that pmb_groupby_sketch(select = true) left in the pinned staging at
+// PMB_SEL_PINNED_OFF, decoded
 #define PMB_SEL_PINNED_OFF 61440
-bool pmb_selector_launch(pmb_handle* h, const CompiledQuery& cq);
 bool pmb_selector_read(pmb_handle* h, const CompiledQuery& cq, int* strategy, int64_t* groups);
 // group counts the selector predicts for a batch of queries (device DQuery array); false without
 // an installed selector

@@ -13,162 +13,16 @@
 #include <vector>
 
 #include "pmb_groupby.h"
+#include "pmb_selector.cuh"
 
 namespace {
 
-constexpr int NF = PMB_SELECTOR_FEATURES;
-constexpr int NH = PMB_SELECTOR_HIDDEN;
-constexpr int NO = PMB_SELECTOR_OUTPUTS;
-constexpr int NS = PMB_SELECTOR_STRATEGIES;  // outputs 0..NS-1: strategy scores; output NS: log2(groups)
-constexpr int OFF_W1 = 0, OFF_B1 = OFF_W1 + NH * NF, OFF_W2 = OFF_B1 + NH, OFF_B2 = OFF_W2 + NH * NH,
-              OFF_W3 = OFF_B2 + NH, OFF_B3 = OFF_W3 + NO * NH, N_PARAMS = OFF_B3 + NO;
-static_assert(N_PARAMS == PMB_SELECTOR_PARAMS, "parameter layout");
-
-constexpr int SAMPLE = 4096;
-constexpr int F_NT = 1024;
-constexpr int TSLOTS = 8192;  // sample counts: slots (count << 32 | 32-bit key fingerprint), dynamic smem
-constexpr int HLL = 256;
-constexpr int BUCKETS = 1024;
+constexpr int SAMPLE_NT = 256;  // threads (samples) per CTA of the sampling kernels
 
 struct FeatParams {
   DQuery q;
   float* out;  // NF floats
 };
-
-__device__ __forceinline__ float lg2p1(double x) { return (float)log2(x + 1.0); }
-
-// sample i of query q (rows evenly spaced over the input): its key hash, never 0, or 0 when the
-// filter drops the row or i is past the sample; `nul` tells whether a key column is null there.
-// One thread per sample, so the sample's loads are all in flight at once.
-__device__ __forceinline__ void sample_one(const DQuery& q, int i, unsigned long long& hv, unsigned char& nul) {
-  hv = 0ULL;
-  nul = 0;
-  const int64_t n = q.n_rows;
-  const int m = (int)(n < SAMPLE ? n : SAMPLE);
-  if (i >= m) return;
-  const TileCtx t{nullptr, nullptr, nullptr, 0};
-  const int64_t r = (int64_t)((__int128)i * n / m);  // evenly spaced rows
-  if (q.prog.n_ops > 0 && !eval_keep(q, t, r)) return;
-  bool anynull = false;
-  for (int k = 0; k < q.n_keys; k++) anynull |= !tc_isvalid(q, t, q.key[k].col, r);
-  unsigned long long lo, hi = 0;
-  if (q.key_bits > 64) {
-    Key128 kk = pack_key128(q, t, r);
-    lo = kk.lo;
-    hi = kk.hi;
-  } else {
-    lo = pack_key64(q, t, r);
-  }
-  hv = pmb_fmix64(lo ^ pmb_fmix64(hi + 0x9E3779B97F4A7C15ULL)) | 1ULL;  // never 0 (empty)
-  nul = anynull ? 1 : 0;
-}
-
-// the features of query q into out[NF] from its samples (hs, ns: SAMPLE entries written by
-// sample_one); called by one whole CTA of F_NT threads
-__device__ __forceinline__ void features_body(const DQuery& q, const unsigned long long* __restrict__ hs,
-                                              const unsigned char* __restrict__ ns, float* out) {
-  extern __shared__ unsigned long long s_slot[];  // TSLOTS
-  __shared__ unsigned int s_hll[HLL];
-  __shared__ unsigned int s_bkt[BUCKETS];
-  __shared__ unsigned int s_acc[16];
-  const int tid = threadIdx.x;
-  for (int i = tid; i < TSLOTS; i += F_NT) s_slot[i] = 0ULL;
-  for (int i = tid; i < HLL; i += F_NT) s_hll[i] = 0u;
-  for (int i = tid; i < BUCKETS; i += F_NT) s_bkt[i] = 0u;
-  if (tid < 16) s_acc[tid] = 0u;
-  __syncthreads();
-  const int64_t n = q.n_rows;
-  const int m = (int)(n < SAMPLE ? n : SAMPLE);
-  const bool pred = q.prog.n_ops > 0;
-  for (int i = tid; i < m; i += F_NT) {
-    const unsigned long long h = hs[i];
-    if (h == 0ULL) continue;  // dropped by the filter
-    atomicAdd(&s_acc[0], 1u);  // kept
-    if (ns[i]) atomicAdd(&s_acc[1], 1u);
-    // HyperLogLog register: index from the top 8 bits, rank of the rest
-    const unsigned reg = (unsigned)(h >> 56);
-    const unsigned rank = (unsigned)__clzll((h << 8) | 0xFFULL) + 1u;
-    atomicMax(&s_hll[reg], rank);
-    atomicAdd(&s_bkt[(h >> 20) & (BUCKETS - 1)], 1u);
-    // exact counts by 32-bit fingerprint (a collision among 4096 samples is rare and only blurs a
-    // feature); a slot holds count << 32 | fingerprint
-    const unsigned fp = (unsigned)(h >> 32) | 1u;
-    unsigned s = (unsigned)(h >> 11) & (TSLOTS - 1);
-    for (int p = 0; p < TSLOTS; p++) {
-      unsigned long long cur = s_slot[s];
-      if (cur == 0ULL) {
-        cur = atomicCAS(&s_slot[s], 0ULL, (1ULL << 32) | fp);
-        if (cur == 0ULL) break;
-      }
-      if ((unsigned)cur == fp) {
-        atomicAdd(&s_slot[s], 1ULL << 32);
-        break;
-      }
-      s = (s + 1) & (TSLOTS - 1);
-    }
-  }
-  __syncthreads();
-  // frequency profile of the sample keys
-  for (int i = tid; i < TSLOTS; i += F_NT) {
-    const unsigned c = (unsigned)(s_slot[i] >> 32);
-    if (!c) continue;
-    atomicAdd(&s_acc[2], 1u);  // distinct
-    if (c == 1) atomicAdd(&s_acc[3], 1u);
-    else if (c == 2) atomicAdd(&s_acc[4], 1u);
-    else if (c <= 4) atomicAdd(&s_acc[5], 1u);
-    else if (c <= 8) atomicAdd(&s_acc[6], 1u);
-    else atomicAdd(&s_acc[7], 1u);
-    atomicMax(&s_acc[8], c);
-  }
-  for (int i = tid; i < BUCKETS; i += F_NT) {
-    if (s_bkt[i]) atomicAdd(&s_acc[9], 1u);
-    atomicMax(&s_acc[10], s_bkt[i]);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    const double kept = s_acc[0], mk = kept > 0 ? kept : 1.0;
-    const double d = s_acc[2], f1 = s_acc[3], f2 = s_acc[4];
-    // HyperLogLog estimate (Flajolet et al. 2007) with linear counting for small ranges
-    double z = 0.0;
-    int zeros = 0;
-    for (int i = 0; i < HLL; i++) {
-      z += ldexp(1.0, -(int)s_hll[i]);
-      zeros += s_hll[i] == 0;
-    }
-    double hll = (0.7213 / (1.0 + 1.079 / HLL)) * HLL * HLL / z;
-    if (hll <= 2.5 * HLL && zeros) hll = HLL * log((double)HLL / zeros);
-    const double neff = (double)n * (m > 0 ? kept / m : 0.0);
-    const double gee = kept > 0 ? sqrt(neff / mk) * f1 + (d - f1) : 0.0;
-    const double chao = d + f1 * f1 / (2.0 * (f2 > 0 ? f2 : 1.0));
-    float* o = out;
-    o[0] = lg2p1((double)n) / 32.f;
-    o[1] = q.key_bits / 128.f;
-    o[2] = (float)(s_acc[1] / mk);
-    o[3] = m > 0 ? (float)(kept / m) : 0.f;
-    o[4] = (float)(d / mk);
-    o[5] = (float)(f1 / mk);
-    o[6] = (float)(f2 / mk);
-    o[7] = (float)(s_acc[5] / mk);
-    o[8] = (float)(s_acc[6] / mk);
-    o[9] = (float)(s_acc[7] / mk);
-    o[10] = (float)(s_acc[8] / mk);
-    o[11] = s_acc[9] / (float)BUCKETS;
-    o[12] = lg2p1(s_acc[10]) / 12.f;
-    o[13] = lg2p1(hll) / 13.f;
-    o[14] = lg2p1(gee) / 32.f;
-    o[15] = lg2p1(chao) / 32.f;
-    o[16] = lg2p1(neff) / 32.f;
-    o[17] = q.rec_bytes / 256.f;
-    o[18] = q.n_fields / 24.f;
-    o[19] = q.n_aggs / 24.f;
-    o[20] = pred ? 1.f : 0.f;
-    o[21] = q.n_keys / 8.f;
-    o[22] = (kept > 0 && d == kept) ? 1.f : 0.f;
-    o[23] = 1.f;
-  }
-}
-
-constexpr int SAMPLE_NT = 256;  // threads (samples) per CTA of the sampling kernels
 
 __global__ void __launch_bounds__(SAMPLE_NT) k_feat_sample(const __grid_constant__ FeatParams F,
                                                            unsigned long long* __restrict__ hs,
@@ -180,7 +34,8 @@ __global__ void __launch_bounds__(SAMPLE_NT) k_feat_sample(const __grid_constant
 __global__ void __launch_bounds__(F_NT) k_features(const __grid_constant__ FeatParams F,
                                                    const unsigned long long* __restrict__ hs,
                                                    const unsigned char* __restrict__ ns) {
-  features_body(F.q, hs, ns, F.out);
+  extern __shared__ unsigned long long s_slots[];
+  features_body(F.q, hs, ns, F.out, s_slots);
 }
 
 // a batch: SAMPLE / SAMPLE_NT sampling CTAs per query, then one feature CTA per query
@@ -198,7 +53,8 @@ __global__ void __launch_bounds__(F_NT) k_features_batch(const DQuery* __restric
                                                          const unsigned char* __restrict__ ns,
                                                          float* __restrict__ out) {
   const size_t qi = blockIdx.x;
-  features_body(qs[qi], hs + qi * SAMPLE, ns + qi * SAMPLE, out + qi * NF);
+  extern __shared__ unsigned long long s_slots[];
+  features_body(qs[qi], hs + qi * SAMPLE, ns + qi * SAMPLE, out + qi * NF, s_slots);
 }
 
 // ---------------------------------------------------------------- MLP (one CTA of 64 threads per sample)
@@ -417,22 +273,8 @@ static bool selector_decode(const float* o, int64_t n_rows, int* strategy, int64
   return true;
 }
 
-// pmb_selector_pick in two halves around a synchronisation the caller makes anyway: the launch
-// queues the feature and MLP kernels and the copy of the outputs into the handle's pinned staging
-// (at PMB_SEL_PINNED_OFF); the read decodes them once the stream has been synchronised.
-bool pmb_selector_launch(pmb_handle* h, const CompiledQuery& cq) {
-  if (!h->selector || cq.dq.n_rows == 0) return false;
-  float* buf = (float*)pmb_ws_alloc(h, (NF + NO) * sizeof(float));
-  if (!buf) return false;
-  if (features_device(h, cq, buf) != PMB_OK) return false;
-  pmb_kernel_begin(h, "mlp_forward");
-  k_mlp_forward<<<1, NH, 0, h->stream>>>(h->selector, buf, 1, buf + NF);
-  pmb_kernel_end(h);
-  if (cudaGetLastError() != cudaSuccess) return false;
-  return cudaMemcpyAsync(h->pinned + PMB_SEL_PINNED_OFF, buf + NF, NO * sizeof(float), cudaMemcpyDeviceToHost,
-                         h->stream) == cudaSuccess;
-}
-
+// The selector's outputs of the sampling launch (pmb_groupby_sketch), once the stream has been
+// synchronised: scores and group count from the handle's pinned staging.
 bool pmb_selector_read(pmb_handle* h, const CompiledQuery& cq, int* strategy, int64_t* groups) {
   float o[NO];
   memcpy(o, h->pinned + PMB_SEL_PINNED_OFF, sizeof(o));

@@ -5,8 +5,9 @@ oracle's; float sums as in tests/helpers.py."""
 import numpy as np
 import pytest
 
-from helpers import as_dict, pack
+from helpers import as_dict, assert_results_match, pack
 from oracle import pyoracle
+from polars_b200 import _abi as A
 from polars_b200 import _native as N
 from test_gpu_sort import assert_same_rows
 
@@ -33,3 +34,19 @@ def test_radix_pass_tiles(n, wide):
     by = ["a", "b"] if wide else ["a"]
     got, want = _sorted_both(cols, by, [True, False][: len(by)])
     assert_same_rows(got, want, f"{n} rows")
+
+
+# the selector's network in the sampling launch: the same pick and table size as selector_choose,
+# whose features and network run as kernels of their own
+@pytest.mark.parametrize("card,width", [(50, 4), (3000, 4), (90_000, 8), (400_000, 8), (1_500_000, 8)])
+def test_selector_in_the_sampling_launch(card, width):
+    rng = np.random.default_rng(card)
+    n = 3_000_000
+    k = rng.integers(0, card, n).astype(np.int32 if width == 4 else np.int64)
+    v = rng.standard_normal(n)
+    q = ({"k": k, "v": v}, ["k"], [("Sum", "v", "s"), ("Len", None, "c")])
+    strategy, groups = N.selector_choose(*q)
+    got = N.groupby(*q)
+    assert got.strategy == strategy and got.n_groups == len(np.unique(k))
+    if got.rehash_count == 0 and strategy.endswith("hash"):
+        assert min(max(2 * groups, 1024), 2 * n) <= got.capacity <= max(3 * groups, 1024) + 3  # slots per estimated group
