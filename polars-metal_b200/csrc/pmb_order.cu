@@ -20,6 +20,7 @@
 //                       the sorted keys when one round holds them all; the other columns are
 //                       gathered by row index, without reading the validity of a column that
 //                       k_null_flags found to have no nulls.
+// A small table takes k_order_small instead, which does all of it in one launch.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -333,8 +334,209 @@ __global__ void __launch_bounds__(OR_NT) k_order_gather(const __grid_constant__ 
   }
 }
 
+// ---------------------------------------------------------------- small tables in one launch
+// Up to SMALL_ROWS rows whose sort columns fit 128 key bits at their full widths: one CTA packs the
+// keys, sorts them in shared memory and gathers the slice, in one launch without a read-back. The
+// general path's launches (ranges, null flags, encode, a pass per digit, gather) and its two
+// read-backs cost 340 us of a 1000-group call whatever the size.
+constexpr int SMALL_ROWS = 8192;
+constexpr int SMALL_NT = 1024;
+
+struct SmallOrder {
+  OrderLayout L;  // fields at the columns' full widths
+  GatherCols G;   // dec >= 0: an integer or Bool sort column (its null rows read 0)
+  int W;
+  int n, n2;      // rows; the next power of two (at least 64)
+  int drop_nulls;
+  long long offset, limit;
+  unsigned long long* out_rows;  // rows written
+};
+
+template <int W>
+__device__ __forceinline__ bool small_less(const unsigned long long* lo, const unsigned long long* hi,
+                                           const unsigned short* ix, int a, int b) {
+  if (W > 1 && hi[a] != hi[b]) return hi[a] < hi[b];
+  if (lo[a] != lo[b]) return lo[a] < lo[b];
+  return ix[a] < ix[b];  // rows with equal keys keep their order
+}
+
+template <int W>
+__global__ void __launch_bounds__(SMALL_NT, 1) k_order_small(const __grid_constant__ SmallOrder S) {
+  extern __shared__ __align__(16) unsigned long long smem_keys[];
+  __shared__ int s_nulls;
+  const int n = S.n, n2 = S.n2, tid = threadIdx.x, lane = tid & 31;
+  unsigned long long* lo = smem_keys;
+  unsigned long long* hi = smem_keys + n2;  // W == 2 only
+  unsigned short* ix = reinterpret_cast<unsigned short*>(smem_keys + (size_t)W * n2);
+  if (tid == 0) s_nulls = 0;
+  __syncthreads();
+  const OrderLayout& L = S.L;
+  for (int r = tid; r < n2; r += SMALL_NT) {
+    unsigned long long k[W];
+    for (int i = 0; i < W; i++) k[i] = r < n ? 0ULL : ~0ULL;  // padding rows sort behind every row
+    if (r < n) {
+      for (int c = 0; c < L.n; c++) {
+        const bool v = pmb_valid_bit(L.valid[c], r);
+        if (L.null_off[c] >= 0) put_bits<W>(k, L.null_off[c], (L.nulls_last[c] ? !v : v) ? 1ULL : 0ULL, 1);
+        if (!v) {
+          if (c == 0 && S.drop_nulls) atomicAdd(&s_nulls, 1);
+          continue;
+        }
+        const unsigned long long o = order_key(pmb_load_bits(L.data[c], L.elem[c], r), L.dtype[c]);
+        put_bits<W>(k, L.data_off[c], L.desc[c] ? L.hi[c] - o : o - L.lo[c], L.data_bits[c]);
+      }
+    }
+    lo[r] = k[0];
+    if (W > 1) hi[r] = k[W - 1];
+    ix[r] = (unsigned short)r;
+  }
+  __syncthreads();
+  // bitonic network; a warp's 32 pairs of a step with j <= 32 lie in its own 64 elements, so those
+  // steps need no CTA barrier among them
+  for (int kk = 2; kk <= n2; kk <<= 1) {
+    for (int j = kk >> 1; j > 0; j >>= 1) {
+      for (int t = tid; t < n2 / 2; t += SMALL_NT) {
+        const int a = 2 * t - (t & (j - 1)), b = a + j;
+        const bool up = (a & kk) == 0;
+        if (small_less<W>(lo, hi, ix, b, a) == up) {
+          const unsigned long long x = lo[a];
+          lo[a] = lo[b];
+          lo[b] = x;
+          if (W > 1) {
+            const unsigned long long y = hi[a];
+            hi[a] = hi[b];
+            hi[b] = y;
+          }
+          const unsigned short z = ix[a];
+          ix[a] = ix[b];
+          ix[b] = z;
+        }
+      }
+      if (j > 32 || j == 1) __syncthreads();
+      else __syncwarp();
+    }
+  }
+  const long long total = S.drop_nulls ? n - s_nulls : n;
+  const long long start = S.offset >= 0 ? min(S.offset, total) : max(0LL, total + S.offset);
+  const int m = (int)(S.limit < 0 ? total - start : min(S.limit, total - start));
+  if (tid == 0) *S.out_rows = (unsigned long long)m;
+  // a warp fills whole validity words; its columns' loads are independent
+  const GatherCols& G = S.G;
+  const int words = (m + 31) / 32;
+  for (int w = tid / 32; w < words; w += SMALL_NT / 32) {
+    const int p = w * 32 + lane;
+    const bool in = p < m;
+    const int r = in ? ix[start + p] : 0;
+    for (int c = 0; c < G.n; c++) {
+      const int e = G.elem[c];
+      const bool v = in && pmb_valid_bit(G.valid[c], r);
+      uint64_t b = in ? pmb_load_bits(G.data[c], e, r) : 0;
+      if (G.dec[c] >= 0 && !v) b = 0;
+      if (in) {
+        switch (e) {
+          case 0: break;
+          case 1: G.out_data[c][p] = (uint8_t)b; break;
+          case 2: reinterpret_cast<uint16_t*>(G.out_data[c])[p] = (uint16_t)b; break;
+          case 4: reinterpret_cast<uint32_t*>(G.out_data[c])[p] = (uint32_t)b; break;
+          default: reinterpret_cast<uint64_t*>(G.out_data[c])[p] = b; break;
+        }
+      }
+      const unsigned vw = __ballot_sync(0xffffffffu, v);
+      const unsigned dw = __ballot_sync(0xffffffffu, in && e == 0 && b);
+      if (lane == 0) {
+        G.out_valid[c][w] = vw;
+        if (e == 0) reinterpret_cast<unsigned int*>(G.out_data[c])[w] = dw;
+      }
+    }
+  }
+}
+
+// order keys of a dtype's smallest value, and the key bits of its whole range
+void full_field(int dt, unsigned long long* lo, int* bits) {
+  *lo = 0;
+  *bits = pmb_dtype_bits(dt);
+  if (pmb_is_signed(dt)) *lo = 0x8000000000000000ULL - (1ULL << (*bits - 1));
+}
+
 int blocks_for(const pmb_handle* h, int64_t threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((threads + OR_NT - 1) / OR_NT, (int64_t)h->sm_count * 8));
+}
+
+// pmb_order_columns for a table that k_order_small takes
+int order_small(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, const pmb_sort_spec& s, const int* desc,
+                const int* nlast, pmb_result* r) {
+  SmallOrder S;
+  memset(&S, 0, sizeof(S));
+  S.n = (int)n;
+  S.n2 = 64;
+  while (S.n2 < S.n) S.n2 *= 2;
+  S.drop_nulls = s.drop_nulls && cols[s.by[0]].valid;
+  S.offset = s.offset;
+  S.limit = s.limit;
+  OrderLayout& L = S.L;
+  GatherCols& G = S.G;
+  L.n = s.n_by;
+  G.n = n_cols;
+  for (int c = 0; c < n_cols; c++) G.dec[c] = -1;
+  int off = 0;
+  for (int k = s.n_by - 1; k >= 0; k--) {  // the most significant column highest
+    const DCol& d = cols[s.by[k]];
+    L.data[k] = d.data;
+    L.valid[k] = d.valid;
+    L.elem[k] = d.elem;
+    L.dtype[k] = d.dtype;
+    L.desc[k] = desc[k];
+    L.nulls_last[k] = nlast[k];
+    full_field(d.dtype, &L.lo[k], &L.data_bits[k]);
+    L.hi[k] = L.lo[k] + (L.data_bits[k] == 64 ? ~0ULL : (1ULL << L.data_bits[k]) - 1ULL);
+    L.data_off[k] = off;
+    off += L.data_bits[k];
+    L.null_off[k] = d.valid ? off : -1;
+    off += d.valid ? 1 : 0;
+    if (!pmb_is_float(d.dtype)) G.dec[s.by[k]] = k;
+  }
+  L.bits = off;
+  S.W = off > 64 ? 2 : 1;
+  // rows of the slice: known here unless rows with a null first column are dropped
+  int64_t start = s.offset >= 0 ? std::min<int64_t>(s.offset, n) : std::max<int64_t>(0, n + s.offset);
+  int64_t m = s.limit < 0 ? n - start : std::min<int64_t>(s.limit, n - start);
+  if (S.drop_nulls) m = n;
+  const int64_t words = (m + 31) / 32;
+  for (int c = 0; c < n_cols; c++) {
+    const int e = cols[c].elem;
+    G.data[c] = cols[c].data;
+    G.valid[c] = cols[c].valid;
+    G.elem[c] = e;
+    G.out_data[c] = (uint8_t*)pmb_ws_alloc(h, (e ? (size_t)m * e : (size_t)words * 4) + 16);
+    G.out_valid[c] = (unsigned int*)pmb_ws_alloc(h, (size_t)words * 4 + 16);
+    if (!G.out_data[c] || !G.out_valid[c]) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort outputs)");
+  }
+  S.out_rows = (unsigned long long*)pmb_ws_alloc(h, 16);
+  if (!S.out_rows) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort rows)");
+  const int smem = S.n2 * (8 * S.W + 2);
+  pmb_kernel_begin(h, "order_small");
+  if (S.W == 1) {
+    PMB_CUDA(h, cudaFuncSetAttribute(k_order_small<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_order_small<1><<<1, SMALL_NT, smem, h->stream>>>(S);
+  } else {
+    PMB_CUDA(h, cudaFuncSetAttribute(k_order_small<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_order_small<2><<<1, SMALL_NT, smem, h->stream>>>(S);
+  }
+  pmb_kernel_end(h);
+  PMB_CUDA(h, cudaGetLastError());
+  if (S.drop_nulls) {
+    PMB_CUDA(h, cudaMemcpyAsync(h->pinned, S.out_rows, 8, cudaMemcpyDeviceToHost, h->stream));
+    PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+    m = (int64_t) * (unsigned long long*)h->pinned;
+  }
+  r->n_groups = m;
+  for (int c = 0; c < n_cols; c++) {
+    r->columns[c].data = G.out_data[c];
+    r->columns[c].validity = (uint8_t*)G.out_valid[c];
+    r->columns[c].length = m;
+    r->columns[c].on_device = 1;
+  }
+  return PMB_OK;
 }
 
 }  // namespace
@@ -354,6 +556,12 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     nlast[k] = s.nulls_last ? (s.nulls_last[k] != 0) : 0;
   }
   if (s.drop_nulls) nlast[0] = 1;  // the first column's nulls last, then cut off
+  int full_bits = 0;
+  for (int k = 0; k < nb; k++) {
+    const DCol& d = cols[s.by[k]];
+    full_bits += pmb_dtype_bits(d.dtype) + (d.valid != nullptr);
+  }
+  if (n > 1 && n <= SMALL_ROWS && full_bits <= 128) return order_small(h, cols, n_cols, n, s, desc, nlast, r);
   // ranges and null counts of the sort columns
   SortCols C;
   memset(&C, 0, sizeof(C));

@@ -36,6 +36,25 @@ def test_radix_pass_tiles(n, wide):
     assert_same_rows(got, want, f"{n} rows")
 
 
+# the one-launch sort of small tables: padding to a power of two (at least 64), its largest size and
+# the general path's smallest, one- and two-word keys, dropped nulls, slices
+@pytest.mark.parametrize("spec", [(["a"], [False], {}), (["b", "a"], [True, False], {"nulls_last": True}),
+                                  (["a"], [True], {"drop_nulls": True, "nulls_last": True, "limit": 7}),
+                                  (["f", "s"], [False, True], {"offset": -20, "limit": 15})], ids=lambda s: "-".join(s[0]))
+@pytest.mark.parametrize("n", [2, 33, 64, 65, 1000, 4096, 8191, 8192, 8193])
+def test_small_sort(n, spec):
+    by, desc, kw = spec
+    rng = np.random.default_rng(n)
+    f = rng.standard_normal(n).astype(np.float32)
+    f[rng.random(n) < 0.2] = np.float32(-0.0)
+    f[rng.random(n) < 0.1] = np.float32("nan")
+    cols = {"a": (rng.integers(-40, 40, n), pack(rng.random(n) > 0.2)), "f": (f, None),
+            "b": (rng.integers(-2**31, 2**31, n).astype(np.int32), pack(rng.random(n) > 0.1)),
+            "s": (rng.integers(-128, 128, n).astype(np.int8), None), "row": (np.arange(n), None)}
+    got, want = _sorted_both(cols, by, desc, **kw)
+    assert_same_rows(got, want, f"{n} rows by {by}")
+
+
 # the selector's network in the sampling launch: the same pick and table size as selector_choose,
 # whose features and network run as kernels of their own
 @pytest.mark.parametrize("card,width", [(50, 4), (3000, 4), (90_000, 8), (400_000, 8), (1_500_000, 8)])
