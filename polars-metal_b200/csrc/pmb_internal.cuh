@@ -182,6 +182,7 @@ struct pmb_handle {
   // pinned host staging (pmb_host_stage)
   uint8_t* hstage = nullptr;
   size_t hstage_cap = 0, hstage_used = 0, hstage_want = 0;
+  uint8_t* rstage = nullptr;  // pinned staging of small results (pmb_finish_outputs), allocated at first use
   // profiling
   bool profiling = false;
   bool batching = true;  // pmb_groupby_batched may batch (else: one pmb_groupby per query)

@@ -55,6 +55,24 @@ def test_small_sort(n, spec):
     assert_same_rows(got, want, f"{n} rows by {by}")
 
 
+# host results: in one copy up to 4 MB of span (whole and partial bitmap bytes), a copy per buffer above
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 4099, 170_000, 180_000, 400_003])
+def test_host_results(n):
+    rng = np.random.default_rng(n)
+    x, y = rng.standard_normal(n), rng.integers(-100, 100, n).astype(np.int8)
+    z, ok = rng.integers(0, 2**60, n), rng.random(n) > 0.3
+    keep = x > -3.0
+    got = N.filter_columns({"x": x, "y": y, "z": N.ColumnData(z, pack(ok))},
+                           {"kind": "Compare", "op": "Gt", "lhs": {"kind": "Column", "name": "x"},
+                            "rhs": {"kind": "LiteralF64", "value": -3.0}})
+    m = int(keep.sum())
+    assert got.n_groups == m
+    for have, want in zip(got.data, (x, y, z)):
+        assert np.array_equal(have[:m], want[keep])
+    assert np.array_equal(np.unpackbits(got.validity[2], bitorder="little")[:m].astype(bool), ok[keep])
+    assert np.unpackbits(got.validity[0], bitorder="little")[:m].all() if m else True
+
+
 # the selector's network in the sampling launch: the same pick and table size as selector_choose,
 # whose features and network run as kernels of their own
 @pytest.mark.parametrize("card,width", [(50, 4), (3000, 4), (90_000, 8), (400_000, 8), (1_500_000, 8)])
