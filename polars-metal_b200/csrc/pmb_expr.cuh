@@ -259,7 +259,7 @@ __device__ __forceinline__ uint64_t pack_key64(const DQuery& q, const TileCtx& t
       k |= 1ULL << K.null_off;
       continue;
     }
-    uint64_t v = tc_bits(q, t, K.col, lr);
+    uint64_t v = tc_bits(q, t, K.col, lr) - K.bias;
     if (K.bits < 64) v &= (1ULL << K.bits) - 1ULL;
     k |= v << K.data_off;
   }
@@ -308,6 +308,7 @@ __device__ __forceinline__ bool unpack_field(const DKey& K, uint64_t lo, uint64_
     v = hi >> (o - 64);
   }
   if (K.bits < 64) v &= (1ULL << K.bits) - 1ULL;
+  v += K.bias;
   return true;
 }
 

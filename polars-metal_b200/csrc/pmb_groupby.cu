@@ -1230,6 +1230,8 @@ int recompile_dd(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int3
     nc.dq.col[c].data = cq.dq.col[c].data;
     nc.dq.col[c].valid = cq.dq.col[c].valid;
   }
+  nc.ranges = cq.ranges;
+  if (cq.dq.packed) pmb_apply_packed_keys(nc);
   cq = nc;
   return PMB_OK;
 }
@@ -1262,6 +1264,9 @@ extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* 
     if (rc) return bail(rc);
   }
   pmb_phase(h, "stage");
+  rc = pmb_pack_wide_keys(h, cq);
+  if (rc) return bail(rc);
+  pmb_phase(h, "pack");
   if (cq.dq.n_rows == 0) {
     r->n_groups = 0;
     r->strategy_used = q->strategy ? q->strategy : PMB_STRATEGY_GLOBAL_HASH;

@@ -93,6 +93,11 @@ int pmb_plan_hash(pmb_handle* h, int max_smem_optin, CompiledQuery& cq, int stra
 // group count (two estimates, so the table is sized tighter: 2 slots per group instead of 4)
 int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int strategy, int64_t est,
                      const SketchOut* sk, pmb_result* r, bool est_learned = false);
+// Keys wider than 64 bits at their types' widths: reads the key columns' ranges and, when the values
+// fit 64 bits, lays the key out as (value - smallest value) fields (pmb_sort.cu)
+int pmb_pack_wide_keys(pmb_handle* h, CompiledQuery& cq);
+// the layout alone, from cq.ranges; false (and nothing changed) when it needs more than 64 bits
+bool pmb_apply_packed_keys(CompiledQuery& cq);
 // compiles the query again with cq.dd_user_cols, keeping the staged column pointers
 int recompile_dd(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols, CompiledQuery& cq);
 // keys = EMPTY, records = identity (k_table_init) on stream s

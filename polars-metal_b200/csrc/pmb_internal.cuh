@@ -101,6 +101,7 @@ struct DKey {
   int8_t bits;
   int16_t null_off;
   int16_t data_off;
+  uint64_t bias;  // subtracted from the value's raw bits (0 unless the keys are range-packed)
 };
 
 // aggregation state field kinds
@@ -147,7 +148,7 @@ struct DQuery {
   int64_t n_rows;
   int16_t fx_e[8];   // exact float sums: every value of slot i satisfies |x| < 2^fx_e[i]
   uint32_t valid_if_kept;  // bit c: column c is non-null in every row the filter keeps
-  uint32_t pad_vk;
+  uint32_t packed;  // key width by the types when the fields hold value - smallest value (pmb_pack_wide_keys), else 0
   DCol col[PMB_MAX_COLS];
   DKey key[PMB_MAX_KEYS];
   DField field[PMB_MAX_FIELDS];

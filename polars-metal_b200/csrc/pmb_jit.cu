@@ -711,10 +711,19 @@ __device__ __forceinline__ long long j_fdiv_i(long long a, long long b, bool& ok
     fxcheck(o);
     o << "}\n";
     // key
-    o << "__device__ __forceinline__ unsigned long long j_key(const JRow& r) {\n  unsigned long long k = 0ULL;\n";
+    o << "__device__ __forceinline__ unsigned long long j_key(const JParams& P, const JRow& r) {\n  unsigned long long k = 0ULL;\n";
     // (keys wider than 64 bits never use it: the partitioned kernel reads packed sort keys)
     for (int i = 0; i < q.n_keys && q.key_bits <= 64; i++) {
       const DKey& K = q.key[i];
+      if (q.packed) {
+        const std::string is = std::to_string(i);
+        const int e = q.col[K.col].elem;
+        const std::string wrap = e == 8 ? "" : e == 0 ? " & 1ULL" : " & " + std::to_string((1ULL << (8 * e)) - 1ULL) + "ULL";
+        const std::string put = "k |= ((" + raw_bits(K.col) + " - P.kbias[" + is + "])" + wrap + ") << P.kshift[" + is + "];";
+        if (K.nullable) o << "  if (!" << ok(K.col) << ") k |= 1ULL << P.knull[" << is << "]; else " << put << "\n";
+        else o << "  " << put << "\n";
+        continue;
+      }
       std::string mask = K.bits < 64 ? std::to_string((1ULL << K.bits) - 1ULL) + "ULL" : "0xFFFFFFFFFFFFFFFFULL";
       std::string put = "k |= (" + raw_bits(K.col) + " & " + mask + ") << " + std::to_string(K.data_off) + ";";
       if (K.nullable)
@@ -725,7 +734,7 @@ __device__ __forceinline__ long long j_fdiv_i(long long a, long long b, bool& ok
     o << "  return k;\n}\n";
     // hash of a packed key: MurmurHash3's 32-bit finalizer for keys of at most 32 bits (its word
     // repeated, so that the high and the low bits both vary), the 64-bit finalizer otherwise
-    if (q.key_bits <= 32)
+    if (q.key_bits <= 32 && !q.packed)
       o << "__device__ __forceinline__ unsigned long long j_hash(unsigned long long k) {\n"
            "  const unsigned x = pmb_fmix32((unsigned)k);\n  return ((unsigned long long)x << 32) | x;\n}\n";
     else
@@ -861,7 +870,7 @@ int pmb_plan_jit(pmb_handle* h, const CompiledQuery& cq, bool have_sketch, int m
   // hot keys: one record per warp each; warm keys: the largest count whose table and records fit.
   // The sampled-key table: buckets of 4 keys and 4 16-bit values, filled to at most 50% (a key
   // sits in its first bucket unless that one was full, so most lookups read one bucket).
-  J->tkey = q.key_bits <= 32 ? 4 : 8;
+  J->tkey = q.key_bits <= 32 && !q.packed ? 4 : 8;
   auto buckets = [](int keys) { return keys ? ((keys / 2 + 2) + 1) & ~1 : 0; };
   auto tbytes = [&](int keys) { return buckets(keys) * 4 * (J->tkey + 2); };
   // 24 hot keys (a record per warp each): measured best on the hash workload (100M rows, Zipf 1.1
@@ -968,6 +977,15 @@ static std::string hash_signature(const CompiledQuery& cq, const JitPlan& J) {
     d.col[c].valid = d.col[c].valid ? reinterpret_cast<const uint8_t*>(1) : nullptr;
   }
   for (int f = 0; f < PMB_MAX_FIELDS; f++) d.field[f].fx = 0;
+  if (d.packed) {
+    d.packed = 1;
+    d.key_bits = 64;
+    for (int i = 0; i < PMB_MAX_KEYS; i++) {
+      d.key[i].bias = 0;
+      d.key[i].bits = 0;
+      d.key[i].null_off = d.key[i].data_off = 0;
+    }
+  }
   std::string k(reinterpret_cast<const char*>(&d), sizeof d);
   k.append(reinterpret_cast<const char*>(&J), sizeof J);
   if (const char* path = getenv("PMB_JIT_SKELETON")) k.append(path);
@@ -1216,6 +1234,11 @@ int pmb_jit_launch(pmb_handle* h, cudaKernel_t k, const CompiledQuery& cq, const
   A.kstats = P.kstats;
   A.ttab = ttab;
   A.tnb = ttab ? tnb : 0;
+  for (int k2 = 0; k2 < cq.dq.n_keys; k2++) {
+    A.kbias[k2] = cq.dq.key[k2].bias;
+    A.kshift[k2] = cq.dq.key[k2].data_off;
+    A.knull[k2] = cq.dq.key[k2].null_off;
+  }
   for (int i = 0; i < cq.dq.n_fields; i++)
     if (cq.dq.field[i].kind == F_SUM_FX) {
       A.fx[cq.dq.field[i].fx_slot] = cq.dq.field[i].fx;

@@ -25,6 +25,9 @@ struct JitParams {
   int flags;  // batched kernel: bit 0 = fill the CTA's warm table
   int fx[8];
   int fx_e[8];
+  unsigned long long kbias[8];
+  int kshift[8];
+  int knull[8];
 };
 
 // shared-memory layout of the run-time kernel: per-warp 128-row unit buffers and queues, the

@@ -137,7 +137,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_batch_agg(const __
         const bool keep = lr < rows && j_load_pk(P, st, lr, r);
         ent[j] = 0u;
         if (keep) {
-          const unsigned long long key = j_key(r);
+          const unsigned long long key = j_key(P, r);
           unsigned rec = J_MISS;
           for (int i = 0; i < nhot; i++)
             if (hk[i] == key) rec = (unsigned)(warp * J_H + i);
@@ -173,7 +173,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_batch_agg(const __
           JRow r;
           j_load_key(P, st, lr, r);
           j_load_vals(P, st, lr, r);
-          const unsigned long long key = j_key(r);
+          const unsigned long long key = j_key(P, r);
           j_fxcheck(P, r);
           bool claimed;
           const long long gi = j_gresolve(P, key, j_hash(key), claimed);

@@ -6,7 +6,8 @@
 //   JRow           the values of one row of a unit buffer
 //   j_load_pk      the predicate and key columns of a row, and the filter verdict
 //   j_load_vals    the aggregated columns of a row
-//   j_key          the packed 64-bit group key
+//   j_key          the packed 64-bit group key (range-packed keys: their layout is a parameter, so
+//                  that another range of values needs no other kernel)
 //   j_fxcheck      range report of the exact float sums (the call is re-run wider on a report)
 //   j_shared       one row into a shared-memory record (native 32-bit atomics only: counters,
 //                  carry-chained 32-bit words for the exact sums, 64-bit min/max)
@@ -51,6 +52,9 @@ struct JParams {
   int flags;                  // batched kernel: bit 0 = fill the CTA's warm table
   int fx[8];    // fraction bits F of each exact float-sum slot (sums hold x * 2^F)
   int fx_e[8];  // every value of the slot satisfies |x| < 2^fx_e
+  unsigned long long kbias[8];  // range-packed keys: smallest value, field and null bit positions
+  int kshift[8];
+  int knull[8];
 };
 
 #define J_UNIT 128
@@ -236,7 +240,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_hash_agg(const __g
       const int lr = lane + 32 * j;  // rows past a partial unit read stale buffer bytes, then drop
       JRow r;
       const bool keep = j_load_pk(P, st, lr, r) && lr < rows;
-      const unsigned long long key = j_key(r);
+      const unsigned long long key = j_key(P, r);
       const unsigned a = (unsigned)(j_hash(key) >> 32);
       unsigned v = J_MISS;
       bool full = false;
@@ -291,7 +295,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_hash_agg(const __g
         JRow r;
         j_load_key(P, st, lr, r);
         j_load_vals(P, st, lr, r);
-        const unsigned long long key = j_key(r);
+        const unsigned long long key = j_key(P, r);
         j_fxcheck(P, r);
         const unsigned long long hk = j_hash(key);
         bool claimed = false;

@@ -341,6 +341,8 @@ extern "C" int pmb_selector_choose(pmb_handle* h, const pmb_query* q, const pmb_
   CompiledQuery cq;
   int rc = stage_query(h, q, cols, n_cols, &cq);
   if (rc) return rc;
+  rc = pmb_pack_wide_keys(h, cq);
+  if (rc) return rc;
   int s = 0;
   int64_t g = 0;
   // the same decisions as pmb_groupby's AUTO: sample estimate, selector (which can only enlarge

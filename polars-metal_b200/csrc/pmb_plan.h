@@ -24,6 +24,12 @@ struct CompiledQuery {
   // caller's columns whose float sums use double-double accumulation instead of the exact
   // fixed point (kept by pmb_compile_groupby; see PMB_FX_MIN_F)
   std::vector<int> dd_user_cols;
+  // ranges of the key columns' values over all rows, as order-preserving integers (have: read)
+  struct KeyRanges {
+    bool have = false;
+    unsigned long long lo[PMB_MAX_KEYS], hi[PMB_MAX_KEYS];
+    unsigned int nulls[PMB_MAX_KEYS], any[PMB_MAX_KEYS];
+  } ranges;
 };
 
 // Fewest fraction bits an exact float sum may have. A column whose range needs more integer bits

@@ -156,7 +156,7 @@ __device__ __forceinline__ void features_body(const DQuery& q, const unsigned lo
     const double chao = d + f1 * f1 / (2.0 * (f2 > 0 ? f2 : 1.0));
     float* o = out;
     o[0] = lg2p1((double)n) / 32.f;
-    o[1] = q.key_bits / 128.f;
+    o[1] = (q.packed ? (int)q.packed : q.key_bits) / 128.f;  // by the key's types
     o[2] = (float)(s_acc[1] / mk);
     o[3] = m > 0 ? (float)(kept / m) : 0.f;
     o[4] = (float)(d / mk);

@@ -73,6 +73,37 @@ def test_host_results(n):
     assert np.unpackbits(got.validity[0], bitorder="little")[:m].all() if m else True
 
 
+# keys wider than 64 bits by their types whose values fit 64: nullable Int64 alone, column pairs, the
+# extremes of the types, a span of exactly 64 bits and one of 65 (which stays on the 128-bit path)
+@pytest.mark.parametrize("n", [1, 3000, 2_200_000])
+@pytest.mark.parametrize("case", ["nullable", "all null", "pair", "negative", "span64", "span65", "floats"])
+def test_wide_keys(case, n):
+    rng = np.random.default_rng(len(case) + n)
+    g = rng.integers(0, 300, n)
+    ok = pack(rng.random(n) > 0.1)
+    big = np.where(g % 2 == 0, np.int64(-2**63), np.int64(2**63 - 1))
+    keys = {
+        "nullable": {"k": (g * 7_000_000_000 - 900, ok)},
+        "all null": {"k": (g, pack(np.zeros(n, bool)))},
+        "pair": {"k": (g - (1 << 40), None), "j": (rng.integers(-5, 5, n).astype(np.int32), ok)},
+        "negative": {"k": (-(g << 33), ok), "j": ((g % 3 - 128).astype(np.int8), None), "b": (pack(g % 5 == 0), None, A.BOOL, n)},
+        "span64": {"k": (big, None), "j": (np.full(n, 9, np.int16), None)},
+        "span65": {"k": (big, None), "j": ((g % 2).astype(np.int16), None)},
+        "floats": {"k": ((g % 50) * 0.25 - 3.0, ok), "j": ((g % 4).astype(np.float32) - 1.5, None)},
+    }[case]
+    v = rng.standard_normal(n)
+    cols = {**keys, "v": (v, pack(rng.random(n) > 0.05))}
+    aggs = [("Sum", "v", "s"), ("Max", "v", "m"), ("Len", None, "c")]
+    inv = {d: k for k, d in A.NUMPY_NAME.items()}
+    data = {k: N.ColumnData(c[0], c[1], dtype=c[2], length=c[3]) if len(c) > 2 else N.ColumnData(c[0], c[1])
+            for k, c in cols.items()}
+    full = {k: c if len(c) > 2 else (c[0], c[1], inv[c[0].dtype.name], n) for k, c in cols.items()}
+    want = pyoracle.groupby(full, list(keys), aggs, None)
+    for strategy in ("auto", "global_hash"):
+        got = N.groupby(data, list(keys), aggs, strategy=strategy)
+        assert_results_match(as_dict(got), want, len(keys), aggs, f"{case} {strategy}")
+
+
 # the selector's network in the sampling launch: the same pick and table size as selector_choose,
 # whose features and network run as kernels of their own
 @pytest.mark.parametrize("card,width", [(50, 4), (3000, 4), (90_000, 8), (400_000, 8), (1_500_000, 8)])
