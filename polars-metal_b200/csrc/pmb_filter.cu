@@ -267,52 +267,55 @@ int run_compact(pmb_handle* h, CompiledQuery& cq, const uint8_t* keep_d, const u
   pmb_result* r = pmb_result_new(n_out);
   if (!r) return pmb_fail(h, PMB_E_OOM, "host allocation failed");
   for (int c = 0; c < n_out; c++) r->columns[c].dtype = q.col[c].dtype;
-  int64_t tiles = std::max<int64_t>(1, (n + CT_TILE - 1) / CT_TILE);
+  // a predicate over many rows: the run-time compiled compaction (literal offsets and dtypes)
+  cudaKernel_t jk = nullptr;
+  JitCompactPlan C;
+  if (n > 0 && !keep_d && pmb_jit_enabled(n)) {
+    std::string keep_err = h->err;
+    if (pmb_jit_compact_kernel(h, cq, n_out, &C, &jk) != PMB_OK) jk = nullptr;  // prebuilt kernel: same results
+    h->err = keep_err;
+  }
+  const int64_t tile = jk ? C.tile : CT_TILE;
+  const int64_t tiles = std::max<int64_t>(1, (n + tile - 1) / tile);
   CompactParams P;
   memset(&P, 0, sizeof(P));
   P.q = q;
   P.keep_data = keep_d;
   P.keep_valid = keep_v;
   P.n_out_cols = n_out;
-  // look-back states for whichever kernel runs (the run-time compiled one has smaller tiles)
-  const int64_t lb_tiles = std::max<int64_t>(tiles, (n + JC_TILE_ROWS - 1) / JC_TILE_ROWS);
-  P.lb = (unsigned long long*)pmb_ws_alloc(h, (size_t)lb_tiles * 8 + 64);
-  unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
-  if (!P.lb || !status) {
+  // what must start zeroed, in one block and one memset: status, ticket, row count and look-back
+  // states, then the output bitmaps (they were a memset each: 64 us of a 7-column call)
+  const size_t ctr_bytes = pmb_align(64 + (size_t)tiles * 8, 256);
+  const size_t vb = pmb_align((size_t)((n + 31) / 32 * 4) + 16, 256);
+  size_t bitmaps = (size_t)n_out;
+  for (int c = 0; c < n_out; c++) bitmaps += q.col[c].elem == 0;
+  uint8_t* zeroed = (uint8_t*)pmb_ws_alloc(h, ctr_bytes + bitmaps * vb);
+  if (!zeroed) {
     pmb_result_free(r);
     return pmb_fail(h, PMB_E_OOM, "workspace exhausted (compaction)");
   }
-  P.ticket = P.lb + lb_tiles;
-  P.n_out = P.lb + lb_tiles + 1;
-  P.status = status;
-  cudaMemsetAsync(P.lb, 0, (size_t)lb_tiles * 8 + 64, h->stream);
-  cudaMemsetAsync(status, 0, 64, h->stream);
+  P.status = (unsigned int*)zeroed;
+  P.n_out = (unsigned long long*)(zeroed + 8);
+  P.ticket = (unsigned long long*)(zeroed + 16);
+  P.lb = (unsigned long long*)(zeroed + 64);
+  uint8_t* next = zeroed + ctr_bytes;
   for (int c = 0; c < n_out; c++) {
-    int e = q.col[c].elem;
-    size_t db = e ? (size_t)n * e : (size_t)((n + 31) / 32 * 4);
-    size_t vb = (size_t)((n + 31) / 32 * 4);
-    P.out_data[c] = (uint8_t*)pmb_ws_alloc(h, db + 16);
-    P.out_valid[c] = (unsigned int*)pmb_ws_alloc(h, vb + 16);
-    if (!P.out_data[c] || !P.out_valid[c]) {
+    const int e = q.col[c].elem;
+    P.out_valid[c] = (unsigned int*)next;
+    next += vb;
+    if (e) {
+      P.out_data[c] = (uint8_t*)pmb_ws_alloc(h, (size_t)n * e + 16);
+    } else {
+      P.out_data[c] = next;
+      next += vb;
+    }
+    if (!P.out_data[c]) {
       pmb_result_free(r);
       return pmb_fail(h, PMB_E_OOM, "workspace exhausted (compaction outputs)");
     }
-    cudaMemsetAsync(P.out_valid[c], 0, vb + 16, h->stream);
-    if (!e) cudaMemsetAsync(P.out_data[c], 0, db + 16, h->stream);
   }
-  // a predicate over many rows: the run-time compiled compaction (literal offsets and dtypes)
-  cudaKernel_t jk = nullptr;
-  if (n > 0 && !keep_d && pmb_jit_enabled(n)) {
-    std::string keep_err = h->err;
-    if (pmb_jit_compact_kernel(h, cq, n_out, &jk) != PMB_OK) jk = nullptr;  // prebuilt kernel: same results
-    h->err = keep_err;
-  }
+  cudaMemsetAsync(zeroed, 0, ctr_bytes + bitmaps * vb, h->stream);
   if (n > 0 && jk) {
-    const int64_t jt = (n + JC_TILE_ROWS - 1) / JC_TILE_ROWS;
-    if (jt > lb_tiles) {
-      pmb_result_free(r);
-      return pmb_fail(h, PMB_E_CUDA, "internal: compaction tiles");
-    }
     JitCompactParams A;
     memset(&A, 0, sizeof(A));
     for (int c = 0; c < q.n_cols; c++) {
@@ -328,9 +331,14 @@ int run_compact(pmb_handle* h, CompiledQuery& cq, const uint8_t* keep_d, const u
       A.out_data[c] = P.out_data[c];
       A.out_valid[c] = P.out_valid[c];
     }
+    // persistent CTAs: as many as an SM's shared memory and threads hold
+    const int per_sm = std::max(1, std::min(2048 / JC_THREADS, (227 << 10) / (C.smem + (4 << 10))));
+    const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)h->sm_count * per_sm);
     void* args[] = {&A};
+    cudaError_t e = cudaFuncSetAttribute((const void*)jk, cudaFuncAttributeMaxDynamicSharedMemorySize, C.smem);
     pmb_kernel_begin(h, "compact");
-    cudaError_t e = cudaLaunchKernel((const void*)jk, dim3((unsigned)jt), dim3(256), args, 0, h->stream);
+    if (e == cudaSuccess)
+      e = cudaLaunchKernel((const void*)jk, dim3(grid), dim3(JC_THREADS), args, (size_t)C.smem, h->stream);
     pmb_kernel_end(h);
     if (e != cudaSuccess) {
       pmb_result_free(r);
@@ -346,8 +354,7 @@ int run_compact(pmb_handle* h, CompiledQuery& cq, const uint8_t* keep_d, const u
       return pmb_cuda_check(h, e, "k_compact launch");
     }
   }
-  cudaMemcpyAsync(h->pinned, status, 4, cudaMemcpyDeviceToHost, h->stream);
-  cudaMemcpyAsync(h->pinned + 8, P.n_out, 8, cudaMemcpyDeviceToHost, h->stream);
+  cudaMemcpyAsync(h->pinned, zeroed, 16, cudaMemcpyDeviceToHost, h->stream);
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
     pmb_result_free(r);

@@ -533,55 +533,62 @@ struct Gen {
     }
   }
 
-  // the top-level filter's row functions. A row's values (the predicate's columns and the first
-  // `n_out` columns, the outputs) are read once into a JCRow (j_cload), its verdict is taken from
-  // those registers (j_ckeep), and the kept row is written from them (j_cscatter; every lane of
-  // the warp calls it: the validity words are OR-ed warp-wide). Reading the columns once matters:
-  // a second read at the scatter, after the tile's look-back, mostly missed L2 (1.48x the
-  // algorithmic DRAM reads on the hash workload's filter).
-  std::string compact_funcs(int n_out) {
+  // the top-level filter's functions over a stage of `tile` rows (this generator's plan holds the
+  // stage's column offsets): copies in, verdict, output of the first `n_out` columns
+  std::string compact_funcs(int n_out, int tile) {
     std::ostringstream b;
     mark();
     std::ostringstream body;
-    std::string keep = predicate(body);
-    std::vector<bool> use(q.n_cols, false);
-    for (int c = 0; c < q.n_cols; c++) use[c] = pred_col[c] || c < n_out;
-    b << "struct JCRow {\n";
+    const std::string keep = predicate(body);
+    b << "#define JC_TILE " << tile << "\n#define JC_STAGE " << P.buf_bytes << "\n";
+    b << "__device__ __forceinline__ void jc_issue(const JCParams& P, unsigned char* st, long long t, "
+         "unsigned long long* bar, unsigned long long pol) {\n  mbar_arrive_expect_tx(bar, " << P.tx_bytes << "u);\n";
     for (int c = 0; c < q.n_cols; c++) {
-      if (!use[c]) continue;
+      const DCol& C = q.col[c];
+      const int db = C.elem ? tile * C.elem : tile / 8;
+      b << "  bulk_g2s_hint(st + " << P.doff[c] << ", P.col_data[" << c << "] + t * " << db << "LL, " << db
+        << "u, bar, pol);\n";
+      if (C.valid)
+        b << "  bulk_g2s_hint(st + " << P.voff[c] << ", P.col_valid[" << c << "] + t * " << tile / 8 << "LL, " << tile / 8
+          << "u, bar, pol);\n";
+    }
+    b << "}\n__device__ void jc_copy(const JCParams& P, unsigned char* st, long long row0, int rows) {\n";
+    for (int c = 0; c < q.n_cols; c++) {
+      const DCol& C = q.col[c];
+      if (C.elem)
+        b << "  for (int i = threadIdx.x; i < rows; i += blockDim.x) reinterpret_cast<" << ctype(C.dtype) << "*>(st + "
+          << P.doff[c] << ")[i] = reinterpret_cast<const " << ctype(C.dtype) << "*>(P.col_data[" << c << "])[row0 + i];\n";
+      else
+        b << "  for (int i = threadIdx.x; i < (rows + 7) / 8; i += blockDim.x) st[" << P.doff[c] << " + i] = P.col_data["
+          << c << "][row0 / 8 + i];\n";
+      if (C.valid)
+        b << "  for (int i = threadIdx.x; i < (rows + 7) / 8; i += blockDim.x) st[" << P.voff[c] << " + i] = P.col_valid["
+          << c << "][row0 / 8 + i];\n";
+    }
+    b << "}\nstruct JCRow {\n";
+    for (int c = 0; c < q.n_cols; c++) {
+      if (!pred_col[c]) continue;
       b << "  " << (q.col[c].dtype == PMB_BOOL ? "bool" : ctype(q.col[c].dtype)) << " v" << c << ";\n";
       if (q.col[c].valid) b << "  bool ok" << c << ";\n";
     }
-    b << "};\n";
-    b << "__device__ __forceinline__ void j_cload(const JCParams& P, long long row, JCRow& r) {\n";
+    b << "};\n__device__ __forceinline__ bool jc_keep(const unsigned char* st, int lr) {\n  JCRow r;\n";
     for (int c = 0; c < q.n_cols; c++) {
-      if (!use[c]) continue;
-      const DCol& C = q.col[c];
-      const std::string cs = std::to_string(c);
-      if (C.dtype == PMB_BOOL)
-        b << "  r.v" << cs << " = ((P.col_data[" << cs << "][row >> 3] >> (row & 7)) & 1) != 0;\n";
-      else
-        b << "  r.v" << cs << " = reinterpret_cast<const " << ctype(C.dtype) << "*>(P.col_data[" << cs << "])[row];\n";
-      if (C.valid) b << "  r.ok" << cs << " = ((P.col_valid[" << cs << "][row >> 3] >> (row & 7)) & 1) != 0;\n";
+      if (!pred_col[c]) continue;
+      b << "  r.v" << c << " = " << load_val(c) << ";\n";
+      if (q.col[c].valid) b << "  r.ok" << c << " = " << load_valid(c) << ";\n";
     }
-    b << "}\n";
-    b << "__device__ __forceinline__ bool j_ckeep(const JCRow& r) {\n" << body.str() << "  return " << keep << ";\n}\n";
-    b << "__device__ __forceinline__ void j_cscatter(const JCParams& P, const JCRow& r, bool keep, long long p, "
-         "long long p_first) {\n";
+    b << body.str() << "  return " << keep << ";\n}\n";
+    b << "__device__ __forceinline__ void jc_out(const JCParams& P, const unsigned char* st, int lr, bool in, long long p, "
+         "long long w, bool full) {\n";
     for (int c = 0; c < n_out && c < q.n_cols; c++) {
       const DCol& C = q.col[c];
-      const std::string cs = std::to_string(c);
-      if (C.dtype == PMB_BOOL) {
-        b << "  jc_set_bits(reinterpret_cast<unsigned int*>(P.out_data[" << cs << "]), p, p_first, keep && r.v" << cs
-          << ");\n";
-      } else {
-        const std::string T = ctype(C.dtype);
-        b << "  if (keep) reinterpret_cast<" << T << "*>(P.out_data[" << cs << "])[p] = r.v" << cs << ";\n";
-      }
-      if (C.valid)
-        b << "  jc_set_bits(P.out_valid[" << cs << "], p, p_first, keep && r.ok" << cs << ");\n";
+      if (C.dtype == PMB_BOOL)
+        b << "  jc_word(reinterpret_cast<unsigned int*>(P.out_data[" << c << "]), w, __ballot_sync(0xffffffffu, in && "
+          << load_val(c) << "), full);\n";
       else
-        b << "  jc_set_bits(P.out_valid[" << cs << "], p, p_first, keep);\n";
+        b << "  if (in) reinterpret_cast<" << ctype(C.dtype) << "*>(P.out_data[" << c << "])[p] = " << load_val(c) << ";\n";
+      b << "  jc_word(P.out_valid[" << c << "], w, __ballot_sync(0xffffffffu, in"
+        << (C.valid ? " && " + load_valid(c) : std::string()) << "), full);\n";
     }
     b << "}\n";
     return b.str();
@@ -1088,23 +1095,66 @@ int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, b
 
 // the top-level filter's compaction (pmb_jit_compact.cuh): device helpers, the parameter block,
 // the generated row functions of the hash skeleton's prefix, the compaction's own parameter block
-// and helpers, its generated row functions, then its kernel
-std::string pmb_jit_compact_source(const CompiledQuery& cq, const JitPlan& J, int n_out) {
+// and helpers, its generated functions, then its kernel
+std::string pmb_jit_compact_source(const CompiledQuery& cq, const JitPlan& J, int n_out, const JitCompactPlan& C) {
   Gen g(cq.dq, J);
   std::string skel(kSkeleton);
   const size_t cut = skel.find("__device__ __forceinline__ long long j_gresolve");
   std::string comp(kCompactSkeleton);
   const size_t kcut = comp.find("extern \"C\" __global__");
-  Gen g2(cq.dq, J);
+  Gen g2(cq.dq, C.J);
   return std::string(kDeviceHeader) + "\n" + skel.substr(0, cut) + "\n" + g.build() + "\n" + comp.substr(0, kcut) +
-         "\n" + g2.compact_funcs(n_out) + "\n" + comp.substr(kcut);
+         "\n" + g2.compact_funcs(n_out, C.tile) + "\n" + comp.substr(kcut);
 }
 
-int pmb_jit_compact_kernel(pmb_handle* h, const CompiledQuery& cq, int n_out, cudaKernel_t* out) {
+// Stage layout of the compaction: 1024 rows, fewer when wide rows would leave an SM with less than
+// four CTAs (a tile's offsets stay multiples of 16 bytes: rows in multiples of 128).
+void pmb_jit_compact_plan(const DQuery& q, JitCompactPlan* C) {
+  memset(C, 0, sizeof(*C));
+  for (C->tile = 1024;; C->tile /= 2) {
+    int off = 0, tx = 0;
+    for (int c = 0; c < q.n_cols; c++) {
+      const int db = q.col[c].elem ? C->tile * q.col[c].elem : C->tile / 8;
+      C->J.doff[c] = off;
+      off += db;
+      tx += db;
+      C->J.voff[c] = -1;
+      if (q.col[c].valid) {
+        C->J.voff[c] = off;
+        off += C->tile / 8;
+        tx += C->tile / 8;
+      }
+    }
+    C->J.buf_bytes = (int)pmb_align((size_t)off, 128);
+    C->J.tx_bytes = tx;
+    C->smem = C->J.buf_bytes;
+    if (C->smem <= 48 << 10 || C->tile == 256) return;
+  }
+}
+
+int pmb_jit_compact_kernel(pmb_handle* h, const CompiledQuery& cq, int n_out, JitCompactPlan* C, cudaKernel_t* out) {
+  static std::mutex sig_mu;
+  static std::unordered_map<std::string, cudaKernel_t> by_sig;
   JitPlan J;
   int rc = pmb_plan_jit_batch(h, cq, 1024, 1, h->max_smem_optin, &J);
   if (rc) return rc;
-  return jit_kernel(h, pmb_jit_compact_source(cq, J, n_out), "pmb_jit_compact", out);
+  pmb_jit_compact_plan(cq.dq, C);
+  std::string sig = hash_signature(cq, J);
+  sig.push_back((char)n_out);
+  {
+    std::lock_guard<std::mutex> lock(sig_mu);
+    auto it = by_sig.find(sig);
+    if (it != by_sig.end()) {
+      *out = it->second;
+      return PMB_OK;
+    }
+  }
+  rc = jit_kernel(h, pmb_jit_compact_source(cq, J, n_out, *C), "pmb_jit_compact", out);
+  if (rc == PMB_OK) {
+    std::lock_guard<std::mutex> lock(sig_mu);
+    by_sig[sig] = *out;
+  }
+  return rc;
 }
 
 int pmb_jit_batch_kernel(pmb_handle* h, const CompiledQuery& cq, const JitPlan& J, cudaKernel_t* out) {
@@ -1150,7 +1200,9 @@ static int debug_compile(const pmb_query* q, const pmb_column* cols, int32_t n_c
       if (rc == PMB_OK) rc = pmb_plan_jit_batch(&h, cq, 1024, 1, 232448, &J);
       if (rc != PMB_OK) msg = h.err;
       std::vector<char> cubin;
-      if (rc == PMB_OK && !jit_compile(pmb_jit_compact_source(cq, J, n_cols), cubin, msg)) rc = PMB_E_UNSUPPORTED;
+      JitCompactPlan C;
+      pmb_jit_compact_plan(cq.dq, &C);
+      if (rc == PMB_OK && !jit_compile(pmb_jit_compact_source(cq, J, n_cols, C), cubin, msg)) rc = PMB_E_UNSUPPORTED;
       else if (rc == PMB_OK && getenv("PMB_JIT_DEBUG") && getenv("PMB_JIT_DEBUG")[0] == '2') fprintf(stderr, "%s\n", msg.c_str());
     } else if (mode == 2) {
       JitPlan J;

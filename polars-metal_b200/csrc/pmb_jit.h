@@ -116,12 +116,20 @@ struct JitCompactParams {
   unsigned char* out_data[16];
   unsigned int* out_valid[16];
 };
-constexpr int JC_TILE_ROWS = 256 * 4;  // rows per tile of pmb_jit_compact (JC_TILE)
+// stage layout of pmb_jit_compact: rows per tile, the columns' offsets in a stage (J.doff, J.voff,
+// J.buf_bytes, J.tx_bytes), dynamic shared memory
+struct JitCompactPlan {
+  JitPlan J;
+  int tile;
+  int smem;
+};
+void pmb_jit_compact_plan(const DQuery& q, JitCompactPlan* C);
+constexpr int JC_THREADS = 256;  // JC_NT
 
 // the top-level filter's compaction of the first n_out columns by the query's predicate
 // (pmb_jit_compact.cuh); the source alone for the compile checks
-std::string pmb_jit_compact_source(const CompiledQuery& cq, const JitPlan& J, int n_out);
-int pmb_jit_compact_kernel(pmb_handle* h, const CompiledQuery& cq, int n_out, cudaKernel_t* out);
+std::string pmb_jit_compact_source(const CompiledQuery& cq, const JitPlan& J, int n_out, const JitCompactPlan& C);
+int pmb_jit_compact_kernel(pmb_handle* h, const CompiledQuery& cq, int n_out, JitCompactPlan* C, cudaKernel_t* out);
 // launches over the global table and key lists set up in P (gkeys, grecs, gcap, status, lists)
 int pmb_jit_launch(pmb_handle* h, cudaKernel_t k, const CompiledQuery& cq, const JitPlan& J, const HashParams& P,
                    int grid, const uint8_t* ttab, int tnb);

@@ -104,6 +104,33 @@ def test_wide_keys(case, n):
         assert_results_match(as_dict(got), want, len(keys), aggs, f"{case} {strategy}")
 
 
+# the staged compaction (PMB_JIT=1: at every size): stage tiles of 1024 rows, 256 with many columns;
+# partial last tiles, more tiles than CTAs, nothing and everything kept, bitmap words shared by tiles
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("n", [1, 31, 255, 256, 257, 1023, 1024, 1025, 5 * 1024 + 3, 1_500_001])
+@pytest.mark.parametrize("share", [0.0, 0.4, 1.0])
+def test_staged_compaction(n, share, wide, monkeypatch):
+    monkeypatch.setenv("PMB_JIT", "1")
+    rng = np.random.default_rng(n)
+    u, uok = rng.random(n), rng.random(n) > (0.0 if share == 1.0 else 0.1)
+    cols = {"u": (u, pack(uok)), "b": (rng.random(n) > 0.5, None), "i8": (rng.integers(-9, 9, n).astype(np.int8), None),
+            "i16": (rng.integers(-9, 9, n).astype(np.int16), rng.random(n) > 0.5), "f": (rng.random(n).astype(np.float32), None)}
+    if wide:
+        cols |= {f"w{i}": (rng.integers(0, 2**60, n), rng.random(n) > 0.2) for i in range(11)}
+    data = {k: N.ColumnData(pack(d), None, dtype=A.BOOL, length=n) if d.dtype == bool else
+            N.ColumnData(d, v if k == "u" or v is None else pack(v)) for k, (d, v) in cols.items()}
+    got = N.filter_columns(data, {"kind": "Compare", "op": "Lt", "lhs": {"kind": "Column", "name": "u"},
+                                  "rhs": {"kind": "LiteralF64", "value": share}})
+    keep = (u < share) & uok
+    m = int(keep.sum())
+    assert got.n_groups == m
+    for i, (k, (d, v)) in enumerate(cols.items()):
+        have = np.unpackbits(got.data[i], bitorder="little")[:m].astype(bool) if d.dtype == bool else got.data[i][:m]
+        assert np.array_equal(have, d[keep]), k
+        ok = np.unpackbits(got.validity[i], bitorder="little")[:m].astype(bool)
+        assert np.array_equal(ok, np.ones(m, bool) if v is None or k == "u" else v[keep]), k
+
+
 # the selector's network in the sampling launch: the same pick and table size as selector_choose,
 # whose features and network run as kernels of their own
 @pytest.mark.parametrize("card,width", [(50, 4), (3000, 4), (90_000, 8), (400_000, 8), (1_500_000, 8)])
