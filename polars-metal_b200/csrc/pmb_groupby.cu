@@ -626,6 +626,33 @@ __global__ void __launch_bounds__(NT, 1) k_hash_agg(const __grid_constant__ Hash
   }
 }
 
+// Rows straight from the columns into the global table, a thread per row: for calls whose keys spread
+// enough that the records' reductions do not queue behind each other (direct_rows). k_hash_agg's CTAs
+// set up and merge a table of their own whatever the input: 126 us for 20K rows, 34 us here; 326 us
+// for 1M rows of 1000 groups, 138 us here.
+template <bool K128>
+__global__ void __launch_bounds__(256, 4) k_hash_direct(const __grid_constant__ HashParams P) {
+  __shared__ __align__(16) DQuery q;  // read with data-dependent indices on every row
+  for (int i = threadIdx.x; i < (int)(sizeof(DQuery) / 4); i += 256)
+    reinterpret_cast<uint32_t*>(&q)[i] = reinterpret_cast<const uint32_t*>(&P.q)[i];
+  __syncthreads();
+  const TileCtx t{nullptr, nullptr, nullptr, 0};
+  const int64_t stride = (int64_t)gridDim.x * 256;
+  for (int64_t r = (int64_t)blockIdx.x * 256 + threadIdx.x; r < q.n_rows; r += stride) {
+    if (!eval_keep(q, t, r)) continue;
+    fx_range_check(q, t, r, P.status);
+    int64_t gi;
+    if (K128) {
+      const Key128 k = pack_key128(q, t, r);
+      gi = gfind128(P, k, pmb_fmix64(k.lo ^ pmb_fmix64(k.hi + 0x9E3779B97F4A7C15ULL)));
+    } else {
+      const uint64_t k = pack_key64(q, t, r);
+      gi = gfind64(P, k, pmb_fmix64(k));
+    }
+    if (gi >= 0) apply_row_global(q, t, P.grecs + (size_t)gi * q.rec_bytes, r);
+  }
+}
+
 // ============================================================================ finalize
 template <int NT, int PER, bool K128>
 __global__ void __launch_bounds__(NT) k_finalize(const __grid_constant__ FinParams F) {
@@ -987,6 +1014,19 @@ int pmb_plan_hash(pmb_handle* h, int max_smem_optin, CompiledQuery& cq, int stra
   return PMB_OK;
 }
 
+// Whether the prebuilt kernels should send every row to the global table (k_hash_direct): the rows of
+// the heaviest key, each with a reduction per record word, are served one after another by one L2
+// slice at about one a nanosecond, so up to 64K of them stay below what k_hash_agg's tables cost.
+static bool direct_rows(const DQuery& q, const SketchOut* sk) {
+  if (!sk || sk->samples <= 0) return false;
+  int top = 0;
+  for (int c = SK_HIST - 1; c > 0 && !top; c--)
+    if (sk->hist[c]) top = c;
+  double rows = (double)top * (double)q.n_rows / (double)sk->samples;
+  if (top >= SK_HIST - 1) rows = (double)q.n_rows;  // the histogram's last bin is open
+  return rows * (q.rec_bytes / 8) <= 65536.0;
+}
+
 int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int strategy, int64_t est,
                      const SketchOut* sk, pmb_result* r, bool est_learned) {
   DQuery& q = cq.dq;
@@ -1004,8 +1044,9 @@ int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int 
     h->err = keep_err;
   }
   pmb_phase(h, "jit");
-  const int hot_cap = jk ? J.hot_cap : P.hot_cap;
-  const int S = jk ? 2 * J.warm_cap : P.smem_slots;
+  const bool direct = !jk && direct_rows(q, sk);
+  const int hot_cap = direct ? 0 : jk ? J.hot_cap : P.hot_cap;
+  const int S = direct ? 0 : jk ? 2 * J.warm_cap : P.smem_slots;
   const int rec = q.rec_bytes;
   Plan pl;
   pl.strategy = (K128 && strategy == PMB_STRATEGY_SMEM_HASH) ? PMB_STRATEGY_GLOBAL_HASH : strategy;
@@ -1139,6 +1180,15 @@ int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int 
     P.kstats = kst;
     int rc;
     if (jk) rc = pmb_jit_launch(h, jk, cq, J, P, h->sm_count, ttab, tnb);
+    else if (direct) {
+      const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, (int64_t)h->sm_count * 4);
+      pmb_kernel_begin(h, "hash_agg");
+      if (K128) k_hash_direct<true><<<blocks, 256, 0, h->stream>>>(P);
+      else k_hash_direct<false><<<blocks, 256, 0, h->stream>>>(P);
+      pmb_kernel_end(h);
+      PMB_CUDA(h, cudaGetLastError());
+      rc = PMB_OK;
+    }
     else if (K128) rc = launch_hash<512, true>(h, P, smem, grid);
     else if (nt == 1024) rc = launch_hash<1024, false>(h, P, smem, grid);
     else if (nt == 256) rc = launch_hash<256, false>(h, P, smem, grid);

@@ -145,3 +145,22 @@ def test_selector_in_the_sampling_launch(card, width):
     assert got.strategy == strategy and got.n_groups == len(np.unique(k))
     if got.rehash_count == 0 and strategy.endswith("hash"):
         assert min(max(2 * groups, 1024), 2 * n) <= got.capacity <= max(3 * groups, 1024) + 3  # slots per estimated group
+
+
+# rows straight into the global table: block edges, one- and two-word keys that do not pack, and the
+# rule's other side (a key with too many rows for it)
+@pytest.mark.parametrize("wide", [False, True])
+@pytest.mark.parametrize("groups", [1, 3, 900])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 30_000])
+def test_direct_rows(n, groups, wide):
+    rng = np.random.default_rng(n + groups)
+    k = rng.integers(0, groups, n)
+    cols = {"k": (np.where(k % 2 == 0, k, -k) * (2**52 if wide else 1), pack(rng.random(n) > 0.1)),
+            "v": (rng.standard_normal(n).astype(np.float32), pack(rng.random(n) > 0.2)), "x": (rng.integers(-9, 9, n), None)}
+    if wide:
+        cols["j"] = (rng.integers(0, 2, n) * (2**63 - 1), None)
+    keys = ["k", "j"] if wide else ["k"]
+    aggs = [("Sum", "v", "s"), ("Min", "v", "lo"), ("Max", "x", "hi"), ("Count", "v", "c"), ("Len", None, "l")]
+    pred = {"kind": "Compare", "op": "Ne", "lhs": {"kind": "Column", "name": "x"}, "rhs": {"kind": "LiteralI64", "value": 3}}
+    got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, keys, aggs, pred)
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, pred), len(keys), aggs)
