@@ -970,6 +970,15 @@ static int jit_kernel(pmb_handle* h, const std::string& src, const char* name, c
   return PMB_OK;
 }
 
+bool pmb_jit_check(const std::string& src, std::string* log) {
+  std::vector<char> cubin;
+  return jit_compile(src, cubin, *log);
+}
+
+int pmb_jit_plain_kernel(pmb_handle* h, const std::string& src, const char* name, cudaKernel_t* out) {
+  return jit_kernel(h, src, name, out);
+}
+
 // The signature of a hash kernel as bytes: the query descriptor without what only the launch
 // parameters carry (buffer addresses, row count, fixed-point widths and ranges; only whether a
 // column has a validity bitmap reaches the source), the launch plan, and the skeleton's origin.

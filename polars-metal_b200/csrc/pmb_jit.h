@@ -58,6 +58,11 @@ void pmb_jit_slayout(const DQuery& q, JitSLayout* S);
 
 int pmb_plan_jit(pmb_handle* h, const CompiledQuery& cq, bool have_sketch, int max_smem_optin, JitPlan* J);
 
+// kernel `name` of a self-contained source text, compiled once per text; PMB_E_UNSUPPORTED when the
+// run-time compiler is unavailable
+int pmb_jit_plain_kernel(pmb_handle* h, const std::string& src, const char* name, cudaKernel_t* out);
+// compiles a source text without a GPU; false with the compiler's log
+bool pmb_jit_check(const std::string& src, std::string* log);
 // JIT policy: PMB_JIT=0 never, PMB_JIT=1 always, otherwise inputs of at least 2M rows
 bool pmb_jit_enabled(int64_t n_rows);
 // compiled kernel for this signature and layout (cached); PMB_E_UNSUPPORTED when unavailable

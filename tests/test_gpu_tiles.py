@@ -147,6 +147,57 @@ def test_selector_in_the_sampling_launch(card, width):
         assert min(max(2 * groups, 1024), 2 * n) <= got.capacity <= max(3 * groups, 1024) + 3  # slots per estimated group
 
 
+# expressions: tails of a thread's four rows and of a bitmap word, flat and deep trees, an output that
+# overlaps an input (computed aside, then copied)
+@pytest.mark.parametrize("jit", ["0", "1"])  # the interpreter, the run-time compiled kernel
+@pytest.mark.parametrize("n", [1, 7, 31, 32, 33, 127, 128, 129, 1025, 100_003])
+def test_expression_rows(n, jit, monkeypatch):
+    import torch
+
+    monkeypatch.setenv("PMB_JIT", jit)
+
+    rng = np.random.default_rng(n)
+    a, b = rng.standard_normal(n), rng.integers(-9, 9, n).astype(np.int32)
+    ok = rng.random(n) > 0.3
+    A_, B_ = {"kind": "Column", "name": "a"}, {"kind": "Column", "name": "b"}
+    flat = {"kind": "Binary", "op": "Mul", "lhs": A_, "rhs": {"kind": "Binary", "op": "Sub", "lhs": B_, "rhs": A_}}
+    deep = A_
+    for _ in range(6):  # right-nested: seven entries on the stack
+        deep = {"kind": "Binary", "op": "Add", "lhs": B_, "rhs": deep}
+    want_deep = a.copy()
+    for _ in range(6):
+        want_deep = b + want_deep
+    for e, want in ((flat, a * (b - a)), (deep, want_deep)):
+        for dev in (False, True):
+            cols = {"a": N.ColumnData(torch.from_numpy(a).cuda() if dev else a,
+                                      torch.from_numpy(pack(ok)).cuda() if dev else pack(ok)),
+                    "b": N.ColumnData(torch.from_numpy(b).cuda() if dev else b)}
+            got = N.eval_expr(cols, e)
+            data = got.data.cpu().numpy() if dev else got.data
+            valid = got.validity.cpu().numpy() if dev else got.validity
+            assert np.array_equal(np.unpackbits(valid, bitorder="little")[:n].astype(bool), ok)
+            assert np.array_equal(data[:n][ok], want[ok])
+
+
+def test_expression_in_place():
+    import ctypes as C
+
+    import torch
+
+    n = 5000
+    x = torch.randn(n + 1, dtype=torch.float64, device="cuda")
+    want = (x[:n] + x[:n]).cpu().numpy()
+    cols = {"x": N.ColumnData(x[:n])}
+    abi, _keep = N._to_abi_columns(list(cols.values()))
+    e, _k = N.compile_predicate({"kind": "Arith", "op": "Add", "lhs": {"kind": "Column", "name": "x"},
+                                 "rhs": {"kind": "Column", "name": "x"}}, {"x": 0})
+    valid = torch.zeros(N._bitmap_bytes(n), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    h, dt = N.default_handle(), C.c_int32()
+    h.check(h._lib.pmb_eval_expr(h.raw, C.byref(e), abi, 1, x[1:].data_ptr(), valid.data_ptr(), 1, C.byref(dt)))
+    assert np.array_equal(x[1:].cpu().numpy(), want)
+
+
 # rows straight into the global table: block edges, one- and two-word keys that do not pack, and the
 # rule's other side (a key with too many rows for it)
 @pytest.mark.parametrize("wide", [False, True])
@@ -158,7 +209,7 @@ def test_direct_rows(n, groups, wide):
     cols = {"k": (np.where(k % 2 == 0, k, -k) * (2**52 if wide else 1), pack(rng.random(n) > 0.1)),
             "v": (rng.standard_normal(n).astype(np.float32), pack(rng.random(n) > 0.2)), "x": (rng.integers(-9, 9, n), None)}
     if wide:
-        cols["j"] = (rng.integers(0, 2, n) * (2**63 - 1), None)
+        cols["j"] = ((rng.integers(0, 2, n) * (2**31 - 1)).astype(np.int32), None)
     keys = ["k", "j"] if wide else ["k"]
     aggs = [("Sum", "v", "s"), ("Min", "v", "lo"), ("Max", "x", "hi"), ("Count", "v", "c"), ("Len", None, "l")]
     pred = {"kind": "Compare", "op": "Ne", "lhs": {"kind": "Column", "name": "x"}, "rhs": {"kind": "LiteralI64", "value": 3}}
