@@ -162,6 +162,8 @@ struct KernelTiming {
   cudaEvent_t start, stop;
 };
 
+struct pmb_h2d_pool;  // threads that stage pageable host columns (pmb_runtime.cu)
+
 struct pmb_handle {
   int device = 0;
   cudaStream_t own_stream = nullptr;
@@ -184,6 +186,8 @@ struct pmb_handle {
   uint8_t* hstage = nullptr;
   size_t hstage_cap = 0, hstage_used = 0, hstage_want = 0;
   uint8_t* rstage = nullptr;  // pinned staging of small results (pmb_finish_outputs), allocated at first use
+  pmb_h2d_pool* h2d_pool = nullptr;
+  bool h2d_pool_failed = false;
   // profiling
   bool profiling = false;
   bool batching = true;  // pmb_groupby_batched may batch (else: one pmb_groupby per query)

@@ -198,6 +198,21 @@ def test_expression_in_place():
     assert np.array_equal(x[1:].cpu().numpy(), want)
 
 
+# pageable columns staged by several threads: sizes around the pool's smallest copy and its chunks,
+# bitmaps at a bit offset, several columns in a row through the same chunks
+@pytest.mark.parametrize("n", [524_287, 524_288, 655_361, 4_000_003])
+def test_pageable_columns(n):
+    rng = np.random.default_rng(n)
+    k, x = rng.integers(0, 5, n + 3), rng.integers(-2**40, 2**40, n + 3)
+    ok = rng.random(n + 3) > 0.25
+    big = pack(np.tile(ok, 1))
+    cols = {"k": N.ColumnData(k, None, offset=3, length=n), "x": N.ColumnData(x, big, offset=3, length=n)}
+    got = as_dict(N.groupby(cols, ["k"], [("Sum", "x", "s"), ("Count", "x", "c")], sort={"by": "k"}))
+    kk, xx, oo = k[3:], x[3:], ok[3:]
+    assert np.array_equal(got["data"][1][:5], [xx[(kk == i) & oo].sum() for i in range(5)])
+    assert np.array_equal(got["data"][2][:5], [((kk == i) & oo).sum() for i in range(5)])
+
+
 # rows straight into the global table: block edges, one- and two-word keys that do not pack, and the
 # rule's other side (a key with too many rows for it)
 @pytest.mark.parametrize("wide", [False, True])
