@@ -1281,6 +1281,7 @@ int recompile_dd(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int3
     nc.dq.col[c].valid = cq.dq.col[c].valid;
   }
   nc.ranges = cq.ranges;
+  nc.order = cq.order;
   if (cq.dq.packed) pmb_apply_packed_keys(nc);
   cq = nc;
   return PMB_OK;
@@ -1288,6 +1289,13 @@ int recompile_dd(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int3
 
 extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
                            pmb_result** out) {
+  bool ordered;
+  return pmb_groupby_call(h, q, cols, n_cols, nullptr, &ordered, out);
+}
+
+int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
+                     const pmb_sort_spec* spec, bool* ordered, pmb_result** out) {
+  *ordered = false;
   if (!h) return PMB_E_INVALID;
   if (!out) return pmb_fail(h, PMB_E_INVALID, "out is NULL");
   *out = nullptr;
@@ -1297,6 +1305,7 @@ extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* 
   CompiledQuery cq;
   int rc = pmb_compile_groupby(h, q, cols, n_cols, &cq);
   if (rc) return rc;
+  cq.order = spec;
   rc = pmb_ws_begin(h);
   if (rc) return rc;
   pmb_call_begin(h);
@@ -1383,6 +1392,7 @@ extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* 
     break;
   }
   pmb_phase(h, "strategy");
+  *ordered = cq.ordered;
   rc = pmb_finish_outputs(h, r, q->output_on_device == 0);
   if (rc) return bail(rc);
   PMB_CUDA(h, cudaStreamSynchronize(h->stream));

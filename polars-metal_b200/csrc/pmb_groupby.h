@@ -114,6 +114,10 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
 // output sort (pmb_order.cu): the n rows of the device columns in the order of the spec, the first
 // `limit` of them, as device columns of r (r->n_groups set); the workspace is not reset
 int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, const pmb_sort_spec& s, pmb_result* r);
+// pmb_groupby, told the order its result will be sorted in (null: none); *ordered: the result's rows
+// already are the sorted slice
+int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
+                     const pmb_sort_spec* spec, bool* ordered, pmb_result** out);
 // learned selector (pmb_learned.cu): strategy and group count for AUTO; false when no selector is
 // installed or its output is unusable
 bool pmb_selector_pick(pmb_handle* h, const CompiledQuery& cq, int* strategy, int64_t* groups);

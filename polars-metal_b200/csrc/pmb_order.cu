@@ -768,8 +768,20 @@ extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_c
   pmb_query qd = *q;
   qd.output_on_device = 1;
   pmb_result* g = nullptr;
-  int rc = pmb_groupby(h, &qd, cols, n_cols, &g);
+  bool ordered = false;
+  int rc = pmb_groupby_call(h, &qd, cols, n_cols, spec, &ordered, &g);
   if (rc) return rc;
+  if (ordered) {
+    rc = pmb_finish_outputs(h, g, q->output_on_device == 0);
+    if (rc) {
+      pmb_result_free(g);
+      return rc;
+    }
+    PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+    pmb_call_end(h);
+    *out = g;
+    return PMB_OK;
+  }
   // the group-by's device columns stay in the workspace; the sort's buffers follow them (no
   // workspace reset), and its launches add to the same call's statistics
   DCol d[PMB_MAX_OUT];

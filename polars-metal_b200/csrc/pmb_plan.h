@@ -24,6 +24,10 @@ struct CompiledQuery {
   // caller's columns whose float sums use double-double accumulation instead of the exact
   // fixed point (kept by pmb_compile_groupby; see PMB_FX_MIN_F)
   std::vector<int> dd_user_cols;
+  // the output order the caller wants next (null: none): a strategy that can leave its groups in
+  // that order, sliced, does so and sets `ordered`
+  const pmb_sort_spec* order = nullptr;
+  bool ordered = false;
   // ranges of the key columns' values over all rows, as order-preserving integers (have: read)
   struct KeyRanges {
     bool have = false;

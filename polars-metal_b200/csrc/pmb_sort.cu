@@ -1009,6 +1009,176 @@ __global__ void __launch_bounds__(ST_NT) k_part_finalize(const __grid_constant__
   }
 }
 
+// ---------------------------------------------------------------- dense groups in a wanted order
+// A group-by whose result is then sorted by its keys: the dense groups' packed keys are rearranged
+// into order keys (the sort columns' fields, most significant highest, then the other keys), sorted
+// with the group numbers, and the records finalised in that order. A group is one contiguous record
+// until then, so following the order costs two or three sectors a group; sorting the finished
+// columns gathered one random 32-byte sector per group and column (49M groups of 9 columns:
+// finalise 2.0 ms and gather 8.7 ms, 6.8 ms here), and needed the ranges and encode passes again.
+struct GroupOrder {
+  SortKeyLayout L;  // the packed keys' fields
+  int null_off[PMB_MAX_KEYS];  // per key column, its fields in the order key (null_off -1: none)
+  int data_off[PMB_MAX_KEYS];
+  int desc[PMB_MAX_KEYS];
+  int nulls_last[PMB_MAX_KEYS];
+};
+
+template <int W>
+__device__ __forceinline__ unsigned long long key_field(const PKey<W>& k, int off, int bits) {
+  if (bits == 0) return 0ULL;
+  const int wi = off >> 6, sh = off & 63;
+  unsigned long long v = k.w[wi] >> sh;
+  if (W > 1 && sh + bits > 64 && wi + 1 < W) v |= k.w[wi + 1] << (64 - sh);
+  return bits == 64 ? v : (v & ((1ULL << bits) - 1ULL));
+}
+template <int W>
+__device__ __forceinline__ void put_field(PKey<W>& k, int off, unsigned long long v, int bits) {
+  if (bits == 0) return;
+  const int wi = off >> 6, sh = off & 63;
+  k.w[wi] |= v << sh;
+  if (W > 1 && sh + bits > 64 && wi + 1 < W) k.w[wi + 1] |= v >> (64 - sh);
+}
+__device__ __forceinline__ unsigned long long field_max(int bits) {
+  return bits == 0 ? 0ULL : ~0ULL >> (64 - bits);
+}
+
+template <int W>
+__global__ void __launch_bounds__(ST_NT) k_group_order(const __grid_constant__ GroupOrder O,
+                                                       const unsigned long long* gkeys, uint64_t gcap, int64_t ng,
+                                                       unsigned long long* okeys, uint64_t ocap, unsigned int* idx,
+                                                       int passes, unsigned int* hist) {
+  __shared__ unsigned int s_hist[MAX_PASSES * RADIX];
+  for (int i = threadIdx.x; i < passes * RADIX; i += ST_NT) s_hist[i] = 0u;
+  __syncthreads();
+  const int64_t stride = (int64_t)gridDim.x * ST_NT;
+  for (int64_t g = (int64_t)blockIdx.x * ST_NT + threadIdx.x; g < ng; g += stride) {
+    PKey<W> k, o;
+    for (int w = 0; w < W; w++) {
+      k.w[w] = gkeys[(uint64_t)w * gcap + g];
+      o.w[w] = 0ULL;
+    }
+    for (int c = 0; c < O.L.n_keys; c++) {
+      const bool null = O.L.null_off[c] >= 0 && key_field<W>(k, O.L.null_off[c], 1) != 0;
+      if (O.null_off[c] >= 0) put_field<W>(o, O.null_off[c], null == (O.nulls_last[c] != 0) ? 1ULL : 0ULL, 1);
+      if (null) continue;
+      const unsigned long long v = key_field<W>(k, O.L.data_off[c], O.L.data_bits[c]);
+      put_field<W>(o, O.data_off[c], O.desc[c] ? field_max(O.L.data_bits[c]) - v : v, O.L.data_bits[c]);
+    }
+    for (int w = 0; w < W; w++) okeys[(uint64_t)w * ocap + g] = o.w[w];
+    idx[g] = (unsigned)g;
+    for (int p = 0; p < passes; p++) atomicAdd(&s_hist[p * RADIX + digit_of<W>(o, 8 * p)], 1u);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * RADIX; i += ST_NT) {
+    const unsigned v = s_hist[i];
+    if (v) atomicAdd(&hist[i], v);
+  }
+}
+
+// output rows 0 .. m-1 = the groups at positions start .. start + m - 1 of the order
+template <int W>
+__global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constant__ PartFinParams F,
+                                                            const __grid_constant__ GroupOrder O,
+                                                            const unsigned long long* okeys, uint64_t ocap,
+                                                            const unsigned int* idx, int64_t start, int64_t m) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  // every lane of a warp runs the same number of iterations (warp-wide bit setting)
+  const int64_t span = (m + stride - 1) / stride * stride;
+  for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x; p0 < span; p0 += stride) {
+    const int64_t p = p0 + threadIdx.x;
+    const bool have = p < m;
+    PKey<W> k{}, o{};
+    const uint8_t* rec = nullptr;
+    if (have) {
+      rec = F.grecs + (uint64_t)idx[start + p] * F.R.q.rec_bytes;
+      for (int w = 0; w < W; w++) o.w[w] = okeys[(uint64_t)w * ocap + start + p];
+      for (int c = 0; c < O.L.n_keys; c++) {  // the packed key back from the order key
+        const bool null = O.null_off[c] >= 0 && (key_field<W>(o, O.null_off[c], 1) != 0) == (O.nulls_last[c] != 0);
+        if (null) {
+          put_field<W>(k, O.L.null_off[c], 1ULL, 1);
+          continue;
+        }
+        const unsigned long long v = key_field<W>(o, O.data_off[c], O.L.data_bits[c]);
+        put_field<W>(k, O.L.data_off[c], O.desc[c] ? field_max(O.L.data_bits[c]) - v : v, O.L.data_bits[c]);
+      }
+    }
+    write_group<W, true>(F.R, p, p0 + (threadIdx.x & ~31), have, k, rec);
+  }
+}
+
+// whether the order names key columns only, each once (then the groups' packed keys decide it)
+bool ordered_by_keys(const CompiledQuery& cq, const SortKeyLayout& L) {
+  const pmb_sort_spec* s = cq.order;
+  if (!s || !s->by || s->n_by < 1 || s->n_by > L.n_keys) return false;
+  unsigned seen = 0;
+  for (int i = 0; i < s->n_by; i++) {
+    const int c = s->by[i];
+    if (c < 0 || c >= L.n_keys || ((seen >> c) & 1u)) return false;
+    if (pmb_is_float(L.dtype[c])) return false;  // packed as raw bits, which do not order
+    seen |= 1u << c;
+  }
+  return !(s->drop_nulls && L.null_off[s->by[0]] >= 0);
+}
+
+template <int W>
+int ordered_finalize(pmb_handle* h, const CompiledQuery& cq, const PartFinParams& F, int64_t ng, int64_t* rows) {
+  const pmb_sort_spec& s = *cq.order;
+  GroupOrder O;
+  memset(&O, 0, sizeof(O));
+  O.L = F.R.L;
+  const int nk = O.L.n_keys;
+  // fields from the least significant up: the keys the order does not name, then its columns backwards
+  std::vector<int> cols;
+  for (int c = 0; c < nk; c++) {
+    bool named = false;
+    for (int i = 0; i < s.n_by; i++) named |= s.by[i] == c;
+    if (!named) cols.push_back(c);
+  }
+  for (int i = s.n_by - 1; i >= 0; i--) {
+    cols.push_back(s.by[i]);
+    O.desc[s.by[i]] = s.descending && s.descending[i];
+    O.nulls_last[s.by[i]] = s.nulls_last && s.nulls_last[i];
+  }
+  int off = 0;
+  for (int c : cols) {
+    O.data_off[c] = off;
+    off += O.L.data_bits[c];
+    O.null_off[c] = O.L.null_off[c] >= 0 ? off : -1;
+    off += O.L.null_off[c] >= 0;
+  }
+  const int passes = (off + 7) / 8;
+  const uint64_t ocap = (uint64_t)ng;
+  unsigned long long* k0 = (unsigned long long*)pmb_ws_alloc(h, (size_t)W * ng * 8 + 16);
+  unsigned long long* k1 = (unsigned long long*)pmb_ws_alloc(h, (size_t)W * ng * 8 + 16);
+  unsigned int* i0 = (unsigned int*)pmb_ws_alloc(h, (size_t)ng * 4 + 16);
+  unsigned int* i1 = (unsigned int*)pmb_ws_alloc(h, (size_t)ng * 4 + 16);
+  unsigned int* hist = (unsigned int*)pmb_ws_alloc(h, (size_t)MAX_PASSES * RADIX * 4);
+  if (!k0 || !k1 || !i0 || !i1 || !hist) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (group order)");
+  PMB_CUDA(h, cudaMemsetAsync(hist, 0, (size_t)MAX_PASSES * RADIX * 4, h->stream));
+  const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((ng + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 8));
+  pmb_kernel_begin(h, "group_order");
+  k_group_order<W><<<blocks, ST_NT, 0, h->stream>>>(O, F.gkeys, F.gcap, ng, k0, ocap, i0, passes, hist);
+  pmb_kernel_end(h);
+  PMB_CUDA(h, cudaGetLastError());
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
+  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+  std::vector<unsigned int> hh((const unsigned int*)h->pinned, (const unsigned int*)h->pinned + (size_t)passes * RADIX);
+  const int rc = pmb_sort_pairs(h, W, &k0, &k1, &i0, &i1, ocap, ng, passes, hist, hh.data());
+  if (rc) return rc;
+  const int64_t start = s.offset >= 0 ? std::min<int64_t>(s.offset, ng) : std::max<int64_t>(0, ng + s.offset);
+  const int64_t m = s.limit < 0 ? ng - start : std::min<int64_t>(s.limit, ng - start);
+  if (m > 0) {
+    const int fb = (int)std::max<int64_t>(1, std::min<int64_t>((m + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
+    pmb_kernel_begin(h, "ordered_finalize");
+    k_ordered_finalize<W><<<fb, ST_NT, 0, h->stream>>>(F, O, k0, ocap, i0, start, m);
+    pmb_kernel_end(h);
+    PMB_CUDA(h, cudaGetLastError());
+  }
+  *rows = m;
+  return PMB_OK;
+}
+
 // the per-thread stage of k_part_agg: the aggregated columns' values (widest first, each aligned
 // to its size), then one validity byte per nullable column; returns its bytes (a multiple of 8)
 static int pa_stage(const DQuery& q, unsigned* used, int32_t* sdoff, int32_t* svoff) {
@@ -1210,11 +1380,19 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         F.gkeys = gkeys;
         F.grecs = grecs;
         F.gcap = (uint64_t)out_cap;
-        const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)ng + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
+        if (ordered_by_keys(cq, L)) {
+          int64_t rows = 0;
+          const int orc = ordered_finalize<W>(h, cq, F, (int64_t)ng, &rows);
+          if (orc) return orc;
+          ng = (unsigned long long)rows;
+          cq.ordered = true;
+        } else {
+          const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)ng + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
         pmb_kernel_begin(h, "part_finalize");
         k_part_finalize<W><<<blocks, ST_NT, 0, h->stream>>>(F);
         pmb_kernel_end(h);
         PMB_CUDA(h, cudaGetLastError());
+        }
       }
     }
     if (st[0] & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (partitioned)");

@@ -213,6 +213,52 @@ def test_pageable_columns(n):
     assert np.array_equal(got["data"][2][:5], [((kk == i) & oo).sum() for i in range(5)])
 
 
+# groups left in the wanted order by the partitioned and the sort strategy: directions, null places,
+# some of the keys, slices, one- and two-word keys, one group
+ORDERS = [({"by": ["j", "k"]}, None), ({"by": ["k"], "descending": True, "offset": 5, "limit": 1000}, None),
+          ({"by": ["k", "j"], "descending": [True, False], "nulls_last": [True, False], "offset": -900}, None),
+          ({"by": ["j", "k"], "nulls_last": True, "drop_nulls": True, "limit": 50}, None),
+          ({"by": ["k", "s"]}, None)]
+
+
+@pytest.mark.parametrize("strategy", ["partitioned", "sort"])
+@pytest.mark.parametrize("order", [o for o, _ in ORDERS], ids=lambda o: "-".join(map(str, o.values())))
+@pytest.mark.parametrize("kind", ["narrow", "wide", "one"])
+def test_ordered_groups(kind, order, strategy):
+    rng = np.random.default_rng(len(kind))
+    n = 120_000
+    k = rng.integers(0, 3000, n) if kind != "one" else np.full(n, 7)
+    k = np.where(k % 2 == 0, k, -k) * (3_000_000_000_000_000 if kind == "wide" else 1)
+    j = rng.integers(-20, 20, n).astype(np.int16) if kind != "one" else np.full(n, -3, np.int16)
+    w = (rng.integers(0, 2, n) * 2**30 if kind == "wide" else np.zeros(n)).astype(np.int32)
+    ok = np.ones(n, bool) if kind == "one" else rng.random(n) > 0.02
+    v = rng.standard_normal(n)
+    cols = {"k": (k, None), "j": (j, pack(ok)), "w": (w, None), "v": (v, None)}
+    data = {name: N.ColumnData(*c) for name, c in cols.items()}
+    aggs = [("Min", "v", "s"), ("Len", None, "c")]
+    keys = ["k", "j", "w"]
+    want = pyoracle.groupby(cols, keys, aggs, None)
+    # a total order: the other keys behind the wanted ones settle its ties
+    got = as_dict(N.groupby(data, keys, aggs, strategy=strategy, sort=order))
+    table = {nm: (d, va, dt, want["n_groups"]) for nm, d, va, dt in zip(want["names"], want["data"], want["validity"],
+                                                                       want["dtypes"])}
+    by = order["by"]
+    flags = lambda x: [bool(x)] * len(by) if isinstance(x, bool) else list(x)  # noqa: E731
+    full = pyoracle.sort_table(table, by, flags(order.get("descending", False)), flags(order.get("nulls_last", False)),
+                               order.get("drop_nulls", False), order.get("offset", 0),
+                               -1 if order.get("limit") is None else order["limit"])
+    assert int(got["n_groups"]) == int(full["n_groups"])
+    m = int(full["n_groups"])
+    for name in by:
+        i = keys.index(name) if name in keys else len(keys)
+        g_ok = np.unpackbits(np.asarray(got["validity"][i], np.uint8), bitorder="little")[:m].astype(bool)
+        f_ok = np.unpackbits(np.asarray(full["validity"][i], np.uint8), bitorder="little")[:m].astype(bool)
+        assert np.array_equal(g_ok, f_ok), name
+        assert np.array_equal(np.asarray(got["data"][i])[:m][f_ok], np.asarray(full["data"][i])[:m][f_ok]), name
+    if not order.get("offset") and order.get("limit") is None:
+        assert_results_match(got, want, len(keys), aggs, strategy)
+
+
 # rows straight into the global table: block edges, one- and two-word keys that do not pack, and the
 # rule's other side (a key with too many rows for it)
 @pytest.mark.parametrize("wide", [False, True])
