@@ -1080,8 +1080,8 @@ __global__ void __launch_bounds__(ST_NT) k_group_order(const __grid_constant__ G
 template <int W>
 __global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constant__ PartFinParams F,
                                                             const __grid_constant__ GroupOrder O,
-                                                            const unsigned long long* okeys, uint64_t ocap,
-                                                            const unsigned int* idx, int64_t start, int64_t m) {
+                                                            const unsigned long long* okeys, const unsigned int* idx,
+                                                            int64_t start, int64_t m) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   // every lane of a warp runs the same number of iterations (warp-wide bit setting)
   const int64_t span = (m + stride - 1) / stride * stride;
@@ -1091,9 +1091,12 @@ __global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constan
     PKey<W> k{}, o{};
     const uint8_t* rec = nullptr;
     if (have) {
-      rec = F.grecs + (uint64_t)idx[start + p] * F.R.q.rec_bytes;
-      for (int w = 0; w < W; w++) o.w[w] = okeys[(uint64_t)w * ocap + start + p];
-      for (int c = 0; c < O.L.n_keys; c++) {  // the packed key back from the order key
+      const uint64_t g = idx[start + p];
+      rec = F.grecs + g * F.R.q.rec_bytes;
+      // one-word keys: the packed key back from the sorted order key (read in sequence); two-word
+      // order keys are not sorted whole, the group's own packed key is fetched
+      for (int w = 0; w < W; w++) (W == 1 ? o : k).w[w] = W == 1 ? okeys[start + p] : F.gkeys[(uint64_t)w * F.gcap + g];
+      for (int c = 0; W == 1 && c < O.L.n_keys; c++) {
         const bool null = O.null_off[c] >= 0 && (key_field<W>(o, O.null_off[c], 1) != 0) == (O.nulls_last[c] != 0);
         if (null) {
           put_field<W>(k, O.L.null_off[c], 1ULL, 1);
@@ -1171,7 +1174,7 @@ int ordered_finalize(pmb_handle* h, const CompiledQuery& cq, const PartFinParams
   if (m > 0) {
     const int fb = (int)std::max<int64_t>(1, std::min<int64_t>((m + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
     pmb_kernel_begin(h, "ordered_finalize");
-    k_ordered_finalize<W><<<fb, ST_NT, 0, h->stream>>>(F, O, k0, ocap, i0, start, m);
+    k_ordered_finalize<W><<<fb, ST_NT, 0, h->stream>>>(F, O, k0, i0, start, m);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
   }
@@ -1779,63 +1782,97 @@ int pmb_pack_wide_keys(pmb_handle* h, CompiledQuery& cq) {
   return PMB_OK;
 }
 
-// Stable LSD sort of (key, row index) pairs for callers outside the group-by (the output sort):
-// the same onesweep pass kernel, over the 8-bit digits 0 .. n_passes-1 of W-word keys (word-major,
-// stride cap). hist_host holds every pass's digit counts of all n keys (also at hist_dev); a digit
-// that one value fills is skipped. On return *k and *i are the sorted buffers (the inputs or the
-// alternates).
+// dst[i] = src[idx[i]], four rows of a thread in flight
+__global__ void __launch_bounds__(ST_NT) k_gather_word(const unsigned long long* __restrict__ src,
+                                                       const unsigned int* __restrict__ idx, int64_t n,
+                                                       unsigned long long* __restrict__ dst) {
+  const int64_t stride = (int64_t)gridDim.x * ST_NT;
+  for (int64_t i0 = (int64_t)blockIdx.x * ST_NT + threadIdx.x; i0 < n; i0 += 4 * stride) {
+    unsigned long long v[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = i0 + u * stride < n ? src[idx[i0 + u * stride]] : 0ULL;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (i0 + u * stride < n) dst[i0 + u * stride] = v[u];
+  }
+}
+
+// Stable LSD sort of (key, row index) pairs for callers outside the group-by's own sort: the onesweep
+// pass kernel over the 8-bit digits 0 .. n_passes-1 of W-word keys (word-major, stride cap).
+// hist_host holds every pass's digit counts of all n keys (also at hist_dev); a digit that one value
+// fills is skipped. On return *i is the order and, for one-word keys, *k the sorted keys (the inputs
+// or the alternates). Two-word keys are sorted a word at a time, the second word fetched in the order
+// of the first: a pass over 12-byte pairs takes half the time of one over 20-byte pairs (20M rows: 159
+// against 316 us), the fetch less than one pass; their sorted keys are not returned. The second words
+// are stored by row number; `permuted`: *i is not 0, 1, 2, ... already on entry.
 int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long long** k_alt, unsigned int** i,
                    unsigned int** i_alt, uint64_t cap, int64_t n, int n_passes, const unsigned int* hist_dev,
-                   const unsigned int* hist_host) {
+                   const unsigned int* hist_host, bool permuted) {
   if (W != 1 && W != 2) return pmb_fail(h, PMB_E_INVALID, "sort: key of 1 or 2 words");
   if (n_passes > MAX_PASSES) return pmb_fail(h, PMB_E_INVALID, "sort: more than 16 digit passes");
   if (n <= 1 || n_passes <= 0) return PMB_OK;
-  const int tile = W == 1 ? PassShape<1>::TILE : PassShape<2>::TILE;
-  const int64_t tiles = (n + tile - 1) / tile;
-  unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(h, (size_t)tiles * RADIX * 8);
-  unsigned long long* ticket = (unsigned long long*)pmb_ws_alloc(h, 64);
+  const int64_t tiles = (n + PassShape<1>::TILE - 1) / PassShape<1>::TILE;
+  const size_t lb_bytes = (size_t)tiles * RADIX * 8;
+  // look-back states, then the ticket (cleared together), then status
+  unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(h, lb_bytes + 64);
   unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
   unsigned int* gstart = (unsigned int*)pmb_ws_alloc(h, (size_t)n_passes * RADIX * 4);
-  if (!lb || !ticket || !status || !gstart) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
+  if (!lb || !status || !gstart) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
   PMB_CUDA(h, cudaMemsetAsync(status, 0, 64, h->stream));
-  if (W == 1)
-    PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
-  else
-    PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<2>::SMEM));
+  PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
   pmb_kernel_begin(h, "digit_starts");
   k_digit_starts<<<n_passes, RADIX, 0, h->stream>>>(hist_dev, gstart);
   pmb_kernel_end(h);
   PMB_CUDA(h, cudaGetLastError());
+  unsigned long long* a = *k;       // the current word's keys, and where the next pass writes them
+  unsigned long long* b = *k_alt;
+  bool moved = permuted;            // the order differs from the rows'
   for (int p = 0; p < n_passes; p++) {
+    if (p == 8) {
+      a = *k + cap;
+      b = *k_alt + cap;
+    }
     bool constant = false;
     for (int d = 0; d < RADIX; d++) constant |= hist_host[(size_t)p * RADIX + d] == (unsigned)n;
     if (constant) continue;
+    if (p >= 8 && moved) {  // the second word in the order so far, once
+      const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 4 * ST_NT - 1) / (4 * ST_NT), (int64_t)h->sm_count * 8));
+      pmb_kernel_begin(h, "sort_fetch");
+      k_gather_word<<<blocks, ST_NT, 0, h->stream>>>(a, *i, n, b);
+      pmb_kernel_end(h);
+      PMB_CUDA(h, cudaGetLastError());
+      std::swap(a, b);
+      moved = false;
+    }
     PassParams P;
-    P.kin = *k;
-    P.kout = *k_alt;
+    P.kin = a;
+    P.kout = b;
     P.iin = *i;
     P.iout = *i_alt;
     P.cap = cap;
     P.n = n;
-    P.shift = 8 * p;
+    P.shift = 8 * (p & 7);
     P.hashed = 0;
     P.gstart = gstart + (size_t)p * RADIX;
     P.lb = lb;
-    P.ticket = ticket;
+    P.ticket = lb + (size_t)tiles * RADIX;
     P.status = status;
-    PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)tiles * RADIX * 8, h->stream));
-    PMB_CUDA(h, cudaMemsetAsync(ticket, 0, 8, h->stream));
+    PMB_CUDA(h, cudaMemsetAsync(lb, 0, lb_bytes + 64, h->stream));
     pmb_kernel_begin(h, "sort_pass");
-    if (W == 1) k_sort_pass<1><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
-    else k_sort_pass<2><<<(unsigned)tiles, PassShape<2>::NT, PassShape<2>::SMEM, h->stream>>>(P);
+    k_sort_pass<1><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
-    std::swap(*k, *k_alt);
+    std::swap(a, b);
     std::swap(*i, *i_alt);
+    if (p < 8) moved = true;
   }
-  unsigned int st = 0;
-  PMB_CUDA(h, cudaMemcpyAsync(&st, status, 4, cudaMemcpyDeviceToHost, h->stream));
+  if (W == 1) {
+    *k = a;
+    *k_alt = b;
+  }
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, status, 4, cudaMemcpyDeviceToHost, h->stream));
   PMB_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (st & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (sort)");
+  if (*(unsigned int*)h->pinned & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (sort)");
   return PMB_OK;
 }
+
