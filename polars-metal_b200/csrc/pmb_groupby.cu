@@ -1110,12 +1110,14 @@ int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int 
   pmb_phase(h, "keys");
 
   // Capacity: 4 slots per estimated group (any size: slots come from a multiply-shift, not a
-  // mask; sample estimates of skewed keys run low), 2 per group of a caller's hint or when the
-  // estimate is the larger of the sample estimate and the selector's prediction (hash workload,
-  // 100M rows, 945K groups: table init, aggregation and finalize 1.68 ms with 4, 1.59 ms with 2).
-  // A table that fills up is rebuilt 3x larger; the estimate only sets how often that happens,
-  // never the result.
-  uint64_t cap = (uint64_t)std::max<int64_t>((est_learned ? 2 : 4) * est, 1024);
+  // mask; sample estimates of skewed keys run low), 2 per group of a caller's hint, 3 when the
+  // estimate is the larger of the sample estimate and the selector's prediction. A table that fills
+  // up (80% of its slots) is rebuilt 3x larger, a second pass over the rows; the estimate only sets
+  // how often that happens, never the result. 100M rows of Zipf(1.1) keys: 1.59 ms with 2 slots per
+  // estimated group, 1.68 ms with 4 when the estimate holds, but the larger of the two estimates was
+  // 559K to 1.77M for 1M groups, and with 2 slots half of those tables were rebuilt (+1.0 ms); with 3
+  // none was.
+  uint64_t cap = (uint64_t)std::max<int64_t>((est_learned ? 3 : 4) * est, 1024);
   if (uq->capacity_hint > 0) cap = (uint64_t)std::max<int64_t>(2 * uq->capacity_hint, 1024);
   const uint64_t cap_max = (uint64_t)std::max<int64_t>(2 * n, 1024);
   // tuning override: PMB_GCAP_MULT=<k> multiplies the global table capacity
