@@ -111,7 +111,8 @@ int pmb_groupby_sort(pmb_handle* h, CompiledQuery& cq, pmb_result* r, int64_t pa
 // *k at the sorted keys
 int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long long** k_alt, unsigned int** i,
                    unsigned int** i_alt, uint64_t cap, int64_t n, int n_passes, const unsigned int* hist_dev,
-                   const unsigned int* hist_host, bool permuted = false);
+                   const unsigned int* hist_host, bool permuted, unsigned int** status_dev);
+#define PMB_SORT_NO_READBACK (1 << 20)  // keys up to which callers pass no host copy of the counts
 // output sort (pmb_order.cu): the n rows of the device columns in the order of the spec, the first
 // `limit` of them, as device columns of r (r->n_groups set); the workspace is not reset
 int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, const pmb_sort_spec& s, pmb_result* r);

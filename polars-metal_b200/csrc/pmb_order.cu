@@ -19,7 +19,7 @@
 //                       validity word is one ballot. Integer and Bool sort columns are decoded from
 //                       the sorted keys when one round holds them all; the other columns are
 //                       gathered by row index, without reading the validity of a column that
-//                       k_null_flags found to have no nulls.
+//                       k_order_range found to have no nulls.
 // A small table takes k_order_small instead, which does all of it in one launch.
 #include <cuda_runtime.h>
 
@@ -85,7 +85,8 @@ __device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
 }
 
 // range and null count of one sort column: 16 bytes (V rows) per load, RU loads in flight. 20M rows of
-// Float64 and Int32 with nulls took 172 us with a row per load (four in flight), 89 us so.
+// Float64 and Int32 with nulls took 172 us with a row per load (four in flight), 91 us so,
+// the counts of nulls included.
 constexpr int RU = 4;
 template <typename T>
 __device__ __forceinline__ void order_range_of(const uint8_t* data, const uint8_t* __restrict__ valid, int64_t n, int dtype,
@@ -140,7 +141,35 @@ __device__ __forceinline__ void order_range_of(const uint8_t* data, const uint8_
   }
 }
 
-__global__ void __launch_bounds__(OR_NT) k_order_range(const __grid_constant__ SortCols C, int64_t n, OrderRange* out) {
+struct NullFlagCols {
+  int n;
+  const uint8_t* valid[PMB_MAX_OUT];  // null: no bitmap
+};
+
+// flags[c] = 1 when the bitmap of column c has a null among rows [0, n)
+__device__ __forceinline__ void null_flags(const NullFlagCols& V, int64_t n, unsigned int* flags) {
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t quads = n >> 7;  // whole 16-byte pieces (the bitmaps are 16-byte aligned)
+  for (int c = 0; c < V.n; c++) {
+    const uint8_t* v = V.valid[c];
+    if (!v) continue;
+    bool hole = false;
+    for (int64_t i = t0; i < quads; i += stride) {
+      const uint4 x = reinterpret_cast<const uint4*>(v)[i];
+      hole |= (x.x & x.y & x.z & x.w) != 0xFFFFFFFFu;
+    }
+    for (int64_t r = quads * 128 + t0; r < n; r += stride) hole |= !((v[r >> 3] >> (r & 7)) & 1u);
+    if (__any_sync(0xffffffffu, hole) && (threadIdx.x & 31) == 0) atomicOr(&flags[c], 1u);
+  }
+}
+
+// the sort columns' ranges (blockIdx.y 0) and which columns have nulls (blockIdx.y 1)
+__global__ void __launch_bounds__(OR_NT) k_order_range(const __grid_constant__ SortCols C, int64_t n, OrderRange* out,
+                                                       const __grid_constant__ NullFlagCols V, unsigned int* flags) {
+  if (blockIdx.y == 1) {
+    null_flags(V, n, flags);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   for (int c = 0; c < C.n; c++) {
     unsigned long long lo = ~0ULL, hi = 0, nul = 0;
@@ -246,29 +275,6 @@ __global__ void __launch_bounds__(OR_NT) k_order_encode(const __grid_constant__ 
   for (int i = threadIdx.x; i < passes * OR_RADIX; i += OR_NT) {
     const unsigned v = s_hist[i];
     if (v) atomicAdd(&hist[i], v);
-  }
-}
-
-struct NullFlagCols {
-  int n;
-  const uint8_t* valid[PMB_MAX_OUT];  // null: no bitmap
-};
-
-// flags[c] = 1 when the bitmap of column c has a null among rows [0, n)
-__global__ void __launch_bounds__(OR_NT) k_null_flags(const __grid_constant__ NullFlagCols V, int64_t n,
-                                                      unsigned int* flags) {
-  const int64_t full = n >> 3;
-  const int rest = (int)(n & 7);
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int c = 0; c < V.n; c++) {
-    const uint8_t* v = V.valid[c];
-    if (!v) continue;
-    bool hole = false;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i <= full; i += stride) {
-      if (i < full) hole |= v[i] != 0xFF;
-      else if (rest) hole |= (v[i] & ((1u << rest) - 1u)) != ((1u << rest) - 1u);
-    }
-    if (__any_sync(0xffffffffu, hole) && (threadIdx.x & 31) == 0) atomicOr(&flags[c], 1u);
   }
 }
 
@@ -636,16 +642,12 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     unsigned int* flags = (unsigned int*)(ro + 1);
     PMB_CUDA(h, cudaMemsetAsync(ro, 0, sizeof(OrderRange) + PMB_MAX_OUT * 4, h->stream));
     PMB_CUDA(h, cudaMemsetAsync(ro->lo, 0xFF, sizeof(ro->lo), h->stream));
-    pmb_kernel_begin(h, "order_range");
-    k_order_range<<<blocks_for(h, n), OR_NT, 0, h->stream>>>(C, n, ro);
-    pmb_kernel_end(h);
-    PMB_CUDA(h, cudaGetLastError());
     NullFlagCols V;
     memset(&V, 0, sizeof(V));
     V.n = n_cols;
     for (int c = 0; c < n_cols; c++) V.valid[c] = cols[c].valid;
-    pmb_kernel_begin(h, "null_flags");
-    k_null_flags<<<blocks_for(h, n / 8 + 1), OR_NT, 0, h->stream>>>(V, n, flags);
+    pmb_kernel_begin(h, "order_range");
+    k_order_range<<<dim3((unsigned)blocks_for(h, n), 2), OR_NT, 0, h->stream>>>(C, n, ro, V, flags);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     PMB_CUDA(h, cudaMemcpyAsync(h->pinned, ro, sizeof(got) + PMB_MAX_OUT * 4, cudaMemcpyDeviceToHost, h->stream));
@@ -720,10 +722,14 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     else k_order_encode<2><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
-    PMB_CUDA(h, cudaMemcpyAsync(h->pinned, hist, (size_t)passes * OR_RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
-    PMB_CUDA(h, cudaStreamSynchronize(h->stream));
-    memcpy(hh.data(), h->pinned, (size_t)passes * OR_RADIX * 4);
-    const int rc = pmb_sort_pairs(h, W, &k0, &k1, &i0, &i1, cap, n, passes, hist, hh.data(), perm != nullptr);
+    const bool counts = n > PMB_SORT_NO_READBACK;
+    if (counts) {
+      PMB_CUDA(h, cudaMemcpyAsync(h->pinned, hist, (size_t)passes * OR_RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
+      PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+      memcpy(hh.data(), h->pinned, (size_t)passes * OR_RADIX * 4);
+    }
+    const int rc = pmb_sort_pairs(h, W, &k0, &k1, &i0, &i1, cap, n, passes, hist, counts ? hh.data() : nullptr,
+                                  perm != nullptr, &h->sort_status);
     if (rc) return rc;
     perm = i0;  // the next round reads the rows in this order (and rewrites i0 with the same values)
   }
@@ -774,6 +780,18 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
   return PMB_OK;
 }
 
+// the end of a sorted call: outputs, then the status of the sort's bounded waits
+static int order_finish(pmb_handle* h, pmb_result* r, bool to_host) {
+  unsigned int* st = reinterpret_cast<unsigned int*>(h->pinned);
+  *st = 0;
+  if (h->sort_status) PMB_CUDA(h, cudaMemcpyAsync(st, h->sort_status, 4, cudaMemcpyDeviceToHost, h->stream));
+  const int rc = pmb_finish_outputs(h, r, to_host);
+  if (rc) return rc;
+  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+  if (*st & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (sort)");
+  return PMB_OK;
+}
+
 extern "C" int pmb_sort_columns(pmb_handle* h, const pmb_column* cols, int32_t n_cols, const pmb_sort_spec* spec,
                                 int32_t output_on_device, pmb_result** out) {
   if (!h) return PMB_E_INVALID;
@@ -799,13 +817,12 @@ extern "C" int pmb_sort_columns(pmb_handle* h, const pmb_column* cols, int32_t n
   pmb_result* r = pmb_result_new(n_cols);
   if (!r) return pmb_fail(h, PMB_E_OOM, "host allocation failed");
   rc = pmb_order_columns(h, d, n_cols, n, *spec, r);
-  if (!rc) rc = pmb_finish_outputs(h, r, output_on_device == 0);
+  if (!rc) rc = order_finish(h, r, output_on_device == 0);
   if (rc) {
     pmb_result_free(r);
     return rc;
   }
   r->strategy_used = PMB_STRATEGY_SORT;
-  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
   pmb_call_end(h);
   *out = r;
   return PMB_OK;
@@ -824,12 +841,11 @@ extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_c
   int rc = pmb_groupby_call(h, &qd, cols, n_cols, spec, &ordered, &g);
   if (rc) return rc;
   if (ordered) {
-    rc = pmb_finish_outputs(h, g, q->output_on_device == 0);
+    rc = order_finish(h, g, q->output_on_device == 0);
     if (rc) {
       pmb_result_free(g);
       return rc;
     }
-    PMB_CUDA(h, cudaStreamSynchronize(h->stream));
     pmb_call_end(h);
     *out = g;
     return PMB_OK;
@@ -856,12 +872,11 @@ extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_c
   r->rehash_count = g->rehash_count;
   r->capacity = g->capacity;
   pmb_result_free(g);
-  if (!rc) rc = pmb_finish_outputs(h, r, q->output_on_device == 0);
+  if (!rc) rc = order_finish(h, r, q->output_on_device == 0);
   if (rc) {
     pmb_result_free(r);
     return rc;
   }
-  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
   pmb_call_end(h);
   *out = r;
   return PMB_OK;

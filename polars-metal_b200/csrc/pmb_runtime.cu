@@ -152,6 +152,7 @@ void pmb_phase(pmb_handle* h, const char* name) {
 }
 
 void pmb_call_begin(pmb_handle* h) {
+  h->sort_status = nullptr;
   h->ptr_ok.clear();  // allocation ranges checked in this call (the caller's buffers live through it)
   h->phase_timing = getenv("PMB_CALL_TIMING") != nullptr;
   h->phases.clear();

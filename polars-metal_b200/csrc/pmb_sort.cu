@@ -327,29 +327,12 @@ struct PassParams {
   uint64_t cap;  // word stride of the key arrays
   int64_t n;
   int shift;
-  const unsigned int* gstart;    // exclusive prefix sums of this pass's 256 digit counts
+  const unsigned int* hist;      // this pass's 256 digit counts
   unsigned long long* lb;        // n_tiles x 256 look-back states (tile-major), zeroed
   unsigned long long* ticket;
   unsigned int* status;
   int hashed;  // digits of the key hash (partitioned strategy)
 };
-
-// digit counts of every pass -> first output position of every digit (a CTA per pass)
-__global__ void __launch_bounds__(RADIX) k_digit_starts(const unsigned int* __restrict__ hist,
-                                                        unsigned int* __restrict__ gstart) {
-  __shared__ unsigned int s_scan[RADIX / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned c = hist[blockIdx.x * RADIX + tid];
-  unsigned x = c;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_scan[warp] = x;
-  __syncthreads();
-  for (int w = 0; w < warp; w++) x += s_scan[w];
-  gstart[blockIdx.x * RADIX + tid] = x - c;
-}
 
 // Tile shape of a pass, for W-word keys: three (two) CTAs of 12 (16) warps fit an SM's shared memory
 template <int W>
@@ -422,7 +405,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   unsigned int(*s_off)[RADIX] = reinterpret_cast<unsigned int(*)[RADIX]>(s_idx + TILE);  // NW
   unsigned int(*s_lanes)[RADIX] = s_off + NW;                                            // NW
   __shared__ long long s_out[RADIX];  // output position of a digit's first key, less its tile position
-  __shared__ unsigned int s_scan[RADIX / 32];
+  __shared__ uint2 s_scan[RADIX / 32];
   __shared__ long long s_tile;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_tile = (long long)atomicAdd(P.ticket, 1ULL);
@@ -446,7 +429,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   __syncthreads();
   // thread d: the tile's count of digit d, published at once; then the tile-local exclusive scan
   // over the digits, and every warp's first position of the digit
-  unsigned acc = 0, x = 0;
+  unsigned acc = 0, x = 0, gs = 0;  // gs: output position of the digit's first key, all tiles
   if (tid < RADIX) {
     unsigned c[NW];
 #pragma unroll
@@ -458,17 +441,27 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
       acc += t;
     }
     *((volatile unsigned long long*)&P.lb[tile * RADIX + tid]) = ((tile == 0 ? 2ULL : 1ULL) << 62) | acc;
+    const unsigned hd = P.hist[tid];
     x = acc;
+    gs = hd;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o), z = __shfl_up_sync(0xffffffffu, gs, o);
+      if (lane >= o) {
+        x += y;
+        gs += z;
+      }
     }
-    if (lane == 31) s_scan[warp] = x;
+    if (lane == 31) s_scan[warp] = make_uint2(x, gs);
     asm volatile("bar.sync 1, 256;" ::: "memory");  // the RADIX threads of this scan
 #pragma unroll
-    for (int w = 0; w < RADIX / 32; w++) x += w < warp ? s_scan[w] : 0u;
+    for (int w = 0; w < RADIX / 32; w++)
+      if (w < warp) {
+        x += s_scan[w].x;
+        gs += s_scan[w].y;
+      }
     x -= acc;
+    gs -= hd;
 #pragma unroll
     for (int w = 0; w < NW; w++) s_off[w][tid] = c[w] + x;
   }
@@ -497,7 +490,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   }
   if (tid < RADIX) {
     const unsigned long long pre = digit_lookback(P.lb + tid, tile, acc, P.status);
-    s_out[tid] = (long long)P.gstart[tid] + (long long)pre - (long long)x;
+    s_out[tid] = (long long)gs + (long long)pre - (long long)x;
   }
   __syncthreads();
   const int valid = (int)min((long long)TILE, (long long)P.n - tile * TILE);
@@ -1164,10 +1157,14 @@ int ordered_finalize(pmb_handle* h, const CompiledQuery& cq, const PartFinParams
   k_group_order<W><<<blocks, ST_NT, 0, h->stream>>>(O, F.gkeys, F.gcap, ng, k0, ocap, i0, passes, hist);
   pmb_kernel_end(h);
   PMB_CUDA(h, cudaGetLastError());
-  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
-  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
-  std::vector<unsigned int> hh((const unsigned int*)h->pinned, (const unsigned int*)h->pinned + (size_t)passes * RADIX);
-  const int rc = pmb_sort_pairs(h, W, &k0, &k1, &i0, &i1, ocap, ng, passes, hist, hh.data());
+  std::vector<unsigned int> hh;
+  if (ng > PMB_SORT_NO_READBACK && passes > 0) {
+    PMB_CUDA(h, cudaMemcpyAsync(h->pinned, hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
+    PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+    hh.assign((const unsigned int*)h->pinned, (const unsigned int*)h->pinned + (size_t)passes * RADIX);
+  }
+  const int rc = pmb_sort_pairs(h, W, &k0, &k1, &i0, &i1, ocap, ng, passes, hist, hh.empty() ? nullptr : hh.data(), false,
+                                &h->sort_status);
   if (rc) return rc;
   const int64_t start = s.offset >= 0 ? std::min<int64_t>(s.offset, ng) : std::max<int64_t>(0, ng + s.offset);
   const int64_t m = s.limit < 0 ? ng - start : std::min<int64_t>(s.limit, ng - start);
@@ -1463,8 +1460,7 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   const int64_t max_ptiles = (n + PassShape<W>::TILE - 1) / PassShape<W>::TILE;  // pass tiles
   unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(
       h, (size_t)std::max<int64_t>({max_tiles, max_ptiles * RADIX, 1}) * 8);
-  unsigned int* gstart = (unsigned int*)pmb_ws_alloc(h, (size_t)MAX_PASSES * RADIX * 4);
-  if (!k0 || !k1 || !i0 || !i1 || !hist || !ctr || !status || !lb || !gstart)
+  if (!k0 || !k1 || !i0 || !i1 || !hist || !ctr || !status || !lb)
     return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort buffers)");
   PMB_CUDA(h, cudaMemsetAsync(hist, 0, (size_t)MAX_PASSES * RADIX * 4, h->stream));
   PMB_CUDA(h, cudaMemsetAsync(ctr, 0, 64, h->stream));
@@ -1510,12 +1506,6 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   const int64_t ptiles = (m + PassShape<W>::TILE - 1) / PassShape<W>::TILE;
   constexpr size_t pass_smem = PassShape<W>::SMEM;
   PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
-  if (passes > 0 && m > 1) {
-    pmb_kernel_begin(h, "digit_starts");
-    k_digit_starts<<<passes, RADIX, 0, h->stream>>>(hist, gstart);
-    pmb_kernel_end(h);
-    PMB_CUDA(h, cudaGetLastError());
-  }
   int done = 0;
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
@@ -1530,7 +1520,7 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     P.n = m;
     P.shift = (part_groups > 0 ? 64 - pb : 0) + 8 * p;
     P.hashed = part_groups > 0;
-    P.gstart = gstart + (size_t)p * RADIX;
+    P.hist = hist + (size_t)p * RADIX;
     P.lb = lb;
     P.ticket = ctr + 1;
     P.status = status;
@@ -1804,26 +1794,29 @@ __global__ void __launch_bounds__(ST_NT) k_gather_word(const unsigned long long*
 // or the alternates). Two-word keys are sorted a word at a time, the second word fetched in the order
 // of the first: a pass over 12-byte pairs takes half the time of one over 20-byte pairs (20M rows: 159
 // against 316 us), the fetch less than one pass; their sorted keys are not returned. The second words
-// are stored by row number; `permuted`: *i is not 0, 1, 2, ... already on entry.
+// are stored by row number; `permuted`: *i is not 0, 1, 2, ... already on entry. Without hist_host every
+// digit gets its pass (one more pass of up to a million keys takes less than reading the counts back).
+// The call does not wait: *status_dev (device; null before a call's first round) holds PMB_ST_TIMEOUT
+// after the stream has got there.
 int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long long** k_alt, unsigned int** i,
                    unsigned int** i_alt, uint64_t cap, int64_t n, int n_passes, const unsigned int* hist_dev,
-                   const unsigned int* hist_host, bool permuted) {
+                   const unsigned int* hist_host, bool permuted, unsigned int** status_dev) {
   if (W != 1 && W != 2) return pmb_fail(h, PMB_E_INVALID, "sort: key of 1 or 2 words");
   if (n_passes > MAX_PASSES) return pmb_fail(h, PMB_E_INVALID, "sort: more than 16 digit passes");
   if (n <= 1 || n_passes <= 0) return PMB_OK;
   const int64_t tiles = (n + PassShape<1>::TILE - 1) / PassShape<1>::TILE;
   const size_t lb_bytes = (size_t)tiles * RADIX * 8;
-  // look-back states, then the ticket (cleared together), then status
-  unsigned long long* lb = (unsigned long long*)pmb_ws_alloc(h, lb_bytes + 64);
-  unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
-  unsigned int* gstart = (unsigned int*)pmb_ws_alloc(h, (size_t)n_passes * RADIX * 4);
-  if (!lb || !status || !gstart) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
-  PMB_CUDA(h, cudaMemsetAsync(status, 0, 64, h->stream));
+  // per pass a ticket and look-back states; small ones are cleared for all passes at once
+  const size_t pass_bytes = lb_bytes + 64;
+  const bool at_once = pass_bytes * n_passes <= (size_t)32 << 20;
+  const size_t clear = at_once ? pass_bytes * n_passes : pass_bytes;
+  uint8_t* zeroed = (uint8_t*)pmb_ws_alloc(h, clear + 64);
+  if (!zeroed) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (sort passes)");
+  // the status of an earlier round of the same call goes on being used
+  unsigned int* status = *status_dev ? *status_dev : (unsigned int*)(zeroed + clear);
+  if (at_once) PMB_CUDA(h, cudaMemsetAsync(zeroed, 0, clear + 64, h->stream));
+  else PMB_CUDA(h, cudaMemsetAsync(zeroed + clear, 0, 64, h->stream));
   PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
-  pmb_kernel_begin(h, "digit_starts");
-  k_digit_starts<<<n_passes, RADIX, 0, h->stream>>>(hist_dev, gstart);
-  pmb_kernel_end(h);
-  PMB_CUDA(h, cudaGetLastError());
   unsigned long long* a = *k;       // the current word's keys, and where the next pass writes them
   unsigned long long* b = *k_alt;
   bool moved = permuted;            // the order differs from the rows'
@@ -1833,8 +1826,10 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
       b = *k_alt + cap;
     }
     bool constant = false;
-    for (int d = 0; d < RADIX; d++) constant |= hist_host[(size_t)p * RADIX + d] == (unsigned)n;
+    for (int d = 0; hist_host && d < RADIX; d++) constant |= hist_host[(size_t)p * RADIX + d] == (unsigned)n;
     if (constant) continue;
+    uint8_t* z = zeroed + (at_once ? (size_t)p * pass_bytes : 0);
+    if (!at_once) PMB_CUDA(h, cudaMemsetAsync(z, 0, pass_bytes, h->stream));
     if (p >= 8 && moved) {  // the second word in the order so far, once
       const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 4 * ST_NT - 1) / (4 * ST_NT), (int64_t)h->sm_count * 8));
       pmb_kernel_begin(h, "sort_fetch");
@@ -1853,11 +1848,10 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
     P.n = n;
     P.shift = 8 * (p & 7);
     P.hashed = 0;
-    P.gstart = gstart + (size_t)p * RADIX;
-    P.lb = lb;
-    P.ticket = lb + (size_t)tiles * RADIX;
+    P.hist = hist_dev + (size_t)p * RADIX;
+    P.ticket = (unsigned long long*)z;
+    P.lb = (unsigned long long*)(z + 64);
     P.status = status;
-    PMB_CUDA(h, cudaMemsetAsync(lb, 0, lb_bytes + 64, h->stream));
     pmb_kernel_begin(h, "sort_pass");
     k_sort_pass<1><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
     pmb_kernel_end(h);
@@ -1870,9 +1864,7 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
     *k = a;
     *k_alt = b;
   }
-  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, status, 4, cudaMemcpyDeviceToHost, h->stream));
-  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
-  if (*(unsigned int*)h->pinned & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (sort)");
+  *status_dev = status;
   return PMB_OK;
 }
 
