@@ -87,10 +87,10 @@ struct JPartH {
   unsigned long long kcap;
   const unsigned int* idx;
   const unsigned long long* pstart;
-  const unsigned int* items;
+  long long n_parts;
   long long n_items;
   int slots;
-  int pad;
+  int run;
   unsigned long long* ticket;
   unsigned long long* gkeys;
   unsigned char* grecs;

@@ -24,10 +24,10 @@ struct JPart {
   unsigned long long kcap;
   const unsigned int* idx;            // row index of every sorted key
   const unsigned long long* pstart;   // first sorted row of every partition (and the end)
-  const unsigned int* items;          // first partition of every work item (and the end)
+  long long n_parts;                  // partitions
   long long n_items;
   int slots;                          // table slots
-  int pad;
+  int run;                            // partitions per work item
   unsigned long long* ticket;
   unsigned long long* gkeys;          // dense groups: packed keys, word-major (stride gcap)
   unsigned char* grecs;               // and their records, J_REC bytes each
@@ -66,7 +66,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
     __syncthreads();
     const long long it = s_item;
     if (it >= A.n_items) break;
-    const long long ps = (long long)A.pstart[A.items[it]], pe = (long long)A.pstart[A.items[it + 1]];
+    const long long ps = (long long)A.pstart[it * A.run], pe = (long long)A.pstart[min(A.n_parts, (it + 1) * A.run)];
     for (long long b = ps; b < pe; b += (long long)J_NT * JP_R) {
       unsigned long long k[JP_R][JP_W];
       unsigned slot[JP_R], row[JP_R], probes[JP_R];

@@ -261,56 +261,89 @@ struct EncodeParams {
   unsigned int* status;
   int hashed;                  // digits of the key hash (partitioned strategy)
   int shift0;                  // bit of pass 0's digit; pass p uses shift0 + 8p
-  unsigned int* phist;         // partitioned strategy: rows per partition (2^pb counters), or null
-  int pb;
 };
 
-// filter, pack and compact in row order (4096-row tiles, decoupled look-back), with the digit
-// histograms of every pass
-template <int W>
+// exclusive offsets of a tile's ST_PER x 8 warp counts (item-major), in place, and their total: four
+// counts to a lane of warp 0, which calls this whole
+__device__ __forceinline__ unsigned scan_counts(unsigned int* cnt) {
+  static_assert(ST_PER * (ST_NT / 32) == 128, "four counts per lane");
+  const int lane = threadIdx.x & 31;
+  uint4 c = reinterpret_cast<uint4*>(cnt)[lane];
+  const unsigned sum = c.x + c.y + c.z + c.w;
+  unsigned x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  const unsigned e = x - sum;
+  reinterpret_cast<uint4*>(cnt)[lane] = make_uint4(e, e + c.x, e + c.x + c.y, e + c.x + c.y + c.z);
+  return __shfl_sync(0xffffffffu, x, 31);
+}
+
+// Filter, pack and compact in row order (4096-row tiles, decoupled look-back), with the digit histograms
+// of every pass. Without a predicate (PRED false) every row keeps its place: no verdicts, no look-back,
+// four rows' keys packed before any is counted, so that their loads go out together. 200M rows of
+// 12-byte keys: 2437 us with one thread scanning the tile's counts, a look-back for rows that all stay
+// and a global count per partition, 1371 us now.
+template <int W, bool PRED>
 __global__ void __launch_bounds__(ST_NT) k_sort_encode(const __grid_constant__ EncodeParams E) {
   __shared__ unsigned int s_hist[MAX_PASSES][RADIX];
-  __shared__ unsigned int s_cnt[ST_PER][ST_NT / 32];
+  __shared__ __align__(16) unsigned int s_cnt[ST_PER][ST_NT / 32];
   __shared__ long long s_tile;
   __shared__ unsigned long long s_base;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (int i = tid; i < E.passes * RADIX; i += ST_NT) (&s_hist[0][0])[i] = 0;
-  if (tid == 0) s_tile = (long long)atomicAdd(E.ticket, 1ULL);
+  if (PRED && tid == 0) s_tile = (long long)atomicAdd(E.ticket, 1ULL);
   __syncthreads();
-  const long long tile = s_tile;
-  const TileCtx t{nullptr, nullptr, nullptr, 0};
-  const bool has_pred = E.q.prog.n_ops > 0;
-  bool keep[ST_PER];
-  for (int j = 0; j < ST_PER; j++) {
-    const int64_t r = tile * ST_TILE + (int64_t)j * ST_NT + tid;
-    keep[j] = r < E.n && (!has_pred || eval_keep(E.q, t, r));
-    const unsigned b = __ballot_sync(0xffffffffu, keep[j]);
-    if (lane == 0) s_cnt[j][warp] = __popc(b);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    unsigned acc = 0;
-    for (int j = 0; j < ST_PER; j++)
-      for (int w = 0; w < ST_NT / 32; w++) {
-        unsigned c = s_cnt[j][w];
-        s_cnt[j][w] = acc;
-        acc += c;
+  const long long tile = PRED ? s_tile : (long long)blockIdx.x;
+  unsigned keep = 0;  // bit j: row j of this thread is kept
+  if (PRED) {
+    const TileCtx t{nullptr, nullptr, nullptr, 0};
+    for (int j = 0; j < ST_PER; j++) {
+      const int64_t r = tile * ST_TILE + (int64_t)j * ST_NT + tid;
+      const bool k = r < E.n && eval_keep(E.q, t, r);
+      const unsigned b = __ballot_sync(0xffffffffu, k);
+      if (k) keep |= 1u << j;
+      if (lane == 0) s_cnt[j][warp] = __popc(b);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const unsigned acc = scan_counts(&s_cnt[0][0]);
+      const unsigned long long b = pmb_lookback_warp(E.lb, tile, acc, E.status);
+      if (lane == 0) {
+        s_base = b;
+        if (tile == (long long)gridDim.x - 1) *E.kept = b + acc;
       }
-    const unsigned long long b = pmb_lookback(E.lb, tile, acc, E.status);
-    s_base = b;
-    if (tile == (long long)gridDim.x - 1) *E.kept = b + acc;
+    }
+    __syncthreads();
+  } else if (blockIdx.x == 0 && tid == 0) {
+    *E.kept = (unsigned long long)E.n;
   }
-  __syncthreads();
-  for (int j = 0; j < ST_PER; j++) {
-    const unsigned b = __ballot_sync(0xffffffffu, keep[j]);
-    if (!keep[j]) continue;
-    const int64_t r = tile * ST_TILE + (int64_t)j * ST_NT + tid;
-    const PKey<W> k = pack_sort_key<W>(E.L, r);
-    for (int p = 0; p < E.passes; p++) atomicAdd(&s_hist[p][pass_digit<W>(k, E.shift0 + 8 * p, E.hashed)], 1u);
-    if (E.phist) atomicAdd(&E.phist[part_hash<W>(k) >> (64 - E.pb)], 1u);
-    const uint64_t pos = s_base + s_cnt[j][warp] + __popc(b & ((1u << lane) - 1u));
-    for (int i = 0; i < W; i++) E.keys[(uint64_t)i * E.cap + pos] = k.w[i];
-    E.idx[pos] = (unsigned)r;
+  for (int j0 = 0; j0 < ST_PER; j0 += 4) {
+    PKey<W> k[4];
+    bool in[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int64_t r = tile * ST_TILE + (int64_t)(j0 + u) * ST_NT + tid;
+      in[u] = PRED ? ((keep >> (j0 + u)) & 1u) != 0u : r < E.n;
+      if (in[u]) k[u] = pack_sort_key<W>(E.L, r);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const unsigned b = __ballot_sync(0xffffffffu, in[u]);
+      if (!in[u]) continue;
+      const int64_t r = tile * ST_TILE + (int64_t)(j0 + u) * ST_NT + tid;
+      const unsigned long long h = E.hashed ? part_hash<W>(k[u]) : 0ULL;
+      for (int p = 0; p < E.passes; p++) {
+        const int sh = E.shift0 + 8 * p;
+        atomicAdd(&s_hist[p][E.hashed ? (unsigned)(h >> sh) & 0xFFu : digit_of<W>(k[u], sh)], 1u);
+      }
+      const uint64_t pos = PRED ? s_base + s_cnt[j0 + u][warp] + __popc(b & ((1u << lane) - 1u)) : (uint64_t)r;
+#pragma unroll
+      for (int i = 0; i < W; i++) E.keys[(uint64_t)i * E.cap + pos] = k[u].w[i];
+      E.idx[pos] = (unsigned)r;
+    }
   }
   __syncthreads();
   for (int i = tid; i < E.passes * RADIX; i += ST_NT) {
@@ -331,7 +364,6 @@ struct PassParams {
   unsigned long long* lb;        // n_tiles x 256 look-back states (tile-major), zeroed
   unsigned long long* ticket;
   unsigned int* status;
-  int hashed;  // digits of the key hash (partitioned strategy)
 };
 
 // Tile shape of a pass, for W-word keys: three (two) CTAs of 12 (16) warps fit an SM's shared memory
@@ -395,7 +427,7 @@ __device__ __forceinline__ unsigned long long digit_lookback(unsigned long long*
 // 795 us (3.0 TB/s of the 6.4 a plain copy reaches); 256 threads x 16 keys with match_any, ranks
 // held to the end and a look-back of one state per step took 1020 us. 128-bit keys, 20M: 259 us,
 // against 552 us. Prefetching the next tile with bulk copies (persistent CTAs) took 900-960 us.
-template <int W>
+template <int W, bool HASHED>
 __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
     k_sort_pass(const __grid_constant__ PassParams P) {
   constexpr int NT = PassShape<W>::NT, PER = PassShape<W>::PER, TILE = PassShape<W>::TILE, NW = PassShape<W>::NW;
@@ -423,9 +455,15 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
     for (int w = 0; w < W; w++) k[j].w[w] = e0 + j * 32 < P.n ? __ldcs(&P.kin[(uint64_t)w * P.cap + e0 + j * 32]) : 0ULL;
 #pragma unroll
   for (int j = 0; j < PER; j++) ix[j] = e0 + j * 32 < P.n ? __ldcs(&P.iin[e0 + j * 32]) : 0u;
+  unsigned dg[(PER + 3) / 4];  // digits of the key hash, four to a register (a key's own digit is a shift away)
+#pragma unroll
+  for (int j = 0; j < (PER + 3) / 4; j++) dg[j] = 0u;
+#pragma unroll
+  for (int j = 0; HASHED && j < PER; j++) dg[j >> 2] |= pass_digit<W>(k[j], P.shift, true) << (8 * (j & 3));
+  auto digit = [&](int j) { return HASHED ? (dg[j >> 2] >> (8 * (j & 3))) & 0xFFu : digit_of<W>(k[j], P.shift); };
 #pragma unroll
   for (int j = 0; j < PER; j++)
-    if (e0 + j * 32 < P.n) atomicAdd(&s_off[warp][pass_digit<W>(k[j], P.shift, P.hashed)], 1u);
+    if (e0 + j * 32 < P.n) atomicAdd(&s_off[warp][digit(j)], 1u);
   __syncthreads();
   // thread d: the tile's count of digit d, published at once; then the tile-local exclusive scan
   // over the digits, and every warp's first position of the digit
@@ -471,7 +509,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
 #pragma unroll
   for (int j = 0; j < PER; j++) {
     const bool in = e0 + j * 32 < P.n;
-    const unsigned d = pass_digit<W>(k[j], P.shift, P.hashed);
+    const unsigned d = digit(j);
     if (in) atomicOr(&s_lanes[warp][d], 1u << lane);
     __syncwarp();
     const unsigned peers = s_lanes[warp][d], first = s_off[warp][d], below = __popc(peers & lt);
@@ -501,7 +539,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
     PKey<W> kk;
 #pragma unroll
     for (int w = 0; w < W; w++) kk.w[w] = s_key[w * TILE + i];
-    const uint64_t g = (uint64_t)(s_out[pass_digit<W>(kk, P.shift, P.hashed)] + i);
+    const uint64_t g = (uint64_t)(s_out[pass_digit<W>(kk, P.shift, HASHED)] + i);
 #pragma unroll
     for (int w = 0; w < W; w++) P.kout[(uint64_t)w * P.cap + g] = kk.w[w];
     P.iout[g] = s_idx[i];
@@ -521,7 +559,7 @@ struct StartsParams {
 
 template <int W>
 __global__ void __launch_bounds__(ST_NT) k_seg_starts(const __grid_constant__ StartsParams S) {
-  __shared__ unsigned int s_cnt[ST_PER][ST_NT / 32];
+  __shared__ __align__(16) unsigned int s_cnt[ST_PER][ST_NT / 32];
   __shared__ long long s_tile;
   __shared__ unsigned long long s_base;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -541,19 +579,15 @@ __global__ void __launch_bounds__(ST_NT) k_seg_starts(const __grid_constant__ St
     if (lane == 0) s_cnt[j][warp] = __popc(b);
   }
   __syncthreads();
-  if (tid == 0) {
-    unsigned acc = 0;
-    for (int j = 0; j < ST_PER; j++)
-      for (int w = 0; w < ST_NT / 32; w++) {
-        unsigned c = s_cnt[j][w];
-        s_cnt[j][w] = acc;
-        acc += c;
+  if (warp == 0) {
+    const unsigned acc = scan_counts(&s_cnt[0][0]);
+    const unsigned long long b = pmb_lookback_warp(S.lb, tile, acc, S.status);
+    if (lane == 0) {
+      s_base = b;
+      if (tile == (long long)gridDim.x - 1) {
+        *S.n_groups = b + acc;
+        S.starts[b + acc] = (unsigned)S.n;
       }
-    const unsigned long long b = pmb_lookback(S.lb, tile, acc, S.status);
-    s_base = b;
-    if (tile == (long long)gridDim.x - 1) {
-      *S.n_groups = b + acc;
-      S.starts[b + acc] = (unsigned)S.n;
     }
   }
   __syncthreads();
@@ -704,8 +738,8 @@ __global__ void __launch_bounds__(BIG_NT) k_seg_reduce_big(const __grid_constant
 
 // ---------------------------------------------------------------- partitioned strategy
 // After the hash-digit passes the kept rows are ordered by partition (the top `pb` bits of the key
-// hash), so every group's rows lie inside one partition; the encode pass counted the rows of every
-// partition, so their offsets are exact. k_part_agg: persistent CTAs take work items (runs of
+// hash), so every group's rows lie inside one partition; the
+// partition starts are read off the sorted keys. k_part_agg: persistent CTAs take work items (runs of
 // consecutive partitions) and aggregate one partition at a time in a shared-memory table (slot claim by a tag word, records in the global-record layout updated by
 // apply_row_shared, values gathered by row index). At the end of each partition the occupied
 // slots are compacted and written straight to the output columns (one atomic per partition for
@@ -722,10 +756,9 @@ struct PartParams {
   uint64_t cap;
   const unsigned int* idx;         // their row indices
   int64_t m;                       // kept rows
-  int pb;                          // partition bits
-  const unsigned long long* pstart;  // 2^pb + 1: first row of every partition
-  const unsigned int* items;       // n_items + 1: first partition of every work item (whole partitions
-                                   // whose rows, an upper bound of their groups, fit the table)
+  const unsigned long long* pstart;  // n_parts + 1: first row of every partition
+  int64_t n_parts;
+  int run;                         // partitions per work item
   int64_t n_items;
   int slots;                       // shared table slots
   int n_out;
@@ -801,7 +834,7 @@ __global__ void __launch_bounds__(PA_NT, 1) k_part_agg(const __grid_constant__ P
     if (it >= A.n_items) break;
     {
       // the item's partitions: rows [ps, pe)
-      const int64_t ps = (int64_t)A.pstart[A.items[it]], pe = (int64_t)A.pstart[A.items[it + 1]];
+      const int64_t ps = (int64_t)A.pstart[it * A.run], pe = (int64_t)A.pstart[min((long long)A.n_parts, (it + 1) * A.run)];
       for (int64_t b = ps; b < pe; b += (int64_t)PA_NT * PA_R) {
         // PA_R rows per thread; their key and row-index loads go out together
         PKey<W> k[PA_R];
@@ -974,6 +1007,27 @@ __global__ void __launch_bounds__(PA_NT, 1) k_part_agg(const __grid_constant__ P
       __syncthreads();
     }
   }
+}
+
+// First row of every partition of the m sorted keys (pstart[2^pb] = m), a binary search each: about 28
+// dependent reads, all partitions at once. Counting the rows of 65,536 partitions in the encode pass cost
+// a global atomic a row and the counts a trip through the host; reading the sorted keys for the places
+// where the partition changes took 600 us for 200M rows, the searches 33 us.
+template <int W>
+__global__ void __launch_bounds__(ST_NT) k_part_starts(const unsigned long long* __restrict__ keys, uint64_t cap, int64_t m,
+                                                       int pb, unsigned long long* __restrict__ pstart) {
+  const long long q = (long long)blockIdx.x * ST_NT + threadIdx.x;
+  if (q > (1LL << pb)) return;
+  int64_t lo = 0, hi = m;
+  while (lo < hi) {
+    const int64_t mid = (lo + hi) >> 1;
+    PKey<W> k;
+#pragma unroll
+    for (int w = 0; w < W; w++) k.w[w] = keys[(uint64_t)w * cap + mid];
+    if ((long long)(part_hash<W>(k) >> (64 - pb)) < q) lo = mid + 1;
+    else hi = mid;
+  }
+  pstart[q] = (unsigned long long)lo;
 }
 
 // dense groups of the run-time compiled partitioned aggregation (packed keys, global-layout
@@ -1242,9 +1296,8 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
 // the aggregation of the partitioned strategy over keys / row indices sorted by partition
 template <int W>
 int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_result* r, const unsigned long long* keys,
-                 const unsigned int* idx, uint64_t cap, int64_t m, int pb, const std::vector<unsigned int>& counts,
-                 int slots, int64_t groups,
-                 unsigned long long* ctr, unsigned int* status, int strategy = PMB_STRATEGY_PARTITIONED) {
+                 const unsigned int* idx, uint64_t cap, int64_t m, const unsigned long long* pstart, int64_t n_parts,
+                 int run, int slots, int64_t groups, unsigned long long* ctr, unsigned int* status, int strategy = PMB_STRATEGY_PARTITIONED) {
   DQuery& q = cq.dq;
   const int n_out = q.n_keys + q.n_aggs;
   PartParams A;
@@ -1255,31 +1308,10 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
   A.cap = cap;
   A.idx = idx;
   A.m = m;
-  A.pb = pb;
-  // partition offsets, and work items: runs of whole partitions whose rows (an upper bound of
-  // their groups) stay within 70% of the table, at least one partition each
-  const unsigned long long lim = (unsigned long long)(0.7 * slots);
-  std::vector<unsigned long long> pstart(counts.size() + 1, 0);
-  std::vector<unsigned int> items(1, 0);
-  unsigned long long run = 0;
-  for (size_t p = 0; p < counts.size(); p++) {
-    pstart[p + 1] = pstart[p] + counts[p];
-    if (run > 0 && run + counts[p] > lim) {
-      items.push_back((unsigned)p);
-      run = 0;
-    }
-    run += counts[p];
-  }
-  if (run > 0 || items.size() == 1) items.push_back((unsigned)counts.size());
-  if ((int64_t)pstart.back() != m) return pmb_fail(h, PMB_E_CUDA, "partition counts do not add up");
-  unsigned long long* d_pstart = (unsigned long long*)pmb_ws_alloc(h, pstart.size() * 8);
-  unsigned int* d_items = (unsigned int*)pmb_ws_alloc(h, items.size() * 4);
-  if (!d_pstart || !d_items) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (partition offsets)");
-  PMB_CUDA(h, cudaMemcpyAsync(d_pstart, pstart.data(), pstart.size() * 8, cudaMemcpyHostToDevice, h->stream));
-  PMB_CUDA(h, cudaMemcpyAsync(d_items, items.data(), items.size() * 4, cudaMemcpyHostToDevice, h->stream));
-  A.pstart = d_pstart;
-  A.items = d_items;
-  A.n_items = (int64_t)items.size() - 1;
+  A.pstart = pstart;
+  A.n_parts = n_parts;
+  A.run = run;
+  A.n_items = (n_parts + run - 1) / run;
   A.slots = slots;
   A.n_out = n_out;
   A.stage_bytes = pa_stage(q, &A.used, A.sdoff, A.svoff);
@@ -1344,7 +1376,8 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         JA.kcap = cap;
         JA.idx = idx;
         JA.pstart = A.pstart;
-        JA.items = A.items;
+        JA.n_parts = n_parts;
+        JA.run = run;
         JA.n_items = A.n_items;
         JA.slots = slots;
         JA.ticket = A.ticket;
@@ -1450,10 +1483,9 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   unsigned int* i0 = (unsigned int*)pmb_ws_alloc(h, (size_t)cap * 4 + 16);
   unsigned int* i1 = (unsigned int*)pmb_ws_alloc(h, (size_t)cap * 4 + 16);
   unsigned int* hist = (unsigned int*)pmb_ws_alloc(h, (size_t)MAX_PASSES * RADIX * 4);
-  const size_t n_parts = part_groups > 0 ? (size_t)1 << pb : 0;
-  unsigned int* phist = n_parts ? (unsigned int*)pmb_ws_alloc(h, n_parts * 4) : nullptr;
-  if (n_parts && !phist) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (partition counts)");
-  if (n_parts) PMB_CUDA(h, cudaMemsetAsync(phist, 0, n_parts * 4, h->stream));
+  const int64_t n_parts = part_groups > 0 ? (int64_t)1 << pb : 0;
+  unsigned long long* pstart = n_parts ? (unsigned long long*)pmb_ws_alloc(h, (size_t)(n_parts + 1) * 8) : nullptr;
+  if (n_parts && !pstart) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (partition offsets)");
   unsigned long long* ctr = (unsigned long long*)pmb_ws_alloc(h, 64);  // kept, ticket, n_groups, big_n
   unsigned int* status = (unsigned int*)pmb_ws_alloc(h, 64);
   const int64_t max_tiles = (n + ST_TILE - 1) / ST_TILE;
@@ -1482,30 +1514,29 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     E.status = status;
     E.hashed = part_groups > 0;
     E.shift0 = part_groups > 0 ? 64 - pb : 0;
-    E.phist = phist;
-    E.pb = pb;
     PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)std::max<int64_t>(max_tiles, 1) * 8, h->stream));
     pmb_kernel_begin(h, "sort_encode");
-    k_sort_encode<W><<<(unsigned)std::max<int64_t>(max_tiles, 1), ST_NT, 0, h->stream>>>(E);
+    const auto encode = q.prog.n_ops > 0 ? k_sort_encode<W, true> : k_sort_encode<W, false>;
+    encode<<<(unsigned)std::max<int64_t>(max_tiles, 1), ST_NT, 0, h->stream>>>(E);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
   }
   std::vector<unsigned int> hh((size_t)std::max(passes, 1) * RADIX);
-  unsigned long long kept = 0;
-  unsigned int st0 = 0;
-  PMB_CUDA(h, cudaMemcpyAsync(&kept, ctr, 8, cudaMemcpyDeviceToHost, h->stream));
-  PMB_CUDA(h, cudaMemcpyAsync(&st0, status, 4, cudaMemcpyDeviceToHost, h->stream));
-  if (passes) PMB_CUDA(h, cudaMemcpyAsync(hh.data(), hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
-  std::vector<unsigned int> ph(n_parts);
-  if (n_parts) PMB_CUDA(h, cudaMemcpyAsync(ph.data(), phist, n_parts * 4, cudaMemcpyDeviceToHost, h->stream));
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, ctr, 8, cudaMemcpyDeviceToHost, h->stream));
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned + 8, status, 4, cudaMemcpyDeviceToHost, h->stream));
+  if (passes) PMB_CUDA(h, cudaMemcpyAsync(h->pinned + 64, hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, h->stream));
   PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+  const unsigned long long kept = *(unsigned long long*)h->pinned;
+  const unsigned int st0 = *(unsigned int*)(h->pinned + 8);
+  memcpy(hh.data(), h->pinned + 64, (size_t)passes * RADIX * 4);
   if (st0 & PMB_ST_TIMEOUT) return pmb_fail(h, PMB_E_TIMEOUT, "a bounded device wait timed out (sort)");
   const int64_t m = (int64_t)kept;
   // LSD passes over the digits that are not the same for every key
   const int64_t tiles = (m + ST_TILE - 1) / ST_TILE;
   const int64_t ptiles = (m + PassShape<W>::TILE - 1) / PassShape<W>::TILE;
   constexpr size_t pass_smem = PassShape<W>::SMEM;
-  PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
+  const auto pass = part_groups > 0 ? k_sort_pass<W, true> : k_sort_pass<W, false>;
+  PMB_CUDA(h, cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
   int done = 0;
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
@@ -1519,7 +1550,6 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     P.cap = cap;
     P.n = m;
     P.shift = (part_groups > 0 ? 64 - pb : 0) + 8 * p;
-    P.hashed = part_groups > 0;
     P.hist = hist + (size_t)p * RADIX;
     P.lb = lb;
     P.ticket = ctr + 1;
@@ -1527,14 +1557,24 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)ptiles * RADIX * 8, h->stream));
     PMB_CUDA(h, cudaMemsetAsync(ctr + 1, 0, 8, h->stream));
     pmb_kernel_begin(h, "sort_pass");
-    k_sort_pass<W><<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
+    pass<<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     std::swap(k0, k1);
     std::swap(i0, i1);
     done++;
   }
-  if (part_groups > 0) return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pb, ph, slots, part_groups, ctr, status);
+  if (part_groups > 0) {
+    pmb_kernel_begin(h, "part_starts");
+    k_part_starts<W><<<(unsigned)(n_parts / ST_NT + 1), ST_NT, 0, h->stream>>>(k0, cap, m, pb, pstart);
+    pmb_kernel_end(h);
+    PMB_CUDA(h, cudaGetLastError());
+    // work items: runs of partitions with half a table of rows on average (rows bound the groups; the
+    // hash spreads them, so a run stays far from the whole table), at least one partition each
+    const int64_t rows = std::max<int64_t>(1, m / n_parts);
+    const int run = (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, slots / 2 / rows));
+    return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pstart, n_parts, run, slots, part_groups, ctr, status);
+  }
   // segment starts
   unsigned int* starts = (unsigned int*)pmb_ws_alloc(h, (size_t)(m + 2) * 4);
   if (!starts) return pmb_fail(h, PMB_E_OOM, "workspace exhausted (segment starts)");
@@ -1580,13 +1620,8 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
       k_chunk_bounds<<<(unsigned)((n_chunks + 1 + 255) / 256), 256, 0, h->stream>>>(starts, ng, m, chunk, n_chunks, bounds);
       pmb_kernel_end(h);
       PMB_CUDA(h, cudaGetLastError());
-      std::vector<unsigned long long> hb((size_t)n_chunks + 1);
-      PMB_CUDA(h, cudaMemcpyAsync(hb.data(), bounds, hb.size() * 8, cudaMemcpyDeviceToHost, h->stream));
-      PMB_CUDA(h, cudaStreamSynchronize(h->stream));
-      std::vector<unsigned int> counts((size_t)n_chunks);
-      for (int64_t c = 0; c < n_chunks; c++) counts[c] = (unsigned)(hb[c + 1] - hb[c]);
       const WsMark mark = pmb_ws_mark(h);
-      const int rc = run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, 0, counts, slots, (int64_t)ng, ctr, status,
+      const int rc = run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, bounds, n_chunks, 1, slots, (int64_t)ng, ctr, status,
                                      PMB_STRATEGY_SORT);
       if (rc != kSegReduce) return rc;
       pmb_ws_release(h, mark);
@@ -1816,7 +1851,7 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
   unsigned int* status = *status_dev ? *status_dev : (unsigned int*)(zeroed + clear);
   if (at_once) PMB_CUDA(h, cudaMemsetAsync(zeroed, 0, clear + 64, h->stream));
   else PMB_CUDA(h, cudaMemsetAsync(zeroed + clear, 0, 64, h->stream));
-  PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
+  PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
   unsigned long long* a = *k;       // the current word's keys, and where the next pass writes them
   unsigned long long* b = *k_alt;
   bool moved = permuted;            // the order differs from the rows'
@@ -1847,13 +1882,12 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
     P.cap = cap;
     P.n = n;
     P.shift = 8 * (p & 7);
-    P.hashed = 0;
     P.hist = hist_dev + (size_t)p * RADIX;
     P.ticket = (unsigned long long*)z;
     P.lb = (unsigned long long*)(z + 64);
     P.status = status;
     pmb_kernel_begin(h, "sort_pass");
-    k_sort_pass<1><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
+    k_sort_pass<1, false><<<(unsigned)tiles, PassShape<1>::NT, PassShape<1>::SMEM, h->stream>>>(P);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     std::swap(a, b);
