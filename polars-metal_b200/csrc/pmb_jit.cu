@@ -608,6 +608,24 @@ struct Gen {
     }
   }
 
+  // the aggregated columns of position i of the carried values: 8-byte values as they are, narrower ones
+  // in the low bytes of 4, Bool values and validity in the mask
+  void payload(std::ostringstream& b) {
+    bool any = false;
+    for (int c = 0; c < q.n_cols; c++) any |= field_col[c] && (q.col[c].valid || q.col[c].dtype == PMB_BOOL);
+    if (any) b << "  const unsigned mk = mask[i];\n";
+    for (int c = 0; c < q.n_cols; c++) {
+      if (!field_col[c]) continue;
+      const DCol& C = q.col[c];
+      const std::string cs = std::to_string(c), T = ctype(C.dtype);
+      if (C.dtype == PMB_BOOL) b << "  r.v" << cs << " = ((mk >> " << 16 + c << ") & 1u) != 0u;\n";
+      else if (C.elem == 8) b << "  r.v" << cs << " = reinterpret_cast<const " << T << "*>(pay[" << cs << "])[i];\n";
+      else if (C.dtype == PMB_F32) b << "  r.v" << cs << " = __uint_as_float(reinterpret_cast<const unsigned*>(pay[" << cs << "])[i]);\n";
+      else b << "  r.v" << cs << " = (" << T << ")reinterpret_cast<const unsigned*>(pay[" << cs << "])[i];\n";
+      if (C.valid) b << "  r.ok" << cs << " = ((mk >> " << c << ") & 1u) != 0u;\n";
+    }
+  }
+
   // range report of the exact float sums: status bit and the largest exponent seen
   void fxcheck(std::ostringstream& b) {
     for (int i = 0; i < q.n_fields; i++) {
@@ -758,6 +776,9 @@ __device__ __forceinline__ long long j_fdiv_i(long long a, long long b, bool& ok
     store_sg(o);
     o << "}\n__device__ __forceinline__ void j_gather(const JParams& P, long long row, JRow& r) {\n";
     gather(o);
+    o << "}\n__device__ __forceinline__ void j_payload(const unsigned char* const* pay, const unsigned int* mask, "
+         "long long i, JRow& r) {\n";
+    payload(o);
     o << "}\n";
     return o.str();
   }
@@ -1087,19 +1108,38 @@ int pmb_plan_jit_batch(pmb_handle* h, const CompiledQuery& cq, int nt, int nbuf,
 
 // source of the partitioned aggregation: device helpers, the parameter block, the generated row
 // functions and pmb_jit_part.cuh (not the hash kernel)
-static std::string part_source(const CompiledQuery& cq, const JitPlan& J, int key_words, bool cas64) {
+static std::string part_source(const CompiledQuery& cq, const JitPlan& J, int key_words, bool cas64, bool payload) {
   Gen g(cq.dq, J);
   std::string skel(kSkeleton);
   size_t cut = skel.find("__device__ __forceinline__ long long j_gresolve");
-  return "#define JP_W " + std::to_string(key_words) + "\n#define JP_CAS64 " + (cas64 ? "1" : "0") + "\n" +
-         std::string(kDeviceHeader) + "\n" + skel.substr(0, cut) + "\n" + g.build() + "\n" + std::string(kPartSkeleton);
+  return "#define JP_W " + std::to_string(key_words) + "\n#define JP_CAS64 " + (cas64 ? "1" : "0") + "\n#define JP_PAY " +
+         (payload ? "1" : "0") + "\n" + std::string(kDeviceHeader) + "\n" + skel.substr(0, cut) + "\n" + g.build() + "\n" +
+         std::string(kPartSkeleton);
 }
 
-int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, JitPlan* J,
+int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, JitPlan* J,
                         cudaKernel_t* out) {
+  static std::mutex sig_mu;
+  static std::unordered_map<std::string, cudaKernel_t> by_sig;
   int rc = pmb_plan_jit_batch(h, cq, 1024, 1, h->max_smem_optin, J);
   if (rc) return rc;
-  return jit_kernel(h, part_source(cq, *J, key_words, cas64 && key_words == 1), "pmb_jit_part_agg", out);
+  cas64 = cas64 && key_words == 1;
+  std::string sig = hash_signature(cq, *J);
+  sig.push_back((char)(key_words * 4 + cas64 * 2 + payload));
+  {
+    std::lock_guard<std::mutex> lock(sig_mu);
+    auto it = by_sig.find(sig);
+    if (it != by_sig.end()) {
+      *out = it->second;
+      return PMB_OK;
+    }
+  }
+  rc = jit_kernel(h, part_source(cq, *J, key_words, cas64, payload), "pmb_jit_part_agg", out);
+  if (rc == PMB_OK) {
+    std::lock_guard<std::mutex> lock(sig_mu);
+    by_sig[sig] = *out;
+  }
+  return rc;
 }
 
 // the top-level filter's compaction (pmb_jit_compact.cuh): device helpers, the parameter block,
@@ -1219,7 +1259,7 @@ static int debug_compile(const pmb_query* q, const pmb_column* cols, int32_t n_c
       if (rc != PMB_OK) msg = h.err;
       for (int v = 0; v < 3 && rc == PMB_OK; v++) {
         std::vector<char> cubin;
-        if (!jit_compile(part_source(cq, J, v == 2 ? 2 : 1, v == 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
+        if (!jit_compile(part_source(cq, J, v == 2 ? 2 : 1, v == 1, v == 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
         else if (getenv("PMB_JIT_DEBUG") && getenv("PMB_JIT_DEBUG")[0] == '2') fprintf(stderr, "%s\n", msg.c_str());
       }
     } else if (cq.dq.key_bits > 64) {

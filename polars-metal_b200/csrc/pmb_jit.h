@@ -96,11 +96,14 @@ struct JPartH {
   unsigned char* grecs;
   unsigned long long gcap;
   unsigned long long* n_groups;
+  const unsigned char* pay[16];
+  const unsigned int* paymask;
 };
 // the partitioned strategy's aggregation kernel (pmb_jit_part.cuh) for packed keys of
 // `key_words` words (cas64: one-word keys that never equal all ones, claimed by a CAS on the key);
 // J receives the plan (threads, shared-memory record bytes)
-int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, JitPlan* J,
+// payload: the values come with the rows (JPart::pay) instead of by row number
+int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, JitPlan* J,
                         cudaKernel_t* out);
 
 // the batched kernel (pmb_jit_batch.cuh): layout for `nt` threads with `nbuf` unit buffers per

@@ -11,7 +11,8 @@
 //      JP_CAS64: a CAS on the key word claims and publishes at once, no barrier; otherwise a CAS
 //      on the slot's tag word claims, and a row that meets a slot being claimed retries it after
 //      the next barrier instead of waiting), the
-//      row's aggregated columns are gathered by row index (j_gather) and applied to the slot's
+//      row's aggregated columns are gathered by row index (j_gather), or read where the passes have
+//      carried them (j_payload), and applied to the slot's
 //      record with native 32-bit shared atomics (j_shared);
 //   2. the claimed slots (listed in claim order) are written as dense groups: the packed key and
 //      the record converted to the global-record layout (j_store_sg), after one atomic per item
@@ -33,6 +34,8 @@ struct JPart {
   unsigned char* grecs;               // and their records, J_REC bytes each
   unsigned long long gcap;
   unsigned long long* n_groups;
+  const unsigned char* pay[16];       // JP_PAY: the values of every position, by column
+  const unsigned int* paymask;        // and its validity bits and Bool values
 };
 
 #define JP_R 2
@@ -83,7 +86,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
         row[r] = 0;
 #pragma unroll
         for (int w = 0; w < JP_W; w++) k[r][w] = pending[r] ? A.keys[(unsigned long long)w * A.kcap + i] : 0ULL;
-        if (pending[r]) row[r] = A.idx[i];
+        if (!JP_PAY && pending[r]) row[r] = A.idx[i];
       }
 #pragma unroll
       for (int r = 0; r < JP_R; r++)
@@ -174,7 +177,11 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
 #pragma unroll
       for (int r = 0; r < JP_R; r++) {
         if (pending[r]) atomicOr(P.status, PMB_ST_OVERFLOW);
+#if JP_PAY
+        if (found[r] >= 0) j_payload(A.pay, A.paymask, b + (long long)r * J_NT + tid, rw[r]);
+#else
         if (found[r] >= 0) j_gather(P, (long long)row[r], rw[r]);
+#endif
       }
 #pragma unroll
       for (int r = 0; r < JP_R; r++) {

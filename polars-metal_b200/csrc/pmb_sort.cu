@@ -364,6 +364,16 @@ struct PassParams {
   unsigned long long* lb;        // n_tiles x 256 look-back states (tile-major), zeroed
   unsigned long long* ticket;
   unsigned int* status;
+  // values carried along instead of row numbers (PAY): element e of the pass's output row goes to
+  // pay_out[e]; it comes from pay_in[e] by position, or (FIRST) from column data by the row number
+  int n_pay;
+  int pay_elem[PMB_MAX_COLS + 1];             // bytes of an output element: 8 or 4
+  const uint8_t* pay_in[PMB_MAX_COLS + 1];    // null: the mask element (FIRST)
+  int pay_src[PMB_MAX_COLS + 1];              // FIRST: bytes of the column's values (1, 2, 4, 8)
+  uint8_t* pay_out[PMB_MAX_COLS + 1];
+  int n_mask;                                 // the mask's bits, from these bitmaps
+  const uint8_t* mask_bits[2 * PMB_MAX_COLS];
+  int mask_pos[2 * PMB_MAX_COLS];
 };
 
 // Tile shape of a pass, for W-word keys: three (two) CTAs of 12 (16) warps fit an SM's shared memory
@@ -427,7 +437,10 @@ __device__ __forceinline__ unsigned long long digit_lookback(unsigned long long*
 // 795 us (3.0 TB/s of the 6.4 a plain copy reaches); 256 threads x 16 keys with match_any, ranks
 // held to the end and a look-back of one state per step took 1020 us. 128-bit keys, 20M: 259 us,
 // against 552 us. Prefetching the next tile with bulk copies (persistent CTAs) took 900-960 us.
-template <int W, bool HASHED>
+// With PAY a row takes its aggregated values with it through the passes instead of its number: the
+// values move element by element through the tile's buffers to the places the keys went to.
+enum { PAY_NONE = 0, PAY_FIRST = 1, PAY_NEXT = 2 };
+template <int W, bool HASHED, int PAY = PAY_NONE>
 __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
     k_sort_pass(const __grid_constant__ PassParams P) {
   constexpr int NT = PassShape<W>::NT, PER = PassShape<W>::PER, TILE = PassShape<W>::TILE, NW = PassShape<W>::NW;
@@ -449,12 +462,13 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   const unsigned lt = (1u << lane) - 1u;
   PKey<W> k[PER];
   unsigned ix[PER];
+  unsigned short lps[PER];  // PAY: the keys' places in the tile
 #pragma unroll
   for (int j = 0; j < PER; j++)
 #pragma unroll
     for (int w = 0; w < W; w++) k[j].w[w] = e0 + j * 32 < P.n ? __ldcs(&P.kin[(uint64_t)w * P.cap + e0 + j * 32]) : 0ULL;
 #pragma unroll
-  for (int j = 0; j < PER; j++) ix[j] = e0 + j * 32 < P.n ? __ldcs(&P.iin[e0 + j * 32]) : 0u;
+  for (int j = 0; j < PER; j++) ix[j] = PAY != PAY_NEXT && e0 + j * 32 < P.n ? __ldcs(&P.iin[e0 + j * 32]) : 0u;
   unsigned dg[(PER + 3) / 4];  // digits of the key hash, four to a register (a key's own digit is a shift away)
 #pragma unroll
   for (int j = 0; j < (PER + 3) / 4; j++) dg[j] = 0u;
@@ -522,7 +536,8 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
       const unsigned lp = first + below;
 #pragma unroll
       for (int w = 0; w < W; w++) s_key[w * TILE + lp] = k[j].w[w];
-      s_idx[lp] = ix[j];
+      if (PAY == PAY_NONE) s_idx[lp] = ix[j];
+      else lps[j] = (unsigned short)lp;
     }
     __syncwarp();
   }
@@ -532,6 +547,7 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   }
   __syncthreads();
   const int valid = (int)min((long long)TILE, (long long)P.n - tile * TILE);
+  unsigned dest[PER];  // PAY: output rows of the tile's places tid, tid + NT, ...
 #pragma unroll
   for (int j = 0; j < PER; j++) {
     const int i = tid + j * NT;
@@ -542,7 +558,57 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
     const uint64_t g = (uint64_t)(s_out[pass_digit<W>(kk, P.shift, HASHED)] + i);
 #pragma unroll
     for (int w = 0; w < W; w++) P.kout[(uint64_t)w * P.cap + g] = kk.w[w];
-    P.iout[g] = s_idx[i];
+    if (PAY == PAY_NONE) P.iout[g] = s_idx[i];
+    else dest[j] = (unsigned)g;
+  }
+  if (PAY != PAY_NONE) {
+    // an 8-byte element goes through the keys' buffer, a 4-byte one through the row numbers'
+    for (int el = 0; el < P.n_pay; el++) {
+      const uint8_t* src = P.pay_in[el];
+      if (P.pay_elem[el] == 8) {
+        unsigned long long v[PER];
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+          v[j] = e0 + j * 32 < P.n
+                     ? reinterpret_cast<const unsigned long long*>(src)[PAY == PAY_FIRST ? (int64_t)ix[j] : e0 + j * 32]
+                     : 0ULL;
+        __syncthreads();  // the buffer's last readers are done
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+          if (e0 + j * 32 < P.n) s_key[lps[j]] = v[j];
+        __syncthreads();
+        unsigned long long* out = reinterpret_cast<unsigned long long*>(P.pay_out[el]);
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+          if (tid + j * NT < valid) out[dest[j]] = s_key[tid + j * NT];
+      } else {
+        unsigned v[PER];
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+          v[j] = 0u;
+          if (e0 + j * 32 >= P.n) continue;
+          if (PAY == PAY_NEXT) {
+            v[j] = reinterpret_cast<const unsigned*>(src)[e0 + j * 32];
+          } else if (src) {
+            const int b = P.pay_src[el];
+            v[j] = b == 4 ? reinterpret_cast<const unsigned*>(src)[ix[j]]
+                          : b == 2 ? (unsigned)reinterpret_cast<const unsigned short*>(src)[ix[j]] : (unsigned)src[ix[j]];
+          } else {
+            for (int q = 0; q < P.n_mask; q++)
+              v[j] |= ((P.mask_bits[q][ix[j] >> 3] >> (ix[j] & 7)) & 1u) << P.mask_pos[q];
+          }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+          if (e0 + j * 32 < P.n) s_idx[lps[j]] = v[j];
+        __syncthreads();
+        unsigned* out = reinterpret_cast<unsigned*>(P.pay_out[el]);
+#pragma unroll
+        for (int j = 0; j < PER; j++)
+          if (tid + j * NT < valid) out[dest[j]] = s_idx[tid + j * NT];
+      }
+    }
   }
 }
 
@@ -1129,6 +1195,12 @@ __global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constan
                                                             const __grid_constant__ GroupOrder O,
                                                             const unsigned long long* okeys, const unsigned int* idx,
                                                             int64_t start, int64_t m) {
+  // a warp's 32 records come into shared memory word by word, all lanes on the same few records, so
+  // that every sector of a record is fetched once and all loads are in flight together (a lane walking
+  // its own record took 6.8 ms for 49M groups, 1.1 TB/s)
+  extern __shared__ __align__(16) unsigned long long s_rec[];
+  const int lane = threadIdx.x & 31, rw = F.R.q.rec_bytes / 8;
+  unsigned long long* mine = s_rec + (size_t)(threadIdx.x / 32) * 32 * rw;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   // every lane of a warp runs the same number of iterations (warp-wide bit setting)
   const int64_t span = (m + stride - 1) / stride * stride;
@@ -1137,9 +1209,27 @@ __global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constan
     const bool have = p < m;
     PKey<W> k{}, o{};
     const uint8_t* rec = nullptr;
+    const unsigned g = have ? idx[start + p] : 0u;
+    {
+      int r = 0, c = lane;  // word c of record r
+      while (c >= rw) {
+        c -= rw;
+        r++;
+      }
+      __syncwarp();  // the warp's reads of the previous records are done
+      for (int w = 0; w < rw; w++) {
+        const unsigned gr = __shfl_sync(0xffffffffu, g, r & 31);
+        mine[w * 32 + lane] = *(reinterpret_cast<const unsigned long long*>(F.grecs + (uint64_t)gr * F.R.q.rec_bytes) + c);
+        c += 32;
+        while (c >= rw) {
+          c -= rw;
+          r++;
+        }
+      }
+      __syncwarp();
+    }
     if (have) {
-      const uint64_t g = idx[start + p];
-      rec = F.grecs + g * F.R.q.rec_bytes;
+      rec = reinterpret_cast<const uint8_t*>(mine + lane * rw);
       // one-word keys: the packed key back from the sorted order key (read in sequence); two-word
       // order keys are not sorted whole, the group's own packed key is fetched
       for (int w = 0; w < W; w++) (W == 1 ? o : k).w[w] = W == 1 ? okeys[start + p] : F.gkeys[(uint64_t)w * F.gcap + g];
@@ -1225,7 +1315,9 @@ int ordered_finalize(pmb_handle* h, const CompiledQuery& cq, const PartFinParams
   if (m > 0) {
     const int fb = (int)std::max<int64_t>(1, std::min<int64_t>((m + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
     pmb_kernel_begin(h, "ordered_finalize");
-    k_ordered_finalize<W><<<fb, ST_NT, 0, h->stream>>>(F, O, k0, i0, start, m);
+    const size_t fsmem = (size_t)ST_NT * F.R.q.rec_bytes;
+    PMB_CUDA(h, cudaFuncSetAttribute(k_ordered_finalize<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+    k_ordered_finalize<W><<<fb, ST_NT, fsmem, h->stream>>>(F, O, k0, i0, start, m);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
   }
@@ -1293,11 +1385,48 @@ static bool widen_fx(CompiledQuery& cq, const unsigned int* st) {
 template <int W>
 int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_result* r, int64_t part_groups);
 
+// The values that the partition passes carry: per element its column (-1: the mask of validity bits, bit
+// c, and Bool values, bit 16 + c), its bytes, where it is now and where the next pass puts it.
+struct Payload {
+  int n = 0;
+  int col[PMB_MAX_COLS + 1];
+  int elem[PMB_MAX_COLS + 1];
+  const uint8_t* cur[PMB_MAX_COLS + 1];
+  uint8_t* buf[2][PMB_MAX_COLS + 1];
+  bool mask = false;
+  int row_bytes = 0;
+};
+
+// Carrying pays where the gathers by row number miss L2: a random read costs a whole DRAM access (42 G/s
+// on 1.6 GB, whatever its width or cache hint), 400M of them 9.5 of the aggregation's 11.5 ms for 200M
+// rows with two value columns. Every pass moves the values instead. Up to PAY_BYTES a row, and from
+// PAY_MIN bytes of value columns (about half of L2) on.
+constexpr int PAY_BYTES = 32;
+constexpr int64_t PAY_MIN = 64LL << 20;
+bool plan_payload(const DQuery& q, Payload* p) {
+  unsigned used = 0;
+  for (int f = 0; f < q.n_fields; f++)
+    if (q.field[f].kind != F_LEN) used |= 1u << q.field[f].col;
+  auto add = [&](int col, int elem) {
+    p->col[p->n] = col;
+    p->elem[p->n++] = elem;
+    p->row_bytes += elem;
+  };
+  for (int c = 0; c < q.n_cols; c++) {
+    if (!((used >> c) & 1u)) continue;
+    if (q.col[c].elem) add(c, q.col[c].elem == 8 ? 8 : 4);
+    p->mask |= q.col[c].valid != nullptr || q.col[c].elem == 0;
+  }
+  if (p->mask) add(-1, 4);
+  return p->n > 0 && p->row_bytes <= PAY_BYTES && q.n_rows * p->row_bytes >= PAY_MIN;
+}
+
 // the aggregation of the partitioned strategy over keys / row indices sorted by partition
 template <int W>
 int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_result* r, const unsigned long long* keys,
                  const unsigned int* idx, uint64_t cap, int64_t m, const unsigned long long* pstart, int64_t n_parts,
-                 int run, int slots, int64_t groups, unsigned long long* ctr, unsigned int* status, int strategy = PMB_STRATEGY_PARTITIONED) {
+                 int run, int slots, int64_t groups, unsigned long long* ctr, unsigned int* status,
+                 int strategy = PMB_STRATEGY_PARTITIONED, const Payload* pay = nullptr) {
   DQuery& q = cq.dq;
   const int n_out = q.n_keys + q.n_aggs;
   PartParams A;
@@ -1346,7 +1475,7 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
     // without NVRTC (or for a signature it cannot take) the prebuilt kernel does both
     JitPlan J;
     cudaKernel_t jk = nullptr;
-    if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, &J, &jk) != PMB_OK) {
+    if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, pay != nullptr, &J, &jk) != PMB_OK) {
       jk = nullptr;  // the prebuilt kernel instead (the compile error stays readable in pmb_last_error)
     }
     unsigned long long* gkeys = nullptr;
@@ -1385,6 +1514,11 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         JA.grecs = grecs;
         JA.gcap = (unsigned long long)out_cap;
         JA.n_groups = A.n_groups;
+        if (pay) {
+          for (int e = 0; e < pay->n; e++)
+            if (pay->col[e] < 0) JA.paymask = (const unsigned int*)pay->cur[e];
+            else JA.pay[pay->col[e]] = pay->cur[e];
+        }
         const size_t jsmem = (((size_t)slots * 4 + 15) & ~(size_t)15) + (size_t)slots * (8 * W + J.srec + 2);
         PMB_CUDA(h, cudaFuncSetAttribute((const void*)jk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
         void* args[] = {&JA};
@@ -1535,14 +1669,33 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   const int64_t tiles = (m + ST_TILE - 1) / ST_TILE;
   const int64_t ptiles = (m + PassShape<W>::TILE - 1) / PassShape<W>::TILE;
   constexpr size_t pass_smem = PassShape<W>::SMEM;
+  // the partition passes carry the aggregated values when the run-time compiled aggregation can take
+  // them and the buffers fit
+  Payload pay;
+  bool carry = part_groups > 0 && m > 1 && plan_payload(q, &pay) && pmb_jit_enabled(1LL << 40);
+  if (carry) {
+    JitPlan J;
+    cudaKernel_t jk;
+    const std::string keep_err = h->err;
+    carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, &J, &jk) == PMB_OK;
+    const WsMark mark = pmb_ws_mark(h);
+    for (int b = 0; carry && b < passes; b++)
+      for (int e = 0; carry && e < pay.n; e++) {
+        pay.buf[b][e] = (uint8_t*)pmb_ws_alloc(h, (size_t)m * pay.elem[e] + 16);
+        carry = pay.buf[b][e] != nullptr;
+      }
+    if (!carry) pmb_ws_release(h, mark);
+    h->err = keep_err;
+  }
   const auto pass = part_groups > 0 ? k_sort_pass<W, true> : k_sort_pass<W, false>;
   PMB_CUDA(h, cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
   int done = 0;
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
     for (int d = 0; d < RADIX; d++) constant |= hh[(size_t)p * RADIX + d] == (unsigned)m;
-    if (constant) continue;
+    if (constant && !carry) continue;
     PassParams P;
+    P.n_pay = 0;
     P.kin = k0;
     P.kout = k1;
     P.iin = i0;
@@ -1557,7 +1710,37 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     PMB_CUDA(h, cudaMemsetAsync(lb, 0, (size_t)ptiles * RADIX * 8, h->stream));
     PMB_CUDA(h, cudaMemsetAsync(ctr + 1, 0, 8, h->stream));
     pmb_kernel_begin(h, "sort_pass");
-    pass<<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
+    if (carry) {
+      P.n_pay = pay.n;
+      P.n_mask = 0;
+      for (int e = 0; e < pay.n; e++) {
+        const int c = pay.col[e];
+        P.pay_elem[e] = pay.elem[e];
+        P.pay_src[e] = c >= 0 ? q.col[c].elem : 0;
+        P.pay_in[e] = p > 0 ? pay.cur[e] : c >= 0 ? q.col[c].data : nullptr;
+        P.pay_out[e] = pay.buf[p][e];
+        pay.cur[e] = pay.buf[p][e];
+      }
+      unsigned used = 0;
+      for (int f = 0; f < q.n_fields; f++)
+        if (q.field[f].kind != F_LEN) used |= 1u << q.field[f].col;
+      for (int c = 0; c < q.n_cols; c++) {
+        if (!((used >> c) & 1u)) continue;
+        if (q.col[c].valid) {
+          P.mask_bits[P.n_mask] = q.col[c].valid;
+          P.mask_pos[P.n_mask++] = c;
+        }
+        if (q.col[c].elem == 0) {
+          P.mask_bits[P.n_mask] = q.col[c].data;
+          P.mask_pos[P.n_mask++] = 16 + c;
+        }
+      }
+      const auto moving = p == 0 ? k_sort_pass<W, true, PAY_FIRST> : k_sort_pass<W, true, PAY_NEXT>;
+      PMB_CUDA(h, cudaFuncSetAttribute(moving, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
+      moving<<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
+    } else {
+      pass<<<(unsigned)ptiles, PassShape<W>::NT, pass_smem, h->stream>>>(P);
+    }
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     std::swap(k0, k1);
@@ -1573,7 +1756,8 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     // hash spreads them, so a run stays far from the whole table), at least one partition each
     const int64_t rows = std::max<int64_t>(1, m / n_parts);
     const int run = (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, slots / 2 / rows));
-    return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pstart, n_parts, run, slots, part_groups, ctr, status);
+    return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pstart, n_parts, run, slots, part_groups, ctr, status,
+                           PMB_STRATEGY_PARTITIONED, carry ? &pay : nullptr);
   }
   // segment starts
   unsigned int* starts = (unsigned int*)pmb_ws_alloc(h, (size_t)(m + 2) * 4);

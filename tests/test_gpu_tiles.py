@@ -276,3 +276,38 @@ def test_direct_rows(n, groups, wide):
     pred = {"kind": "Compare", "op": "Ne", "lhs": {"kind": "Column", "name": "x"}, "rhs": {"kind": "LiteralI64", "value": 3}}
     got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, keys, aggs, pred)
     assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, pred), len(keys), aggs)
+
+
+# values carried through the partition passes (64 MB of them and more): every width, nulls, Bool values,
+# a filter (row numbers with gaps), one and two passes, one- and two-word keys, a row too wide for it
+@pytest.mark.parametrize("groups", [20_000, 900_000])
+@pytest.mark.parametrize("case", ["narrow", "nulls", "filter", "wide key", "too wide"])
+def test_carried_values(case, groups):
+    rng = np.random.default_rng(groups)
+    n = 5_000_011 if case == "narrow" else 3_400_003
+    k = rng.integers(0, groups, n)
+    cols = {"k": (k * (2**40 if case == "wide key" else 1), None), "a": (rng.integers(-100, 100, n).astype(np.int8), None),
+            "c": (rng.integers(-9, 9, n), None), "f": (rng.standard_normal(n).astype(np.float32), None)}
+    aggs = [("Sum", "a", "a_s"), ("Min", "f", "f_lo"), ("Sum", "f", "f_s"), ("Max", "c", "c_hi"), ("Len", None, "n")]
+    keys, pred = ["k"], None
+    if case != "narrow":
+        cols["f"] = (cols["f"][0], pack(rng.random(n) > 0.2))
+        cols["u"] = (rng.integers(0, 60_000, n).astype(np.uint16), pack(rng.random(n) > 0.5))
+        aggs += [("Mean", "u", "u_m"), ("Count", "u", "u_c")]
+    if case == "filter":
+        pred = {"kind": "Compare", "op": "Gt", "lhs": {"kind": "Column", "name": "c"}, "rhs": {"kind": "LiteralI64", "value": -6}}
+        cols["b"] = (pack(rng.random(n) > 0.5), pack(rng.random(n) > 0.1), A.BOOL, n)
+        aggs += [("Sum", "b", "b_s")]
+    if case == "wide key":
+        cols["j"] = ((k % 7 * 2**28).astype(np.int32), None)
+        keys.append("j")
+    if case == "too wide":
+        for i in range(3):
+            cols[f"x{i}"] = (rng.integers(-2**40, 2**40, n), None)
+            aggs.append(("Min", f"x{i}", f"x{i}_lo"))
+    inv = {d: t for t, d in A.NUMPY_NAME.items()}
+    full = {c: d if len(d) > 2 else (d[0], d[1], inv[d[0].dtype.name], n) for c, d in cols.items()}
+    data = {c: N.ColumnData(d, v, dtype=t, length=m) for c, (d, v, t, m) in full.items()}
+    got = N.groupby(data, keys, aggs, pred, strategy="partitioned")
+    assert got.strategy == "partitioned"
+    assert_results_match(as_dict(got), pyoracle.groupby(full, keys, aggs, pred), len(keys), aggs, case)
