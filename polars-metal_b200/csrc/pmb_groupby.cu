@@ -119,6 +119,11 @@ __global__ void __launch_bounds__(F_NT) k_sketch(const __grid_constant__ FrontPa
     k = pack_key64(q, t, row);
   }
   if (k == PMB_EMPTY64) k = PMB_EMPTY64 - 1;
+  // a warp's samples of one key go in as one (a few keys' counters would each take tens of thousands of
+  // additions, about one a nanosecond)
+  const unsigned am = __activemask();
+  const unsigned same = __match_any_sync(am, k);
+  if ((threadIdx.x & 31) != __ffs(same) - 1) return;
   const uint32_t mask = (uint32_t)F.slots - 1u;
   uint32_t s = (uint32_t)pmb_fmix64(k) & mask;
   for (int p = 0; p < F.slots; p++) {
@@ -130,7 +135,7 @@ __global__ void __launch_bounds__(F_NT) k_sketch(const __grid_constant__ FrontPa
     }
     s = (s + 1) & mask;
   }
-  atomicAdd(&F.set_cnt[s], 1u);
+  atomicAdd(&F.set_cnt[s], (unsigned)__popc(same));
 }
 
 // distinct count, singletons, doubletons and the histogram of per-key sample counts (its first bins

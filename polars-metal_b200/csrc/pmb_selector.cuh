@@ -17,7 +17,7 @@ static_assert(N_PARAMS == PMB_SELECTOR_PARAMS, "parameter layout");
 
 constexpr int SAMPLE = 4096;
 constexpr int F_NT = 1024;
-constexpr int TSLOTS = 8192;  // sample counts: slots (count << 32 | 32-bit key fingerprint), dynamic smem
+constexpr int TSLOTS = 8192;  // sample counts: slots of a 32-bit key fingerprint and a count, dynamic smem
 constexpr int HLL = 256;
 constexpr int BUCKETS = 1024;
 
@@ -60,6 +60,10 @@ __device__ __forceinline__ void features_body(const DQuery& q, const unsigned lo
   __shared__ double s_z;
   __shared__ int s_zeros;
   const int tid = threadIdx.x;
+  // fingerprints, then counts: two 32-bit tables, so that a count is a native shared add (a 64-bit one is
+  // a compare-and-swap loop, on which the samples of a few keys queued for 40 us)
+  unsigned int* s_fp = reinterpret_cast<unsigned int*>(s_slot);
+  unsigned int* s_num = s_fp + TSLOTS;
   for (int i = tid; i < TSLOTS; i += F_NT) s_slot[i] = 0ULL;
   for (int i = tid; i < HLL; i += F_NT) s_hll[i] = 0u;
   for (int i = tid; i < BUCKETS; i += F_NT) s_bkt[i] = 0u;
@@ -79,17 +83,14 @@ __device__ __forceinline__ void features_body(const DQuery& q, const unsigned lo
     atomicMax(&s_hll[reg], rank);
     atomicAdd(&s_bkt[(h >> 20) & (BUCKETS - 1)], 1u);
     // exact counts by 32-bit fingerprint (a collision among 4096 samples is rare and only blurs a
-    // feature); a slot holds count << 32 | fingerprint
+    // feature)
     const unsigned fp = (unsigned)(h >> 32) | 1u;
     unsigned s = (unsigned)(h >> 11) & (TSLOTS - 1);
     for (int p = 0; p < TSLOTS; p++) {
-      unsigned long long cur = s_slot[s];
-      if (cur == 0ULL) {
-        cur = atomicCAS(&s_slot[s], 0ULL, (1ULL << 32) | fp);
-        if (cur == 0ULL) break;
-      }
-      if ((unsigned)cur == fp) {
-        atomicAdd(&s_slot[s], 1ULL << 32);
+      unsigned cur = *reinterpret_cast<volatile unsigned int*>(&s_fp[s]);
+      if (cur == 0u) cur = atomicCAS(&s_fp[s], 0u, fp);
+      if (cur == 0u || cur == fp) {
+        atomicAdd(&s_num[s], 1u);
         break;
       }
       s = (s + 1) & (TSLOTS - 1);
@@ -100,7 +101,7 @@ __device__ __forceinline__ void features_body(const DQuery& q, const unsigned lo
   // a shared atomic per key and bin serialised the CTA on ten addresses)
   unsigned cnt[7] = {0, 0, 0, 0, 0, 0, 0}, top = 0, btop = 0;
   for (int i = tid; i < TSLOTS; i += F_NT) {
-    const unsigned c = (unsigned)(s_slot[i] >> 32);
+    const unsigned c = s_num[i];
     if (!c) continue;
     cnt[0]++;  // distinct
     cnt[1] += c == 1;
