@@ -1108,16 +1108,16 @@ int pmb_plan_jit_batch(pmb_handle* h, const CompiledQuery& cq, int nt, int nbuf,
 
 // source of the partitioned aggregation: device helpers, the parameter block, the generated row
 // functions and pmb_jit_part.cuh (not the hash kernel)
-static std::string part_source(const CompiledQuery& cq, const JitPlan& J, int key_words, bool cas64, bool payload) {
+static std::string part_source(const CompiledQuery& cq, const JitPlan& J, int key_words, bool cas64, bool payload, int ctas) {
   Gen g(cq.dq, J);
   std::string skel(kSkeleton);
   size_t cut = skel.find("__device__ __forceinline__ long long j_gresolve");
   return "#define JP_W " + std::to_string(key_words) + "\n#define JP_CAS64 " + (cas64 ? "1" : "0") + "\n#define JP_PAY " +
-         (payload ? "1" : "0") + "\n" + std::string(kDeviceHeader) + "\n" + skel.substr(0, cut) + "\n" + g.build() + "\n" +
+         (payload ? "1" : "0") + "\n#define JP_CTAS " + std::to_string(ctas) + "\n" + std::string(kDeviceHeader) + "\n" + skel.substr(0, cut) + "\n" + g.build() + "\n" +
          std::string(kPartSkeleton);
 }
 
-int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, JitPlan* J,
+int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, int ctas, JitPlan* J,
                         cudaKernel_t* out) {
   static std::mutex sig_mu;
   static std::unordered_map<std::string, cudaKernel_t> by_sig;
@@ -1125,7 +1125,7 @@ int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, b
   if (rc) return rc;
   cas64 = cas64 && key_words == 1;
   std::string sig = hash_signature(cq, *J);
-  sig.push_back((char)(key_words * 4 + cas64 * 2 + payload));
+  sig.push_back((char)(ctas * 16 + key_words * 4 + cas64 * 2 + payload));
   {
     std::lock_guard<std::mutex> lock(sig_mu);
     auto it = by_sig.find(sig);
@@ -1134,7 +1134,7 @@ int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, b
       return PMB_OK;
     }
   }
-  rc = jit_kernel(h, part_source(cq, *J, key_words, cas64, payload), "pmb_jit_part_agg", out);
+  rc = jit_kernel(h, part_source(cq, *J, key_words, cas64, payload, ctas), "pmb_jit_part_agg", out);
   if (rc == PMB_OK) {
     std::lock_guard<std::mutex> lock(sig_mu);
     by_sig[sig] = *out;
@@ -1259,7 +1259,7 @@ static int debug_compile(const pmb_query* q, const pmb_column* cols, int32_t n_c
       if (rc != PMB_OK) msg = h.err;
       for (int v = 0; v < 3 && rc == PMB_OK; v++) {
         std::vector<char> cubin;
-        if (!jit_compile(part_source(cq, J, v == 2 ? 2 : 1, v == 1, v == 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
+        if (!jit_compile(part_source(cq, J, v == 2 ? 2 : 1, v == 1, v == 1, v == 1 ? 2 : 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
         else if (getenv("PMB_JIT_DEBUG") && getenv("PMB_JIT_DEBUG")[0] == '2') fprintf(stderr, "%s\n", msg.c_str());
       }
     } else if (cq.dq.key_bits > 64) {

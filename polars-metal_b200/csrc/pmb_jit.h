@@ -103,7 +103,7 @@ struct JPartH {
 // `key_words` words (cas64: one-word keys that never equal all ones, claimed by a CAS on the key);
 // J receives the plan (threads, shared-memory record bytes)
 // payload: the values come with the rows (JPart::pay) instead of by row number
-int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, JitPlan* J,
+int pmb_jit_part_kernel(pmb_handle* h, const CompiledQuery& cq, int key_words, bool cas64, bool payload, int ctas, JitPlan* J,
                         cudaKernel_t* out);
 
 // the batched kernel (pmb_jit_batch.cuh): layout for `nt` threads with `nbuf` unit buffers per

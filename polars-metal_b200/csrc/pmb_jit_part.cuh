@@ -1,6 +1,6 @@
 // pmb_jit_part.cuh — the aggregation step of the partitioned strategy, compiled at run time for
 // one query signature (follows pmb_jit_skeleton.cuh's parameter block and the generated row
-// functions in the same NVRTC source; JP_W, the words of a packed key, and JP_CAS64 are defined
+// functions in the same NVRTC source; JP_W, the words of a packed key, JP_CAS64, JP_PAY and JP_CTAS are defined
 // before it).
 //
 // Input: the kept rows as packed keys and row indices, ordered by partition (the top bits of the
@@ -38,7 +38,13 @@ struct JPart {
   const unsigned int* paymask;        // and its validity bits and Bool values
 };
 
-#define JP_R 2
+// Bound by the chain of an item (keys, table, records, the groups' place, their writes) and its barriers,
+// not by bytes. The next item's ticket and bounds come in during the item, carried values with the keys.
+// With at most 24 carried bytes a row, two CTAs of 1024 threads and half a table share an SM, a row per
+// thread (JP_CTAS 2): one's barriers hide behind the other's rows. 200M rows in 50M groups: 6.92 ms with
+// two rows and the ticket taken between the items, 6.46 ms with three and the next ticket early, 5.95 ms
+// as two CTAs of 512 threads and two rows, 5.47 ms so; 12M rows in 3.8M groups 652, 596, 535 and 496 us.
+#define JP_R (JP_CTAS == 2 ? 1 : 3)
 
 __device__ __forceinline__ unsigned long long jp_hash(const unsigned long long* k) {
   unsigned long long h = pmb_fmix64(k[0]);
@@ -46,7 +52,7 @@ __device__ __forceinline__ unsigned long long jp_hash(const unsigned long long* 
   return h;
 }
 
-extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __grid_constant__ JPart A) {
+extern "C" __global__ void __launch_bounds__(J_NT, JP_CTAS) pmb_jit_part_agg(const __grid_constant__ JPart A) {
   extern __shared__ __align__(16) unsigned char sm[];
   const JParams& P = A.qp;
   const int S = A.slots, tid = threadIdx.x;
@@ -54,7 +60,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
   unsigned long long* tkey = reinterpret_cast<unsigned long long*>(sm + ((S * 4 + 15) & ~15));  // JP_W x S
   unsigned char* srec = reinterpret_cast<unsigned char*>(tkey + (size_t)JP_W * S);           // S x J_SREC
   unsigned short* list = reinterpret_cast<unsigned short*>(srec + (size_t)S * J_SREC);       // S
-  __shared__ long long s_item;
+  __shared__ long long s_item, s_ps, s_pe;
   __shared__ unsigned long long s_base;
   __shared__ unsigned int s_total;  // claimed slots of the current item
   for (int i = tid; i < S; i += J_NT) {
@@ -62,18 +68,36 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
     if (JP_CAS64) tkey[i] = 0xFFFFFFFFFFFFFFFFULL;
   }
   for (int w = tid; w < S * J_SREC_WORDS; w += J_NT) reinterpret_cast<unsigned int*>(srec)[w] = J_SIDENT[w % J_SREC_WORDS];
-  if (tid == 0) s_total = 0u;
+  // thread 0: a ticket, and the rows of its item
+  auto bounds = [&](long long it, long long& ps, long long& pe) {
+    ps = pe = 0;
+    if (it < A.n_items) {
+      ps = (long long)A.pstart[it * A.run];
+      pe = (long long)A.pstart[min(A.n_parts, (it + 1) * A.run)];
+    }
+  };
+  long long next = 0, nps = 0, npe = 0;
+  if (tid == 0) {
+    s_total = 0u;
+    s_item = (long long)atomicAdd(A.ticket, 1ULL);
+    bounds(s_item, s_ps, s_pe);
+  }
   for (;;) {
-    __syncthreads();
-    if (tid == 0) s_item = (long long)atomicAdd(A.ticket, 1ULL);
     __syncthreads();
     const long long it = s_item;
     if (it >= A.n_items) break;
-    const long long ps = (long long)A.pstart[it * A.run], pe = (long long)A.pstart[min(A.n_parts, (it + 1) * A.run)];
+    const long long ps = s_ps, pe = s_pe;
+    // the next item's ticket comes in while this item is aggregated, its bounds while this one's
+    // groups are written; after an overflow the call starts again, and the items left are not taken
+    if (tid == 0) {
+      next = (long long)atomicAdd(A.ticket, 1ULL);
+      if (*reinterpret_cast<volatile unsigned int*>(P.status) & PMB_ST_OVERFLOW) next = A.n_items;
+    }
     for (long long b = ps; b < pe; b += (long long)J_NT * JP_R) {
       unsigned long long k[JP_R][JP_W];
       unsigned slot[JP_R], row[JP_R], probes[JP_R];
       bool pending[JP_R], claimed[JP_R];
+      JRow rw[JP_R];
       int found[JP_R];
 #pragma unroll
       for (int r = 0; r < JP_R; r++) {
@@ -88,6 +112,11 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
         for (int w = 0; w < JP_W; w++) k[r][w] = pending[r] ? A.keys[(unsigned long long)w * A.kcap + i] : 0ULL;
         if (!JP_PAY && pending[r]) row[r] = A.idx[i];
       }
+#if JP_PAY
+#pragma unroll
+      for (int r = 0; r < JP_R; r++)
+        if (pending[r]) j_payload(A.pay, A.paymask, b + (long long)r * J_NT + tid, rw[r]);
+#endif
 #pragma unroll
       for (int r = 0; r < JP_R; r++)
         if (pending[r]) slot[r] = (unsigned)(((jp_hash(k[r]) & 0xFFFFFFFFULL) * (unsigned long long)S) >> 32);
@@ -173,15 +202,10 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
           if (claimed[r]) list[at + __popc(bl & ((1u << lane) - 1u))] = (unsigned short)found[r];
         }
       }
-      JRow rw[JP_R];
 #pragma unroll
       for (int r = 0; r < JP_R; r++) {
         if (pending[r]) atomicOr(P.status, PMB_ST_OVERFLOW);
-#if JP_PAY
-        if (found[r] >= 0) j_payload(A.pay, A.paymask, b + (long long)r * J_NT + tid, rw[r]);
-#else
-        if (found[r] >= 0) j_gather(P, (long long)row[r], rw[r]);
-#endif
+        if (!JP_PAY && found[r] >= 0) j_gather(P, (long long)row[r], rw[r]);
       }
 #pragma unroll
       for (int r = 0; r < JP_R; r++) {
@@ -193,6 +217,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
     // the item is complete: its groups go to the dense group arrays
     __syncthreads();
     const unsigned total = s_total;
+    if (tid == 0) bounds(next, nps, npe);
     if (tid == 0) s_base = total ? atomicAdd(A.n_groups, (unsigned long long)total) : 0ULL;
     __syncthreads();
     const unsigned long long base = s_base;
@@ -210,7 +235,11 @@ extern "C" __global__ void __launch_bounds__(J_NT, 1) pmb_jit_part_agg(const __g
       if (JP_CAS64) tkey[sl] = 0xFFFFFFFFFFFFFFFFULL;
       for (int w = 0; w < J_SREC_WORDS; w++) reinterpret_cast<unsigned int*>(srec + (size_t)sl * J_SREC)[w] = J_SIDENT[w];
     }
-    if (tid == 0) s_total = 0u;  // every thread read it before the s_base barrier
-    __syncthreads();
+    if (tid == 0) {  // every thread read these before the s_base barrier
+      s_total = 0u;
+      s_item = next;
+      s_ps = nps;
+      s_pe = npe;
+    }
   }
 }

@@ -1421,6 +1421,10 @@ bool plan_payload(const DQuery& q, Payload* p) {
   return p->n > 0 && p->row_bytes <= PAY_BYTES && q.n_rows * p->row_bytes >= PAY_MIN;
 }
 
+// CTAs an SM of the run-time compiled aggregation: two where a row's carried values fit the 32 registers of
+// their threads (pmb_jit_part.cuh has both sides' times), else one
+inline int part_ctas(int W, const Payload* pay) { return pay && W == 1 && pay->row_bytes <= 24 ? 2 : 1; }
+
 // the aggregation of the partitioned strategy over keys / row indices sorted by partition
 template <int W>
 int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_result* r, const unsigned long long* keys,
@@ -1452,6 +1456,8 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
   const size_t smem = pa_layout(slots, W, q.rec_bytes, n_out, A.stage_bytes).bytes;
   PMB_CUDA(h, cudaFuncSetAttribute(k_part_agg<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t out_cap = std::min<int64_t>(std::max<int64_t>(m, 1), 2 * groups + 65536);
+  // should the smaller tables of two CTAs not hold an item's groups, one CTA with the whole table follows
+  int ctas = part_ctas(W, pay);
   for (int attempt = 0;; attempt++) {
     if (attempt >= 6) return pmb_fail(h, PMB_E_CUDA, "partitioned strategy did not converge");
     const WsMark mark = pmb_ws_mark(h);
@@ -1475,7 +1481,7 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
     // without NVRTC (or for a signature it cannot take) the prebuilt kernel does both
     JitPlan J;
     cudaKernel_t jk = nullptr;
-    if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, pay != nullptr, &J, &jk) != PMB_OK) {
+    if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, pay != nullptr, ctas, &J, &jk) != PMB_OK) {
       jk = nullptr;  // the prebuilt kernel instead (the compile error stays readable in pmb_last_error)
     }
     unsigned long long* gkeys = nullptr;
@@ -1488,6 +1494,12 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
     if (m > 0) {
       const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(A.n_items, h->sm_count));
       if (jk) {
+        int jslots = slots, jrun = run;
+        if (ctas == 2) {
+          jslots = std::min(slots, (h->max_smem_optin / 2 - 1536) / (4 + 8 * W + J.srec + 2) & ~7);
+          jrun = (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, jslots / 2 / std::max<int64_t>(1, m / n_parts)));
+        }
+        const int64_t jitems = (n_parts + jrun - 1) / jrun;
         JPartH JA;
         memset(&JA, 0, sizeof(JA));
         for (int c = 0; c < q.n_cols; c++) {
@@ -1506,9 +1518,9 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         JA.idx = idx;
         JA.pstart = A.pstart;
         JA.n_parts = n_parts;
-        JA.run = run;
-        JA.n_items = A.n_items;
-        JA.slots = slots;
+        JA.run = jrun;
+        JA.n_items = jitems;
+        JA.slots = jslots;
         JA.ticket = A.ticket;
         JA.gkeys = gkeys;
         JA.grecs = grecs;
@@ -1519,11 +1531,11 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
             if (pay->col[e] < 0) JA.paymask = (const unsigned int*)pay->cur[e];
             else JA.pay[pay->col[e]] = pay->cur[e];
         }
-        const size_t jsmem = (((size_t)slots * 4 + 15) & ~(size_t)15) + (size_t)slots * (8 * W + J.srec + 2);
+        const size_t jsmem = (((size_t)jslots * 4 + 15) & ~(size_t)15) + (size_t)jslots * (8 * W + J.srec + 2);
         PMB_CUDA(h, cudaFuncSetAttribute((const void*)jk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jsmem));
         void* args[] = {&JA};
         pmb_kernel_begin(h, "part_agg");
-        PMB_CUDA(h, cudaLaunchKernel((const void*)jk, dim3(grid), dim3(J.nt), args, jsmem, h->stream));
+        PMB_CUDA(h, cudaLaunchKernel((const void*)jk, dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>(jitems, (int64_t)h->sm_count * ctas))), dim3(J.nt), args, jsmem, h->stream));
         pmb_kernel_end(h);
       } else {
         pmb_kernel_begin(h, "part_agg");
@@ -1572,6 +1584,10 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
       pmb_ws_release(h, mark);
       if ((int64_t)ng > out_cap) {  // more groups than output rows: the exact upper bound next
         out_cap = std::max<int64_t>(m, 1);
+        continue;
+      }
+      if (ctas > 1) {
+        ctas = 1;
         continue;
       }
       // a partition had more groups than its table: the sort strategy instead (the sort's own
@@ -1677,7 +1693,7 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     JitPlan J;
     cudaKernel_t jk;
     const std::string keep_err = h->err;
-    carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, &J, &jk) == PMB_OK;
+    carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, part_ctas(W, &pay), &J, &jk) == PMB_OK;
     const WsMark mark = pmb_ws_mark(h);
     for (int b = 0; carry && b < passes; b++)
       for (int e = 0; carry && e < pay.n; e++) {
