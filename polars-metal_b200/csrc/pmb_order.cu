@@ -13,6 +13,8 @@
 //                       most significant column highest. Columns that do not fit 128 bits go to
 //                       further rounds, least significant first; every round is a stable sort of
 //                       the previous round's order, so the rounds compose;
+//                       A wide column of few distinct values (measurements of limited resolution)
+//                       goes in as the value's rank among them (order_dict);
 //   3. k_order_encode — keys of the rows in the current order, with the digit histograms;
 //   4. pmb_sort_pairs — the group-by sort's LSD onesweep passes over the digits that vary;
 //   5. k_order_gather — the slice of the sorted rows, a warp per 32 output rows so that each
@@ -73,6 +75,9 @@ struct OrderRange {
   unsigned long long hi[PMB_MAX_KEYS];
   unsigned long long nulls[PMB_MAX_KEYS];
   unsigned int any[PMB_MAX_KEYS];
+  unsigned int distinct[PMB_MAX_KEYS];  // of RS_ROWS sampled rows: distinct values, and those that
+  unsigned int f1[PMB_MAX_KEYS];        // occurred once
+  unsigned int f2[PMB_MAX_KEYS];        // and twice
 };
 
 __device__ __forceinline__ unsigned long long warp_min64(unsigned long long v) {
@@ -163,11 +168,52 @@ __device__ __forceinline__ void null_flags(const NullFlagCols& V, int64_t n, uns
   }
 }
 
-// the sort columns' ranges (blockIdx.y 0) and which columns have nulls (blockIdx.y 1)
+// Distinct values of a sort column among RS_ROWS rows spread over the table, by 32-bit fingerprint.
+constexpr int RS_ROWS = 1024, RS_SLOTS = 2048;
+__device__ void sample_column(const SortCols& C, int c, int64_t n, OrderRange* out) {
+  __shared__ unsigned int s_fp[RS_SLOTS], s_num[RS_SLOTS];
+  for (int i = threadIdx.x; i < RS_SLOTS; i += OR_NT) {
+    s_fp[i] = 0u;
+    s_num[i] = 0u;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < RS_ROWS; i += OR_NT) {
+    const int64_t r = n / RS_ROWS * i;
+    if (!pmb_valid_bit(C.valid[c], r)) continue;
+    const unsigned long long hk = pmb_fmix64(order_key(pmb_load_bits(C.data[c], C.elem[c], r), C.dtype[c]));
+    const unsigned fp = (unsigned)(hk >> 32) | 1u;
+    unsigned s = (unsigned)hk & (RS_SLOTS - 1);
+    for (int p = 0; p < RS_SLOTS; p++) {
+      const unsigned cur = atomicCAS(&s_fp[s], 0u, fp);
+      if (cur == 0u || cur == fp) {
+        atomicAdd(&s_num[s], 1u);
+        break;
+      }
+      s = (s + 1) & (RS_SLOTS - 1);
+    }
+  }
+  __syncthreads();
+  unsigned d = 0, f1 = 0, f2 = 0;
+  for (int i = threadIdx.x; i < RS_SLOTS; i += OR_NT) {
+    d += s_num[i] > 0;
+    f1 += s_num[i] == 1;
+    f2 += s_num[i] == 2;
+  }
+  if (d) atomicAdd(&out->distinct[c], d);
+  if (f1) atomicAdd(&out->f1[c], f1);
+  if (f2) atomicAdd(&out->f2[c], f2);
+}
+
+// the sort columns' ranges (blockIdx.y 0), which columns have nulls (blockIdx.y 1) and, with a third grid
+// row, how many distinct values a sample of each has
 __global__ void __launch_bounds__(OR_NT) k_order_range(const __grid_constant__ SortCols C, int64_t n, OrderRange* out,
                                                        const __grid_constant__ NullFlagCols V, unsigned int* flags) {
   if (blockIdx.y == 1) {
     null_flags(V, n, flags);
+    return;
+  }
+  if (blockIdx.y == 2) {
+    if (blockIdx.x < C.n) sample_column(C, blockIdx.x, n, out);
     return;
   }
   const int lane = threadIdx.x & 31;
@@ -215,6 +261,178 @@ __global__ void __launch_bounds__(OR_NT) k_order_range(const __grid_constant__ S
   }
 }
 
+// ---------------------------------------------------------------- ranks of few distinct values
+// A float column of limited resolution takes 64 key bits for a few thousand values, eight of the eleven
+// passes of 20M rows ordered by (float, int). Its distinct values are collected and ranked, and the ranks
+// sorted instead: 14 bits, four passes of one-word keys, and the column itself read back from its sorted
+// ranks instead of gathered.
+// Every kernel reads the count from the device; the host reads it once, after the last.
+constexpr int DICT_CTA = 16384;            // slots of a CTA's set
+constexpr int DICT_MAX = DICT_CTA / 4 * 3; // distinct values at most
+constexpr int DICT_SEEN = 65536;           // slots of the global set
+constexpr int DICT_SLOTS = 16384;          // slots of the largest lookup table
+constexpr int DICT_NT = 1024;
+
+struct DictCtl {
+  unsigned int count;  // distinct values so far
+  unsigned int fail;   // too many, or two that the lookup table cannot tell apart
+  unsigned int alias;  // some valid value's bits are not those of its order key (-0.0, NaN payloads)
+};
+
+struct DictCol {
+  const uint8_t* data;
+  const uint8_t* valid;
+  int elem, dtype;
+};
+
+// the raw bits of the value whose order key is o (-0.0 reads 0.0, every NaN the same one)
+__device__ __forceinline__ uint64_t dict_value(unsigned long long o, int dt) {
+  switch (dt) {
+    case PMB_I8: case PMB_I16: case PMB_I32: case PMB_I64: return o ^ 0x8000000000000000ULL;
+    case PMB_F32: return (o & 0x80000000ULL) ? (o & 0x7FFFFFFFULL) : (uint64_t)(uint32_t)~(uint32_t)o;
+    case PMB_F64: return (o >> 63) ? (o & 0x7FFFFFFFFFFFFFFFULL) : ~o;
+    default: return o;
+  }
+}
+
+// The distinct values (as order keys, none of them PMB_EMPTY64) of a column's valid rows: each CTA
+// collects its rows' values in shared memory and adds them to the global set at the end, so that the rows
+// wait for no global probe (with every CTA's first meeting of a value sent there at once, 20M rows of
+// 10,000 values took 478 us, 165 us so). A column of too many values stops after some 12,000 rows
+// of every CTA.
+template <typename T>
+__global__ void __launch_bounds__(DICT_NT) k_dict_collect(const DictCol c, int64_t n, unsigned long long* seen,
+                                                          unsigned long long* list, DictCtl* ctl) {
+  extern __shared__ unsigned long long s_seen[];
+  __shared__ unsigned s_n, s_alias;
+  for (int i = threadIdx.x; i < DICT_CTA; i += DICT_NT) s_seen[i] = PMB_EMPTY64;
+  if (threadIdx.x == 0) s_n = s_alias = 0u;
+  __syncthreads();
+  const T* __restrict__ data = reinterpret_cast<const T*>(c.data);
+  const bool fl = c.dtype == PMB_F32 || c.dtype == PMB_F64;
+  constexpr int U = 4;
+  const int64_t stride = (int64_t)gridDim.x * DICT_NT;
+  for (int64_t r0 = (int64_t)blockIdx.x * DICT_NT + threadIdx.x; r0 < n; r0 += U * stride) {
+    unsigned long long k[U], first[U];
+    unsigned at[U];
+    bool ok[U];
+    T x[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t r = r0 + u * stride;
+      x[u] = r < n ? data[r] : (T)0;
+      ok[u] = r < n && pmb_valid_bit(c.valid, r);
+    }
+    if (*reinterpret_cast<volatile unsigned int*>(&s_n) > DICT_MAX) break;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      k[u] = order_key((uint64_t)x[u], c.dtype);
+      if (fl && ok[u] && dict_value(k[u], c.dtype) != (uint64_t)x[u]) s_alias = 1u;
+      at[u] = (unsigned)pmb_fmix64(k[u]) & (DICT_CTA - 1);
+      first[u] = *reinterpret_cast<volatile unsigned long long*>(&s_seen[at[u]]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!ok[u] || first[u] == k[u]) continue;
+      unsigned long long cur = first[u];
+      unsigned s = at[u];
+      for (int p = 0; p < DICT_CTA; p++) {
+        if (cur == PMB_EMPTY64) {
+          cur = atomicCAS(&s_seen[s], PMB_EMPTY64, k[u]);
+          if (cur == PMB_EMPTY64) {
+            atomicAdd(&s_n, 1u);
+            break;
+          }
+        }
+        if (cur == k[u]) break;
+        s = (s + 1) & (DICT_CTA - 1);
+        cur = *reinterpret_cast<volatile unsigned long long*>(&s_seen[s]);
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_alias) ctl->alias = 1u;
+    if (s_n > DICT_MAX) ctl->fail = 1u;
+  }
+  if (s_n > DICT_MAX) return;
+  for (int i = threadIdx.x; i < DICT_CTA; i += DICT_NT) {
+    const unsigned long long v = s_seen[i];
+    if (v == PMB_EMPTY64) continue;
+    unsigned s = (unsigned)(pmb_fmix64(v) >> 20) & (DICT_SEEN - 1);
+    int p = 0;
+    for (; p < 64; p++) {
+      unsigned long long cur = __ldcg(&seen[s]);
+      if (cur == PMB_EMPTY64) {
+        cur = atomicCAS(&seen[s], PMB_EMPTY64, v);
+        if (cur == PMB_EMPTY64) {
+          const unsigned l = atomicAdd(&ctl->count, 1u);
+          if (l < DICT_MAX) list[l] = v;
+          else ctl->fail = 1u;
+          break;
+        }
+      }
+      if (cur == v) break;
+      s = (s + 1) & (DICT_SEEN - 1);
+    }
+    if (p == 64) ctl->fail = 1u;  // a run of 64 in a set a fifth full: it holds too many
+  }
+}
+
+// rank[i] += the values of part blockIdx.y that lie below value i (blockIdx.x * OR_NT + threadIdx.x)
+constexpr int DICT_PARTS = 32;
+__global__ void __launch_bounds__(OR_NT) k_dict_rank(const unsigned long long* __restrict__ list, const DictCtl* ctl,
+                                                     unsigned int* rank) {
+  __shared__ unsigned long long s_v[DICT_MAX / DICT_PARTS];
+  if (ctl->fail) return;  // (the count may exceed DICT_MAX then)
+  const int n = (int)ctl->count, i = blockIdx.x * OR_NT + threadIdx.x;
+  if ((int)blockIdx.x * OR_NT >= n) return;
+  const int part = (n + DICT_PARTS - 1) / DICT_PARTS, j0 = part * blockIdx.y, m = min(part, n - j0);
+  for (int j = threadIdx.x; j < m; j += OR_NT) s_v[j] = list[j0 + j];
+  __syncthreads();
+  if (i >= n || m <= 0) return;
+  const unsigned long long v = list[i];
+  unsigned c = 0;
+#pragma unroll 8
+  for (int j = 0; j < m; j++) c += s_v[j] < v;
+  if (c) atomicAdd(&rank[i], c);
+}
+
+// slots of the lookup table of n values: at most three quarters full
+__host__ __device__ __forceinline__ int dict_slots(int n) {
+  int s = 512;
+  while (s / 4 * 3 < n) s *= 2;
+  return s;
+}
+__device__ __forceinline__ unsigned dict_fp(unsigned long long hk) { return (unsigned)(hk >> 32) | 1u; }
+
+// The lookup table: fingerprints by linear probing, and each one's rank. A lookup takes the first equal
+// fingerprint from its first slot on, and every value looked up is in the table, so that the answer is
+// right as long as no value met its own fingerprint on the way to its slot (the call sorts whole keys
+// then). And the values' bits by rank, from which the sorted column is written.
+__global__ void __launch_bounds__(OR_NT) k_dict_table(const unsigned long long* __restrict__ list,
+                                                      const unsigned int* __restrict__ rank, DictCtl* ctl,
+                                                      int dtype, unsigned int* fps, unsigned short* codes,
+                                                      unsigned long long* values) {
+  const int n = (int)ctl->count, i = blockIdx.x * OR_NT + threadIdx.x;
+  if (i >= n || n > DICT_MAX || ctl->fail == 1u) return;
+  values[rank[i]] = dict_value(list[i], dtype);
+  const unsigned mask = (unsigned)dict_slots(n) - 1u;
+  const unsigned long long hk = pmb_fmix64(list[i]);
+  const unsigned fp = dict_fp(hk);
+  unsigned s = (unsigned)hk & mask;
+  for (unsigned p = 0; p <= mask; p++) {
+    const unsigned cur = atomicCAS(&fps[s], 0u, fp);
+    if (cur == 0u) {
+      codes[s] = (unsigned short)rank[i];
+      return;
+    }
+    if (cur == fp) break;
+    s = (s + 1) & mask;
+  }
+  ctl->fail = 2u;
+}
+
 // one round's packed key: per column a null flag (null_off >= 0) and `data_bits` value bits
 struct OrderLayout {
   int n;
@@ -230,6 +448,10 @@ struct OrderLayout {
   const uint8_t* valid[PMB_MAX_KEYS];
   int elem[PMB_MAX_KEYS];
   int dtype[PMB_MAX_KEYS];
+  int dict;                 // the column that goes in by rank (-1: none)
+  int dict_slots;
+  const unsigned int* dict_fps;
+  const unsigned short* dict_codes;
 };
 
 template <int W>
@@ -246,33 +468,82 @@ __device__ __forceinline__ unsigned key_digit(const unsigned long long (&k)[W], 
   return (unsigned)((k[wi] >> sh) & 0xFFu);  // digits are 8-bit aligned: never across words
 }
 
-template <int W>
-__global__ void __launch_bounds__(OR_NT) k_order_encode(const __grid_constant__ OrderLayout L, int64_t n,
+constexpr int EU = 4;  // rows of a thread in flight
+template <int E>
+__device__ __forceinline__ void encode_load(const uint8_t* d, const unsigned (&r)[EU], uint64_t (&x)[EU]) {
+#pragma unroll
+  for (int u = 0; u < EU; u++) x[u] = pmb_load_bits(d, E, r[u]);
+}
+
+// DICT: the lookup table is copied into shared memory, and the CTAs have DICT_NT threads. 20M rows of
+// (Float64, Int32): 274 us for the eleven digits of whole keys, 246 us for the four with ranks. Bound by
+// the counting's shared atomics, many of one digit.
+template <int W, bool DICT>
+__global__ void __launch_bounds__(DICT ? DICT_NT : OR_NT) k_order_encode(const __grid_constant__ OrderLayout L, int64_t n,
                                                         const unsigned int* perm, unsigned long long* keys,
                                                         uint64_t cap, unsigned int* idx, int passes,
                                                         unsigned int* hist) {
   __shared__ unsigned int s_hist[OR_PASSES * OR_RADIX];
-  for (int i = threadIdx.x; i < passes * OR_RADIX; i += OR_NT) s_hist[i] = 0;
+  extern __shared__ unsigned int s_fps[];
+  unsigned short* s_codes = reinterpret_cast<unsigned short*>(s_fps + (DICT ? L.dict_slots : 0));
+  for (int i = threadIdx.x; i < passes * OR_RADIX; i += blockDim.x) s_hist[i] = 0;
+  if (DICT)
+    for (int i = threadIdx.x; i < L.dict_slots; i += blockDim.x) {
+      s_fps[i] = L.dict_fps[i];
+      s_codes[i] = L.dict_codes[i];
+    }
   __syncthreads();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t pos = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; pos < n; pos += stride) {
-    const unsigned r = perm ? perm[pos] : (unsigned)pos;
-    unsigned long long k[W];
-    for (int i = 0; i < W; i++) k[i] = 0;
-    for (int c = 0; c < L.n; c++) {
-      const bool v = pmb_valid_bit(L.valid[c], r);
-      if (L.null_off[c] >= 0) put_bits<W>(k, L.null_off[c], (L.nulls_last[c] ? !v : v) ? 1ULL : 0ULL, 1);
-      if (!v) continue;
-      const unsigned long long o = order_key(pmb_load_bits(L.data[c], L.elem[c], r), L.dtype[c]);
-      put_bits<W>(k, L.data_off[c], L.desc[c] ? L.hi[c] - o : o - L.lo[c], L.data_bits[c]);
+  for (int64_t p0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p0 < n; p0 += EU * stride) {
+    unsigned r[EU];
+    unsigned long long k[EU][W];
+#pragma unroll
+    for (int u = 0; u < EU; u++) {
+      const int64_t pos = p0 + u * stride;
+      r[u] = pos < n ? (perm ? perm[pos] : (unsigned)pos) : 0u;
+#pragma unroll
+      for (int i = 0; i < W; i++) k[u][i] = 0;
     }
-    keys[pos] = k[0];
-    if (W > 1) keys[cap + r] = k[W - 1];  // the second word by row (see pmb_sort_pairs)
-    idx[pos] = r;
-    for (int p = 0; p < passes; p++) atomicAdd(&s_hist[p * OR_RADIX + key_digit<W>(k, 8 * p)], 1u);
+    for (int c = 0; c < L.n; c++) {
+      uint64_t x[EU];
+      bool v[EU];
+      const uint8_t* d = L.data[c];
+      switch (L.elem[c]) {  // a column's rows are loaded before any is used
+        case 0: encode_load<0>(d, r, x); break;
+        case 1: encode_load<1>(d, r, x); break;
+        case 2: encode_load<2>(d, r, x); break;
+        case 4: encode_load<4>(d, r, x); break;
+        default: encode_load<8>(d, r, x); break;
+      }
+#pragma unroll
+      for (int u = 0; u < EU; u++) v[u] = pmb_valid_bit(L.valid[c], r[u]);
+#pragma unroll
+      for (int u = 0; u < EU; u++) {
+        if (L.null_off[c] >= 0) put_bits<W>(k[u], L.null_off[c], (L.nulls_last[c] ? !v[u] : v[u]) ? 1ULL : 0ULL, 1);
+        if (!v[u]) continue;
+        unsigned long long o = order_key(x[u], L.dtype[c]);
+        if (DICT && c == L.dict) {
+          const unsigned long long hk = pmb_fmix64(o);
+          const unsigned fp = dict_fp(hk), mask = (unsigned)L.dict_slots - 1u;
+          unsigned s = (unsigned)hk & mask;
+          for (unsigned p = 0; p < mask && s_fps[s] != fp; p++) s = (s + 1) & mask;
+          o = s_codes[s];
+        }
+        put_bits<W>(k[u], L.data_off[c], L.desc[c] ? L.hi[c] - o : o - L.lo[c], L.data_bits[c]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < EU; u++) {
+      const int64_t pos = p0 + u * stride;
+      if (pos >= n) break;
+      keys[pos] = k[u][0];
+      if (W > 1) keys[cap + r[u]] = k[u][W - 1];  // the second word by row (see pmb_sort_pairs)
+      idx[pos] = r[u];
+      for (int p = 0; p < passes; p++) atomicAdd(&s_hist[p * OR_RADIX + key_digit<W>(k[u], 8 * p)], 1u);
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < passes * OR_RADIX; i += OR_NT) {
+  for (int i = threadIdx.x; i < passes * OR_RADIX; i += blockDim.x) {
     const unsigned v = s_hist[i];
     if (v) atomicAdd(&hist[i], v);
   }
@@ -288,6 +559,7 @@ struct GatherCols {
   uint8_t* out_data[PMB_MAX_OUT];
   unsigned int* out_valid[PMB_MAX_OUT];
   const unsigned long long* keys;     // the sorted one-word keys, with dec >= 0
+  const unsigned long long* values;   // the bits by rank of the column that went in by rank
 };
 
 __device__ __forceinline__ unsigned long long get_bits(const unsigned long long* keys, uint64_t pos, int off, int bits) {
@@ -342,7 +614,9 @@ __global__ void __launch_bounds__(OR_NT) k_order_gather(const __grid_constant__ 
           v[u] = L.nulls_last[k] ? !flag : flag;
         }
         const unsigned long long f = get_bits(G.keys, pos, L.data_off[k], L.data_bits[k]);
-        b[u] = v[u] ? from_order_key(L.desc[k] ? L.hi[k] - f : L.lo[k] + f, L.dtype[k]) : 0;
+        const unsigned long long o = L.desc[k] ? L.hi[k] - f : L.lo[k] + f;
+        if (v[u]) b[u] = k == L.dict ? G.values[o] : from_order_key(o, L.dtype[k]);
+        else if (!G.zero[c]) b[u] = pmb_load_bits(G.data[c], e, idx[pos]);  // a float's bits under a null
       }
     } else {
       int64_t r[GU];
@@ -515,8 +789,74 @@ void full_field(int dt, unsigned long long* lo, int* bits) {
   if (pmb_is_signed(dt)) *lo = 0x8000000000000000ULL - (1ULL << (*bits - 1));
 }
 
+// Ranks cost 8 us a million rows (20M: 205 us for the set, the ranks and the table) and 50 us for a wait
+// and small kernels; a pass costs 11 us a million rows. So they are tried where two passes and more are
+// saved, DICT_GAIN rows of passes in all (260 us). 20M rows by (Float64 of 8,800 values, Int32): 4240 us
+// with whole keys, 2380 us so.
+constexpr int64_t DICT_ROWS = 1 << 21, DICT_GAIN = 24000000;
+
 int blocks_for(const pmb_handle* h, int64_t threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((threads + OR_NT - 1) / OR_NT, (int64_t)h->sm_count * 8));
+}
+
+// The lookup table of a column's ranks, when it has at most DICT_MAX distinct values (else *count stays 0).
+struct OrderDict {
+  unsigned int count = 0;
+  const unsigned int* fps = nullptr;
+  const unsigned short* codes = nullptr;
+  const unsigned long long* values = nullptr;
+  bool alias = false;
+};
+int order_dict(pmb_handle* h, const DictCol& c, int64_t n, OrderDict* d) {
+  const WsMark mark = pmb_ws_mark(h);
+  // cleared together: control words, ranks, fingerprints
+  const size_t zero = 64 + (size_t)DICT_MAX * 4 + (size_t)DICT_SLOTS * 4;
+  static_assert(DICT_SLOTS / 4 * 3 >= DICT_MAX, "the lookup table's slots");
+  uint8_t* z = (uint8_t*)pmb_ws_alloc(h, zero);
+  unsigned long long* seen = (unsigned long long*)pmb_ws_alloc(h, (size_t)DICT_SEEN * 8);
+  unsigned long long* list = (unsigned long long*)pmb_ws_alloc(h, (size_t)DICT_MAX * 8);
+  unsigned short* codes = (unsigned short*)pmb_ws_alloc(h, (size_t)DICT_SLOTS * 2);
+  unsigned long long* values = (unsigned long long*)pmb_ws_alloc(h, (size_t)DICT_MAX * 8);
+  if (!z || !seen || !list || !codes || !values) {  // the keys go in whole
+    pmb_ws_release(h, mark);
+    return PMB_OK;
+  }
+  DictCtl* ctl = (DictCtl*)z;
+  unsigned int* rank = (unsigned int*)(z + 64);
+  unsigned int* fps = rank + DICT_MAX;
+  PMB_CUDA(h, cudaMemsetAsync(z, 0, zero, h->stream));
+  PMB_CUDA(h, cudaMemsetAsync(seen, 0xFF, (size_t)DICT_SEEN * 8, h->stream));
+  const auto collect = c.elem == 8 ? k_dict_collect<unsigned long long> : k_dict_collect<uint32_t>;
+  PMB_CUDA(h, cudaFuncSetAttribute(collect, cudaFuncAttributeMaxDynamicSharedMemorySize, DICT_CTA * 8));
+  pmb_kernel_begin(h, "dict_collect");
+  collect<<<(unsigned)h->sm_count, DICT_NT, DICT_CTA * 8, h->stream>>>(c, n, seen, list, ctl);
+  pmb_kernel_end(h);
+  pmb_kernel_begin(h, "dict_rank");
+  k_dict_rank<<<dim3(DICT_MAX / OR_NT, DICT_PARTS), OR_NT, 0, h->stream>>>(list, ctl, rank);
+  pmb_kernel_end(h);
+  pmb_kernel_begin(h, "dict_table");
+  k_dict_table<<<DICT_MAX / OR_NT, OR_NT, 0, h->stream>>>(list, rank, ctl, c.dtype, fps, codes, values);
+  pmb_kernel_end(h);
+  PMB_CUDA(h, cudaGetLastError());
+  PMB_CUDA(h, cudaMemcpyAsync(h->pinned, ctl, sizeof(DictCtl), cudaMemcpyDeviceToHost, h->stream));
+  PMB_CUDA(h, cudaStreamSynchronize(h->stream));
+  const DictCtl* got = (const DictCtl*)h->pinned;
+  if (got->fail || got->count > DICT_MAX) {
+    pmb_ws_release(h, mark);
+    return PMB_OK;
+  }
+  d->count = got->count;
+  d->fps = fps;
+  d->codes = codes;
+  d->values = values;
+  d->alias = got->alias != 0;
+  return PMB_OK;
+}
+
+// Distinct values of a sort column from its sample (Chao's estimate: the seen ones and f1^2 / 2 f2)
+double sampled_distinct(const OrderRange& g, int k) {
+  const double f1 = g.f1[k], f2 = g.f2[k];
+  return f1 == 0 ? g.distinct[k] : g.distinct[k] + f1 * f1 / (2 * std::max(f2, 0.5));
 }
 
 // pmb_order_columns for a table that k_order_small takes
@@ -647,7 +987,7 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     V.n = n_cols;
     for (int c = 0; c < n_cols; c++) V.valid[c] = cols[c].valid;
     pmb_kernel_begin(h, "order_range");
-    k_order_range<<<dim3((unsigned)blocks_for(h, n), 2), OR_NT, 0, h->stream>>>(C, n, ro, V, flags);
+    k_order_range<<<dim3((unsigned)blocks_for(h, n), n >= DICT_ROWS ? 3 : 2), OR_NT, 0, h->stream>>>(C, n, ro, V, flags);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     PMB_CUDA(h, cudaMemcpyAsync(h->pinned, ro, sizeof(got) + PMB_MAX_OUT * 4, cudaMemcpyDeviceToHost, h->stream));
@@ -665,6 +1005,36 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
       while (b < 64 && (span >> b) != 0) b++;
     }
     dbits[k] = b;
+  }
+  // the widest column by rank
+  int dict_col = -1;
+  OrderDict dict;
+  if (n >= DICT_ROWS) {
+    int bits = 0;
+    for (int k = 0; k < nb; k++) {
+      bits += nbits[k] + dbits[k];
+      const int e = cols[s.by[k]].elem;  // (narrower columns have too few bits to gain)
+      if ((e == 4 || e == 8) && got.any[k] && got.hi[k] != PMB_EMPTY64 && (dict_col < 0 || dbits[k] > dbits[dict_col])) dict_col = k;
+    }
+    if (dict_col >= 0) {
+      const double est = sampled_distinct(got, dict_col);
+      int b = 1;
+      while (b < 63 && (double)(1ULL << b) < 2 * est) b++;  // (a sample sees few of the rare values)
+      const int saved = (bits + 7) / 8 - (bits - dbits[dict_col] + b + 7) / 8;
+      if (est <= DICT_MAX && saved >= 2 && (int64_t)saved * n >= DICT_GAIN) {
+        const DCol& d = cols[s.by[dict_col]];
+        const int rc = order_dict(h, DictCol{d.data, d.valid, d.elem, d.dtype}, n, &dict);
+        if (rc) return rc;
+      }
+      if (dict.count > 0) {
+        got.lo[dict_col] = 0;
+        got.hi[dict_col] = dict.count - 1;
+        for (b = 0; ((dict.count - 1) >> b) != 0; b++) {}
+        dbits[dict_col] = b;
+      } else {
+        dict_col = -1;
+      }
+    }
   }
   struct Round {
     int first, last, bits;
@@ -695,6 +1065,10 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     if (rd.bits == 0 || n <= 1) continue;  // every key equal: the order stays
     memset(&L, 0, sizeof(L));
     L.n = rd.last - rd.first + 1;
+    L.dict = dict_col >= rd.first && dict_col <= rd.last ? dict_col - rd.first : -1;
+    L.dict_slots = L.dict >= 0 ? dict_slots((int)dict.count) : 0;
+    L.dict_fps = dict.fps;
+    L.dict_codes = dict.codes;
     int off = 0;
     for (int k = rd.last; k >= rd.first; k--) {  // the most significant column highest
       const int i = k - rd.first;
@@ -718,8 +1092,17 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     const int passes = (off + 7) / 8;
     PMB_CUDA(h, cudaMemsetAsync(hist, 0, (size_t)OR_PASSES * OR_RADIX * 4, h->stream));
     pmb_kernel_begin(h, "order_encode");
-    if (W == 1) k_order_encode<1><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
-    else k_order_encode<2><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+    if (L.dict >= 0) {
+      const int smem = L.dict_slots * 6;
+      const auto encode = W == 1 ? k_order_encode<1, true> : k_order_encode<2, true>;
+      PMB_CUDA(h, cudaFuncSetAttribute(encode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      const int per_sm = smem <= 96 << 10 ? 2 : 1;
+      encode<<<h->sm_count * per_sm, DICT_NT, smem, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+    } else if (W == 1) {
+      k_order_encode<1, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+    } else {
+      k_order_encode<2, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+    }
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
     const bool counts = n > PMB_SORT_NO_READBACK;
@@ -741,13 +1124,18 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
   memset(&G, 0, sizeof(G));
   G.n = n_cols;
   G.keys = k0;
+  G.values = dict.values;
   for (int c = 0; c < n_cols; c++) G.dec[c] = -1;
   // one round sorted every column: integer and Bool sort columns come back out of the sorted keys
   // (float keys are canonical in the key, -0.0 and NaN payloads, so floats are gathered)
   if (rounds.size() == 1 && perm != nullptr) {
     for (int k = 0; k < nb; k++) {
       const int dt = cols[s.by[k]].dtype;
-      if (dt == PMB_F32 || dt == PMB_F64) continue;
+      if (dt == PMB_F32 || dt == PMB_F64) {
+        // by rank, unless the ranks read a value's bits differently
+        if (W == 1 && k == dict_col && !dict.alias) G.dec[s.by[k]] = k - rounds[0].first;
+        continue;
+      }
       if (W == 1) G.dec[s.by[k]] = k - rounds[0].first;  // (two-word keys are not sorted whole)
       G.zero[s.by[k]] = 1;
     }

@@ -311,3 +311,28 @@ def test_carried_values(case, groups):
     got = N.groupby(data, keys, aggs, pred, strategy="partitioned")
     assert got.strategy == "partitioned"
     assert_results_match(as_dict(got), pyoracle.groupby(full, keys, aggs, pred), len(keys), aggs, case)
+
+
+# sort columns by rank among few distinct values: one value, the most that the set takes and one more,
+# special floats (whose bits come from their rows) and none, the all-ones order key (which stays whole), both directions and null places, slices
+@pytest.mark.parametrize("case", [("f64", 1, False, {}), ("f64", 5000, False, {}), ("clean", 700, True, {}),
+                                  ("clean", 12288, True, {"nulls_last": True}), ("max", 40, True, {}),
+                                  ("f64", 12289, False, {"offset": 1_000_000, "limit": 70_001}),
+                                  ("i64", 300, True, {"drop_nulls": True, "nulls_last": True, "limit": 100}),
+                                  ("i64", 9000, False, {"nulls_last": True})], ids=lambda c: f"{c[0]}-{c[1]}")
+def test_ranked_sort_columns(case):
+    kind, distinct, desc, kw = case
+    n, rng = 4_200_001, np.random.default_rng(case[1])
+    if kind in ("f64", "clean"):
+        values = rng.standard_normal(distinct) * 10.0 ** rng.integers(-300, 300, distinct)
+        if kind == "f64":  # and values whose bits are not their order key's
+            values[: min(4, distinct - 1)] = [np.inf, -np.inf, np.nan, -0.0][: min(4, distinct - 1)]
+    else:
+        values = rng.integers(-2**63, 2**63 - 1, distinct)
+        values[0] = 2**63 - 1 if kind == "max" else -2**63
+    pick = rng.integers(0, distinct, n)
+    pick[:distinct] = np.arange(distinct)
+    cols = {"v": (values[rng.permutation(pick)], pack(rng.random(n) > 0.05)),
+            "i": (rng.integers(-50_000, 50_000, n).astype(np.int32), None), "row": (np.arange(n, dtype=np.int32), None)}
+    got, want = _sorted_both(cols, ["v", "i"], [desc, not desc], **kw)
+    assert_same_rows(got, want, f"{distinct} {kind}")
