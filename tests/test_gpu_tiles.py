@@ -314,12 +314,14 @@ def test_carried_values(case, groups):
 
 
 # sort columns by rank among few distinct values: one value, the most that the set takes and one more,
-# special floats (whose bits come from their rows) and none, the all-ones order key (which stays whole), both directions and null places, slices
+# special floats (whose bits come from their rows) and none, the all-ones order key (which stays whole),
+# both directions and null places, slices, several rounds
 @pytest.mark.parametrize("case", [("f64", 1, False, {}), ("f64", 5000, False, {}), ("clean", 700, True, {}),
                                   ("clean", 12288, True, {"nulls_last": True}), ("max", 40, True, {}),
                                   ("f64", 12289, False, {"offset": 1_000_000, "limit": 70_001}),
                                   ("i64", 300, True, {"drop_nulls": True, "nulls_last": True, "limit": 100}),
-                                  ("i64", 9000, False, {"nulls_last": True})], ids=lambda c: f"{c[0]}-{c[1]}")
+                                  ("i64", 9000, False, {"nulls_last": True}), ("rounds", 1000, False, {})],
+                         ids=lambda c: f"{c[0]}-{c[1]}")
 def test_ranked_sort_columns(case):
     kind, distinct, desc, kw = case
     n, rng = 4_200_001, np.random.default_rng(case[1])
@@ -334,5 +336,10 @@ def test_ranked_sort_columns(case):
     pick[:distinct] = np.arange(distinct)
     cols = {"v": (values[rng.permutation(pick)], pack(rng.random(n) > 0.05)),
             "i": (rng.integers(-50_000, 50_000, n).astype(np.int32), None), "row": (np.arange(n, dtype=np.int32), None)}
-    got, want = _sorted_both(cols, ["v", "i"], [desc, not desc], **kw)
+    by = ["v", "i"]
+    if kind == "rounds":  # more than 128 key bits: the ranks in the last round, over rows already in an order
+        cols["j"] = (rng.integers(-2**63, 2**63 - 1, n) >> rng.integers(0, 2, n) * 62, None)
+        cols["w"] = (cols["j"][0][::-1].copy(), None)
+        by = ["v", "j", "w", "i"]
+    got, want = _sorted_both(cols, by, [desc, not desc, desc, desc][: len(by)], **kw)
     assert_same_rows(got, want, f"{distinct} {kind}")
