@@ -792,7 +792,8 @@ void full_field(int dt, unsigned long long* lo, int* bits) {
 // Ranks cost 8 us a million rows (20M: 205 us for the set, the ranks and the table) and 50 us for a wait
 // and small kernels; a pass costs 11 us a million rows. So they are tried where two passes and more are
 // saved, DICT_GAIN rows of passes in all (260 us). 20M rows by (Float64 of 8,800 values, Int32): 4240 us
-// with whole keys, 2380 us so.
+// with whole keys, 2380 us so. The sample misses rare values (8,800 look like 2,900 to 4,600), hence half
+// of DICT_MAX as the most that it may promise: values that do not fit cost 115 us for nothing.
 constexpr int64_t DICT_ROWS = 1 << 21, DICT_GAIN = 24000000;
 
 int blocks_for(const pmb_handle* h, int64_t threads) {
@@ -1021,7 +1022,7 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
       int b = 1;
       while (b < 63 && (double)(1ULL << b) < 2 * est) b++;  // (a sample sees few of the rare values)
       const int saved = (bits + 7) / 8 - (bits - dbits[dict_col] + b + 7) / 8;
-      if (est <= DICT_MAX && saved >= 2 && (int64_t)saved * n >= DICT_GAIN) {
+      if (est <= DICT_MAX / 2 && saved >= 2 && (int64_t)saved * n >= DICT_GAIN) {
         const DCol& d = cols[s.by[dict_col]];
         const int rc = order_dict(h, DictCol{d.data, d.valid, d.elem, d.dtype}, n, &dict);
         if (rc) return rc;

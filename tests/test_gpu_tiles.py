@@ -320,19 +320,23 @@ def test_carried_values(case, groups):
                                   ("clean", 12288, True, {"nulls_last": True}), ("max", 40, True, {}),
                                   ("f64", 12289, False, {"offset": 1_000_000, "limit": 70_001}),
                                   ("i64", 300, True, {"drop_nulls": True, "nulls_last": True, "limit": 100}),
-                                  ("i64", 9000, False, {"nulls_last": True}), ("rounds", 1000, False, {})],
+                                  ("i64", 9000, False, {"nulls_last": True}), ("rounds", 1000, False, {}),
+                                  ("f32", 200, True, {}), ("clean32", 3000, False, {"nulls_last": True})],
                          ids=lambda c: f"{c[0]}-{c[1]}")
 def test_ranked_sort_columns(case):
     kind, distinct, desc, kw = case
-    n, rng = 4_200_001, np.random.default_rng(case[1])
-    if kind in ("f64", "clean"):
-        values = rng.standard_normal(distinct) * 10.0 ** rng.integers(-300, 300, distinct)
-        if kind == "f64":  # and values whose bits are not their order key's
+    n, rng = 12_000_001 if "32" in kind else 4_200_001, np.random.default_rng(case[1])
+    if kind in ("f64", "clean", "f32", "clean32"):
+        span = 36 if "32" in kind else 300
+        values = rng.standard_normal(distinct) * 10.0 ** rng.integers(-span, span, distinct)
+        if "32" in kind:
+            values = values.astype(np.float32)
+        if kind[0] == "f":  # and values whose bits are not their order key's
             values[: min(4, distinct - 1)] = [np.inf, -np.inf, np.nan, -0.0][: min(4, distinct - 1)]
     else:
         values = rng.integers(-2**63, 2**63 - 1, distinct)
         values[0] = 2**63 - 1 if kind == "max" else -2**63
-    pick = rng.integers(0, distinct, n)
+    pick = rng.integers(0, max(1, distinct // 4), n)  # most rows have few of them, so that a sample promises few
     pick[:distinct] = np.arange(distinct)
     cols = {"v": (values[rng.permutation(pick)], pack(rng.random(n) > 0.05)),
             "i": (rng.integers(-50_000, 50_000, n).astype(np.int32), None), "row": (np.arange(n, dtype=np.int32), None)}
