@@ -360,9 +360,10 @@ struct pmb_h2d_pool {
 constexpr size_t H2D_POOL_MIN = (size_t)4 << 20;
 
 // a host-to-device copy on the handle's stream; like cudaMemcpyAsync it has read a pageable source
-// when it returns
+// when it returns. The handle cudaStreamPerThread names the calling thread's stream: in the pool's
+// threads it would name theirs, which the call's kernels do not wait for, so the driver copies there.
 static cudaError_t copy_h2d(pmb_handle* h, uint8_t* dst, const void* src, size_t bytes) {
-  if (bytes >= H2D_POOL_MIN && !h->h2d_pool_failed) {
+  if (bytes >= H2D_POOL_MIN && h->stream != cudaStreamPerThread && !h->h2d_pool_failed) {
     cudaPointerAttributes at;
     const bool known = cudaPointerGetAttributes(&at, src) == cudaSuccess;
     if (!known) cudaGetLastError();
