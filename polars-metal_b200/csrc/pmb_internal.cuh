@@ -206,6 +206,8 @@ struct pmb_handle {
   float* selector = nullptr;
   int32_t launches = 0;
   int64_t h2d = 0, d2h = 0;
+  // failures made on the host for tests (pmb_debug_faults)
+  int fault_jit = -1;  // run-time kernels that may still be compiled (-1: any number)
 };
 
 // status helpers (pmb_runtime.cu)

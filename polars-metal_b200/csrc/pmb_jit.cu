@@ -974,6 +974,8 @@ static int jit_kernel(pmb_handle* h, const std::string& src, const char* name, c
     return PMB_OK;
   }
   if (g_fail.count(src)) return pmb_fail(h, PMB_E_UNSUPPORTED, "JIT compile failed earlier for this signature");
+  if (h->fault_jit == 0) return pmb_fail(h, PMB_E_UNSUPPORTED, "JIT compile refused (pmb_debug_faults)");
+  if (h->fault_jit > 0) h->fault_jit--;
   std::vector<char> cubin;
   std::string log;
   if (!jit_compile(src, cubin, log)) {
@@ -1257,9 +1259,11 @@ static int debug_compile(const pmb_query* q, const pmb_column* cols, int32_t n_c
       JitPlan J;
       rc = pmb_plan_jit_batch(&h, cq, 1024, 1, 232448, &J);
       if (rc != PMB_OK) msg = h.err;
-      for (int v = 0; v < 3 && rc == PMB_OK; v++) {
+      for (int v = 0; v < 6 && rc == PMB_OK; v++) {  // one- and two-word keys, gathered and carried values, CTAs an SM
         std::vector<char> cubin;
-        if (!jit_compile(part_source(cq, J, v == 2 ? 2 : 1, v == 1, v == 1, v == 1 ? 2 : 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
+        const int words = v == 2 || v == 5 ? 2 : 1;
+        const bool payload = v == 1 || v >= 3, cas64 = v == 1 || v == 3;
+        if (!jit_compile(part_source(cq, J, words, cas64, payload, v == 1 ? 2 : 1), cubin, msg)) rc = PMB_E_UNSUPPORTED;
         else if (getenv("PMB_JIT_DEBUG") && getenv("PMB_JIT_DEBUG")[0] == '2') fprintf(stderr, "%s\n", msg.c_str());
       }
     } else if (cq.dq.key_bits > 64) {

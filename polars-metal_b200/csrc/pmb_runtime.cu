@@ -790,6 +790,10 @@ int pmb_last_stats(const pmb_handle* h, pmb_stats* out) {
   return PMB_OK;
 }
 
+// Internal check (not part of the C ABI in pmb.h): failures that the handle's next calls meet, made on the
+// host: at most `jit_kernels` more run-time compiled kernels (-1: any number).
+void pmb_debug_faults(pmb_handle* h, int32_t jit_kernels) { h->fault_jit = jit_kernels; }
+
 void pmb_result_free(pmb_result* r) {
   if (!r) return;
   for (int c = 0; c < r->n_columns; c++) {

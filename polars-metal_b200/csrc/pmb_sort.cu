@@ -1395,6 +1395,11 @@ struct Payload {
   uint8_t* buf[2][PMB_MAX_COLS + 1];
   bool mask = false;
   int row_bytes = 0;
+  // the aggregation that reads them, compiled before the passes: no other kernel can take over afterwards
+  // (the passes move no row numbers)
+  cudaKernel_t kernel = nullptr;
+  JitPlan plan;
+  int ctas = 1;
 };
 
 // Carrying pays where the gathers by row number miss L2: a random read costs a whole DRAM access (42 G/s
@@ -1423,7 +1428,7 @@ bool plan_payload(const DQuery& q, Payload* p) {
 
 // CTAs an SM of the run-time compiled aggregation: two where a row's carried values fit the 32 registers of
 // their threads (pmb_jit_part.cuh has both sides' times), else one
-inline int part_ctas(int W, const Payload* pay) { return pay && W == 1 && pay->row_bytes <= 24 ? 2 : 1; }
+inline int part_ctas(int W, const Payload& pay) { return W == 1 && pay.row_bytes <= 24 ? 2 : 1; }
 
 // the aggregation of the partitioned strategy over keys / row indices sorted by partition
 template <int W>
@@ -1456,8 +1461,9 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
   const size_t smem = pa_layout(slots, W, q.rec_bytes, n_out, A.stage_bytes).bytes;
   PMB_CUDA(h, cudaFuncSetAttribute(k_part_agg<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int64_t out_cap = std::min<int64_t>(std::max<int64_t>(m, 1), 2 * groups + 65536);
-  // should the smaller tables of two CTAs not hold an item's groups, one CTA with the whole table follows
-  int ctas = part_ctas(W, pay);
+  // should the smaller tables of two CTAs not hold an item's groups, one CTA of the same kernel with the
+  // whole table follows
+  int ctas = pay ? pay->ctas : 1;
   for (int attempt = 0;; attempt++) {
     if (attempt >= 6) return pmb_fail(h, PMB_E_CUDA, "partitioned strategy did not converge");
     const WsMark mark = pmb_ws_mark(h);
@@ -1481,7 +1487,10 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
     // without NVRTC (or for a signature it cannot take) the prebuilt kernel does both
     JitPlan J;
     cudaKernel_t jk = nullptr;
-    if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, pay != nullptr, ctas, &J, &jk) != PMB_OK) {
+    if (pay) {
+      J = pay->plan;
+      jk = pay->kernel;
+    } else if (m > 0 && pmb_jit_enabled(1LL << 40) && pmb_jit_part_kernel(h, cq, W, L.bits < 64, false, 1, &J, &jk) != PMB_OK) {
       jk = nullptr;  // the prebuilt kernel instead (the compile error stays readable in pmb_last_error)
     }
     unsigned long long* gkeys = nullptr;
@@ -1690,10 +1699,9 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   Payload pay;
   bool carry = part_groups > 0 && m > 1 && plan_payload(q, &pay) && pmb_jit_enabled(1LL << 40);
   if (carry) {
-    JitPlan J;
-    cudaKernel_t jk;
     const std::string keep_err = h->err;
-    carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, part_ctas(W, &pay), &J, &jk) == PMB_OK;
+    pay.ctas = part_ctas(W, pay);
+    carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, pay.ctas, &pay.plan, &pay.kernel) == PMB_OK;
     const WsMark mark = pmb_ws_mark(h);
     for (int b = 0; carry && b < passes; b++)
       for (int e = 0; carry && e < pay.n; e++) {
