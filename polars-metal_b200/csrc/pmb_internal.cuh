@@ -207,7 +207,8 @@ struct pmb_handle {
   int32_t launches = 0;
   int64_t h2d = 0, d2h = 0;
   // failures made on the host for tests (pmb_debug_faults)
-  int fault_jit = -1;  // run-time kernels that may still be compiled (-1: any number)
+  int fault_jit = -1;       // run-time kernels that may still be compiled (-1: any number)
+  bool fault_wait = false;  // sorts run as if a wait had given up
 };
 
 // status helpers (pmb_runtime.cu)

@@ -55,6 +55,7 @@ __device__ __forceinline__ unsigned long long jp_hash(const unsigned long long* 
 extern "C" __global__ void __launch_bounds__(J_NT, JP_CTAS) pmb_jit_part_agg(const __grid_constant__ JPart A) {
   extern __shared__ __align__(16) unsigned char sm[];
   const JParams& P = A.qp;
+  if (*P.status & PMB_ST_TIMEOUT) return;  // the passes gave up: their row numbers need not be any
   const int S = A.slots, tid = threadIdx.x;
   unsigned int* tag = reinterpret_cast<unsigned int*>(sm);  // 0 empty, 1 claimed, 2 key published
   unsigned long long* tkey = reinterpret_cast<unsigned long long*>(sm + ((S * 4 + 15) & ~15));  // JP_W x S

@@ -482,7 +482,8 @@ template <int W, bool DICT>
 __global__ void __launch_bounds__(DICT ? DICT_NT : OR_NT) k_order_encode(const __grid_constant__ OrderLayout L, int64_t n,
                                                         const unsigned int* perm, unsigned long long* keys,
                                                         uint64_t cap, unsigned int* idx, int passes,
-                                                        unsigned int* hist) {
+                                                        unsigned int* hist, const unsigned int* status) {
+  if (perm && status && (*status & PMB_ST_TIMEOUT)) return;  // the round before gave up: perm need not be an order
   __shared__ unsigned int s_hist[OR_PASSES * OR_RADIX];
   extern __shared__ unsigned int s_fps[];
   unsigned short* s_codes = reinterpret_cast<unsigned short*>(s_fps + (DICT ? L.dict_slots : 0));
@@ -592,7 +593,8 @@ __device__ __forceinline__ void gather_rows(const uint8_t* data, const int64_t (
 // thread, four rows at a time, 20M rows of 4 columns took 1195 us, 965 us so.
 __global__ void __launch_bounds__(OR_NT) k_order_gather(const __grid_constant__ GatherCols G,
                                                         const __grid_constant__ OrderLayout L, const unsigned int* idx,
-                                                        int64_t start, int64_t m) {
+                                                        int64_t start, int64_t m, const unsigned int* status) {
+  if (idx && status && (*status & PMB_ST_TIMEOUT)) return;  // the sort gave up: idx need not be an order
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
   const int c = blockIdx.y, e = G.elem[c], k = G.dec[c];
@@ -1098,11 +1100,11 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
       const auto encode = W == 1 ? k_order_encode<1, true> : k_order_encode<2, true>;
       PMB_CUDA(h, cudaFuncSetAttribute(encode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       const int per_sm = smem <= 96 << 10 ? 2 : 1;
-      encode<<<h->sm_count * per_sm, DICT_NT, smem, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+      encode<<<h->sm_count * per_sm, DICT_NT, smem, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
     } else if (W == 1) {
-      k_order_encode<1, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+      k_order_encode<1, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
     } else {
-      k_order_encode<2, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist);
+      k_order_encode<2, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
     }
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
@@ -1155,7 +1157,7 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
   if (m > 0) {
     pmb_kernel_begin(h, "order_gather");
     const dim3 gb((unsigned)blocks_for(h, (words + GU - 1) / GU * 32), (unsigned)n_cols);
-    k_order_gather<<<gb, OR_NT, 0, h->stream>>>(G, L, perm, start, m);
+    k_order_gather<<<gb, OR_NT, 0, h->stream>>>(G, L, perm, start, m, h->sort_status);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
   }

@@ -791,8 +791,12 @@ int pmb_last_stats(const pmb_handle* h, pmb_stats* out) {
 }
 
 // Internal check (not part of the C ABI in pmb.h): failures that the handle's next calls meet, made on the
-// host: at most `jit_kernels` more run-time compiled kernels (-1: any number).
-void pmb_debug_faults(pmb_handle* h, int32_t jit_kernels) { h->fault_jit = jit_kernels; }
+// host: at most `jit_kernels` more run-time compiled kernels (-1: any number); with `wait`, every sort starts
+// with the status of a bounded wait that gave up.
+void pmb_debug_faults(pmb_handle* h, int32_t jit_kernels, int32_t wait) {
+  h->fault_jit = jit_kernels;
+  h->fault_wait = wait != 0;
+}
 
 void pmb_result_free(pmb_result* r) {
   if (!r) return;

@@ -453,10 +453,15 @@ __global__ void __launch_bounds__(PassShape<W>::NT, PassShape<W>::CTAS)
   __shared__ uint2 s_scan[RADIX / 32];
   __shared__ long long s_tile;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = (long long)atomicAdd(P.ticket, 1ULL);
+  if (tid == 0) {
+    const unsigned st = *reinterpret_cast<volatile unsigned int*>(P.status);
+    const long long t = (long long)atomicAdd(P.ticket, 1ULL);
+    s_tile = st & PMB_ST_TIMEOUT ? -1 : t;
+  }
   for (int i = tid; i < 2 * NW * RADIX; i += NT) (&s_off[0][0])[i] = 0u;
   __syncthreads();
   const long long tile = s_tile;
+  if (tile < 0) return;  // a wait gave up: the pass's input need not match its digit counts
   // warp-striped items: item j of lane l of warp w is tile element w * PER * 32 + j * 32 + l
   const int64_t e0 = (int64_t)tile * TILE + warp * (PER * 32) + lane;
   const unsigned lt = (1u << lane) - 1u;
@@ -870,6 +875,7 @@ __host__ __device__ inline PaLayout pa_layout(int slots, int W, int rec_bytes, i
 template <int W>
 __global__ void __launch_bounds__(PA_NT, 1) k_part_agg(const __grid_constant__ PartParams A) {
   extern __shared__ __align__(16) unsigned char smem[];
+  if (*A.status & PMB_ST_TIMEOUT) return;  // the passes gave up: their row numbers need not be any
   const int S = A.slots, rb = A.q.rec_bytes, rw = rb / 8;
   const PaLayout Ly = pa_layout(S, W, rb, A.n_out, A.stage_bytes);
   unsigned int* tag = reinterpret_cast<unsigned int*>(smem + Ly.tag);  // 0 empty, 1 claimed, 2 key published
@@ -1194,7 +1200,8 @@ template <int W>
 __global__ void __launch_bounds__(ST_NT) k_ordered_finalize(const __grid_constant__ PartFinParams F,
                                                             const __grid_constant__ GroupOrder O,
                                                             const unsigned long long* okeys, const unsigned int* idx,
-                                                            int64_t start, int64_t m) {
+                                                            int64_t start, int64_t m, const unsigned int* status) {
+  if (status && (*status & PMB_ST_TIMEOUT)) return;  // the sort gave up: idx need not be an order
   // a warp's 32 records come into shared memory word by word, all lanes on the same few records, so
   // that every sector of a record is fetched once and all loads are in flight together (a lane walking
   // its own record took 6.8 ms for 49M groups, 1.1 TB/s)
@@ -1317,7 +1324,7 @@ int ordered_finalize(pmb_handle* h, const CompiledQuery& cq, const PartFinParams
     pmb_kernel_begin(h, "ordered_finalize");
     const size_t fsmem = (size_t)ST_NT * F.R.q.rec_bytes;
     PMB_CUDA(h, cudaFuncSetAttribute(k_ordered_finalize<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
-    k_ordered_finalize<W><<<fb, ST_NT, fsmem, h->stream>>>(F, O, k0, i0, start, m);
+    k_ordered_finalize<W><<<fb, ST_NT, fsmem, h->stream>>>(F, O, k0, i0, start, m, h->sort_status);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
   }
@@ -1480,7 +1487,8 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
     A.q = q;
     A.out_cap = out_cap;
     PMB_CUDA(h, cudaMemsetAsync(ctr + 1, 0, 16, h->stream));
-    PMB_CUDA(h, cudaMemsetAsync(status, 0, 64, h->stream));
+    // (the first attempt finds the status of the passes, and a wait that gave up there ends it)
+    if (attempt > 0) PMB_CUDA(h, cudaMemsetAsync(status, 0, 64, h->stream));
     unsigned long long ng = 0;
     unsigned int st[12] = {0};
     // the run-time compiled aggregation writes dense groups that a prebuilt kernel finalises;
@@ -1714,6 +1722,7 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   const auto pass = part_groups > 0 ? k_sort_pass<W, true> : k_sort_pass<W, false>;
   PMB_CUDA(h, cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
   int done = 0;
+  if (h->fault_wait) PMB_CUDA(h, cudaMemsetAsync(status, PMB_ST_TIMEOUT, 1, h->stream));
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
     for (int d = 0; d < RADIX; d++) constant |= hh[(size_t)p * RADIX + d] == (unsigned)m;
@@ -2018,7 +2027,8 @@ int pmb_pack_wide_keys(pmb_handle* h, CompiledQuery& cq) {
 // dst[i] = src[idx[i]], four rows of a thread in flight
 __global__ void __launch_bounds__(ST_NT) k_gather_word(const unsigned long long* __restrict__ src,
                                                        const unsigned int* __restrict__ idx, int64_t n,
-                                                       unsigned long long* __restrict__ dst) {
+                                                       unsigned long long* __restrict__ dst, const unsigned int* status) {
+  if (*status & PMB_ST_TIMEOUT) return;  // the passes gave up: idx need not be an order
   const int64_t stride = (int64_t)gridDim.x * ST_NT;
   for (int64_t i0 = (int64_t)blockIdx.x * ST_NT + threadIdx.x; i0 < n; i0 += 4 * stride) {
     unsigned long long v[4];
@@ -2040,7 +2050,8 @@ __global__ void __launch_bounds__(ST_NT) k_gather_word(const unsigned long long*
 // are stored by row number; `permuted`: *i is not 0, 1, 2, ... already on entry. Without hist_host every
 // digit gets its pass (one more pass of up to a million keys takes less than reading the counts back).
 // The call does not wait: *status_dev (device; null before a call's first round) holds PMB_ST_TIMEOUT
-// after the stream has got there.
+// after the stream has got there, and then neither *i nor *k can be relied on: whatever follows an entry of
+// *i to a row looks at the status first.
 int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long long** k_alt, unsigned int** i,
                    unsigned int** i_alt, uint64_t cap, int64_t n, int n_passes, const unsigned int* hist_dev,
                    const unsigned int* hist_host, bool permuted, unsigned int** status_dev) {
@@ -2059,6 +2070,7 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
   unsigned int* status = *status_dev ? *status_dev : (unsigned int*)(zeroed + clear);
   if (at_once) PMB_CUDA(h, cudaMemsetAsync(zeroed, 0, clear + 64, h->stream));
   else PMB_CUDA(h, cudaMemsetAsync(zeroed + clear, 0, 64, h->stream));
+  if (h->fault_wait) PMB_CUDA(h, cudaMemsetAsync(status, PMB_ST_TIMEOUT, 1, h->stream));
   PMB_CUDA(h, cudaFuncSetAttribute(k_sort_pass<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PassShape<1>::SMEM));
   unsigned long long* a = *k;       // the current word's keys, and where the next pass writes them
   unsigned long long* b = *k_alt;
@@ -2076,7 +2088,7 @@ int pmb_sort_pairs(pmb_handle* h, int W, unsigned long long** k, unsigned long l
     if (p >= 8 && moved) {  // the second word in the order so far, once
       const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((n + 4 * ST_NT - 1) / (4 * ST_NT), (int64_t)h->sm_count * 8));
       pmb_kernel_begin(h, "sort_fetch");
-      k_gather_word<<<blocks, ST_NT, 0, h->stream>>>(a, *i, n, b);
+      k_gather_word<<<blocks, ST_NT, 0, h->stream>>>(a, *i, n, b, status);
       pmb_kernel_end(h);
       PMB_CUDA(h, cudaGetLastError());
       std::swap(a, b);

@@ -14,9 +14,17 @@ from polars_b200 import _native as N
 pytestmark = pytest.mark.gpu
 
 
-def faults(h, jit_kernels=-1):
+def faults(h, jit_kernels=-1, wait=False):
     """Failures that the calls of a handle meet from here on (pmb_debug_faults); no arguments: none."""
-    h._lib.pmb_debug_faults(h.raw, C.c_int32(jit_kernels))
+    h._lib.pmb_debug_faults(h.raw, C.c_int32(jit_kernels), C.c_int32(wait))
+
+
+def device_bytes(ptr, nbytes):
+    rt = C.CDLL("libcudart.so.12")
+    rt.cudaMemcpy.argtypes = [C.c_void_p, C.c_void_p, C.c_size_t, C.c_int]
+    out = np.empty(nbytes, np.uint8)
+    assert rt.cudaMemcpy(out.ctypes.data, ptr, nbytes, 2) == 0
+    return out
 
 
 STREAM_LEGACY, STREAM_PER_THREAD = 1, 2  # cudaStreamLegacy, cudaStreamPerThread
@@ -61,4 +69,51 @@ def test_carried_values_need_one_kernel(kernels, monkeypatch):
     if kernels:  # too few output rows, too small tables, and the one that holds them
         assert got.strategy == "partitioned" and h.last_stats()["kernels"]["part_agg"]["launches"] == 3
     assert_results_match(as_dict(got), pyoracle.groupby(cols, ["k"], aggs, None), 1, aggs, f"{kernels} kernels")
+    h.close()
+
+
+def _sort_columns(h, seed, by, n):
+    rng = np.random.default_rng(seed)
+    cols = {c: rng.integers(-2**62, 2**62, n) for c in "abc"} | {"s": rng.integers(0, 2**20, n).astype(np.int32)}
+    return N.sort_columns(cols, by, output="device", handle=h), [8, 8, 8, 4]
+
+
+def _sorted_groups(h, seed, strategy, by, n):
+    rng = np.random.default_rng(seed)
+    k = rng.permutation(n)  # a group a row, so that every call has the same sizes
+    cols = {"k": k * (2**40 if strategy == "two words" else 1), "j": (k % 1000).astype(np.int32), "v": rng.integers(0, 2**40, n),
+            "w": rng.integers(-2**40, 2**40, n)}
+    keys = ["k", "j"] if strategy == "two words" else ["k"]
+    # by an aggregate: the wanted order is not the keys'; the packed keys of "two words" need two
+    if strategy == "two words":
+        cols["k"], strategy = cols["k"] * 4001, "partitioned"
+    got = N.groupby(cols, keys, [("Sum", "v", "s"), ("Max", "w", "m")], strategy=strategy, sort={"by": by}, output="device", handle=h,
+                    capacity_hint=n)
+    return got, [8] + [4] * (len(keys) - 1) + [8, 8]
+
+
+# a wait of the sort's passes that gave up (a status that the host sets): the call ends with an error, and nothing
+# that follows has used the row numbers: the device result of the call before is still there, byte for byte
+@pytest.mark.parametrize("jit", ["0", "1"])
+@pytest.mark.parametrize("call", [(_sort_columns, ["s"], 20_000), (_sort_columns, ["a", "s"], 20_000),
+                                  (_sort_columns, ["a", "b", "c"], 20_000), (_sort_columns, ["a", "b"], 1_100_000),
+                                  (_sorted_groups, "global_hash", ["s"], 30_000), (_sorted_groups, "partitioned", ["k"], 30_000),
+                                  (_sorted_groups, "partitioned", ["m"], 30_000), (_sorted_groups, "two words", ["j", "k"], 30_000),
+                                  (_sorted_groups, "sort", ["k"], 30_000), (_sorted_groups, "partitioned", ["k"], 4_300_000)],
+                         ids=lambda c: "-".join(map(str, c[1:])))
+def test_sort_that_gives_up(call, jit, monkeypatch):
+    monkeypatch.setenv("PMB_JIT", jit)
+    run, *args, n = call
+    h = N.Handle(0)
+    run(h, 1, *args, n)  # (a second call finds the workspace in one block, every later one at the same addresses)
+    first, widths = run(h, 2, *args, n)
+    before = [device_bytes(p, n * b) for p, b in zip(first.data, widths)]
+    faults(h, wait=True)
+    with pytest.raises(RuntimeError, match="timed out"):
+        run(h, 3, *args, n)
+    assert all(np.array_equal(device_bytes(p, n * b), was) for p, b, was in zip(first.data, widths, before))
+    faults(h)
+    again, _ = run(h, 2, *args, n)
+    assert again.data == first.data
+    assert all(np.array_equal(device_bytes(p, n * b), was) for p, b, was in zip(again.data, widths, before))
     h.close()
