@@ -254,6 +254,10 @@ void pmb_close(pmb_handle* h);
 const char* pmb_last_error(const pmb_handle* h);
 /* Makes the handle launch on an existing cudaStream_t (NULL = the handle's own stream). */
 int pmb_set_stream(pmb_handle* h, void* cuda_stream);
+/* The handle's later launches come after the work that is on `cuda_stream` (of the same GPU; NULL = the
+ * legacy default stream) at the time of this call: for device buffers that it still fills or reads. The
+ * host does not wait. */
+int pmb_wait_for_stream(pmb_handle* h, void* cuda_stream);
 /* 1 = record per-kernel CUDA-event timings of every call (readable with pmb_last_stats). */
 int pmb_set_profiling(pmb_handle* h, int32_t enabled);
 int pmb_last_stats(const pmb_handle* h, pmb_stats* out);

@@ -201,6 +201,7 @@ struct pmb_handle {
   std::vector<cudaEvent_t> event_pool;
   size_t event_next = 0;
   cudaEvent_t call_start = nullptr, call_stop = nullptr;
+  cudaEvent_t other_stream = nullptr;  // pmb_wait_for_stream, made at its first use
   pmb_stats last_stats{};
   // strategy selector: MLP parameters on the device (nullptr: the cardinality heuristic decides)
   float* selector = nullptr;

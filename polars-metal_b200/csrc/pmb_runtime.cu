@@ -760,6 +760,7 @@ void pmb_close(pmb_handle* h) {
   for (cudaEvent_t e : h->event_pool) cudaEventDestroy(e);
   if (h->call_start) cudaEventDestroy(h->call_start);
   if (h->call_stop) cudaEventDestroy(h->call_stop);
+  if (h->other_stream) cudaEventDestroy(h->other_stream);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;
 }
@@ -769,6 +770,16 @@ const char* pmb_last_error(const pmb_handle* h) { return h ? h->err.c_str() : "n
 int pmb_set_stream(pmb_handle* h, void* stream) {
   if (!h) return PMB_E_INVALID;
   h->stream = stream ? (cudaStream_t)stream : h->own_stream;
+  return PMB_OK;
+}
+
+int pmb_wait_for_stream(pmb_handle* h, void* stream) {
+  if (!h) return PMB_E_INVALID;
+  if ((cudaStream_t)stream == h->stream) return PMB_OK;
+  PMB_CUDA(h, cudaSetDevice(h->device));
+  if (!h->other_stream) PMB_CUDA(h, cudaEventCreateWithFlags(&h->other_stream, cudaEventDisableTiming));
+  PMB_CUDA(h, cudaEventRecord(h->other_stream, (cudaStream_t)stream));
+  PMB_CUDA(h, cudaStreamWaitEvent(h->stream, h->other_stream, 0));
   return PMB_OK;
 }
 

@@ -216,6 +216,7 @@ SIGNATURES = {
     "pmb_close": (None, [_H]),
     "pmb_last_error": (C.c_char_p, [_H]),
     "pmb_set_stream": (C.c_int, [_H, _P]),
+    "pmb_wait_for_stream": (C.c_int, [_H, _P]),
     "pmb_set_profiling": (C.c_int, [_H, C.c_int32]),
     "pmb_set_batching": (C.c_int, [_H, C.c_int32]),
     "pmb_last_stats": (C.c_int, [_H, C.POINTER(Stats)]),

@@ -398,8 +398,13 @@ def eval_expr(columns: dict[str, ColumnData | Any], expr: dict, handle: Handle |
         import torch
 
         data = torch.empty(max(n, 1), dtype=torch.int64, device=dev)
-        valid = torch.zeros(_bitmap_bytes(n), dtype=torch.uint8, device=dev)
+        valid = torch.empty(_bitmap_bytes(n), dtype=torch.uint8, device=dev)
+        if len(valid) > (n + 7) // 8:
+            valid[(n + 7) // 8:].zero_()  # the padding; the call writes the rest
         dp, vp = data.data_ptr(), valid.data_ptr()
+        if dev.index == h.device:  # (columns of another GPU are refused below)
+            # the memory may be that of tensors which work queued on torch's stream still uses
+            h.check(h._lib.pmb_wait_for_stream(h.raw, torch.cuda.current_stream(dev).cuda_stream))
     else:
         data = np.empty(max(n, 1), np.int64)
         valid = np.zeros(_bitmap_bytes(n), np.uint8)

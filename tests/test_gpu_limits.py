@@ -117,3 +117,28 @@ def test_sort_that_gives_up(call, jit, monkeypatch):
     assert again.data == first.data
     assert all(np.array_equal(device_bytes(p, n * b), was) for p, b, was in zip(again.data, widths, before))
     h.close()
+
+
+# an expression's column goes into memory that torch hands out while earlier work of torch's stream still writes
+# to it: the call waits for that work, and what it wrote stays
+@pytest.mark.parametrize("n", [1, 1000, 300_001])
+def test_expression_behind_work_in_flight(n):
+    import torch
+
+    x = torch.arange(n, dtype=torch.int64, device="cuda")
+    e = {"kind": "Arith", "op": "Add", "lhs": {"kind": "Column", "name": "x"}, "rhs": {"kind": "Column", "name": "x"}}
+    k, key = np.arange(n) % 3, x % 3
+    for _ in range(2):
+        torch.cuda.synchronize()
+        torch.cuda._sleep(200_000_000)  # 0.1 s
+        del_me = [torch.full((n,), 7, dtype=torch.int64, device="cuda"), torch.zeros(N._bitmap_bytes(n), dtype=torch.uint8, device="cuda")]
+        del del_me  # back to torch's allocator, the fills still to come
+        got = N.eval_expr({"x": N.ColumnData(x)}, e)
+        torch.cuda.synchronize()
+        assert np.array_equal(got.data.cpu().numpy()[:n], 2 * np.arange(n))
+        bits = np.unpackbits(got.validity.cpu().numpy(), bitorder="little")
+        assert bits[:n].all() and not bits[n:].any()
+        torch.cuda._sleep(200_000_000)
+        g = N.groupby({"k": N.ColumnData(key), "x": N.ColumnData(x)}, ["k"], [("Sum", e, "s"), ("Count", e, "c")], sort={"by": "k"})
+        assert [int(v) for v in g.data[1][: min(n, 3)]] == [int((2 * np.arange(n))[k == i].sum()) for i in range(min(n, 3))]
+        assert [int(v) for v in g.data[2][: min(n, 3)]] == [int((k == i).sum()) for i in range(min(n, 3))]
