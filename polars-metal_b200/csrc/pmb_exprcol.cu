@@ -560,9 +560,15 @@ extern "C" int pmb_eval_expr(pmb_handle* h, const pmb_expr* expr, const pmb_colu
   const int64_t words = (n + 31) / 32;
   const size_t vbytes = (size_t)((n + 7) / 8);
   const size_t ob = (size_t)n * pmb_dtype_bytes(P.out_dtype);
-  // device outputs are written in place, unless they are misaligned for the kernel's stores or meet
-  // an input (whose rows other threads may still have to read)
-  const bool direct = out_on_device && ((uintptr_t)out_data % 8) == 0 && ((uintptr_t)out_valid % 4) == 0 &&
+  // device outputs are written in place, unless they are not this GPU's memory, misaligned for the kernel's
+  // stores or meet an input (whose rows other threads may still have to read)
+  bool own_data = false, own_valid = false;
+  if (out_on_device && n > 0) {
+    rc = pmb_check_output(h, out_data, &own_data);
+    if (!rc) rc = pmb_check_output(h, out_valid, &own_valid);
+    if (rc) return rc;
+  }
+  const bool direct = own_data && own_valid && ((uintptr_t)out_data % 8) == 0 && ((uintptr_t)out_valid % 4) == 0 &&
                       !ec_overlaps(P, n, out_data, ob) && !ec_overlaps(P, n, out_valid, vbytes);
   uint8_t* dd = direct ? (uint8_t*)out_data : (uint8_t*)pmb_ws_alloc(h, ob + 16);
   uint8_t* dv = direct ? out_valid : (uint8_t*)pmb_ws_alloc(h, (size_t)words * 4 + 16);

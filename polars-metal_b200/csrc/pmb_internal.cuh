@@ -253,6 +253,9 @@ pmb_result* pmb_result_new(int32_t n_columns);
 // column staging (pmb_runtime.cu): makes a device view of a column, copying host data in
 // and realigning device data whose offset breaks 16-byte alignment.
 int pmb_stage_column(pmb_handle* h, const pmb_column& c, int64_t n_rows, DCol* out);
+// *own: a device output pointer is memory of the handle's GPU, which kernels may store to (pinned host memory
+// and other GPUs' are copied to); PMB_E_INVALID when it is neither
+int pmb_check_output(pmb_handle* h, const void* p, bool* own);
 
 // output: copies n rows of device output columns to host memory when requested
 int pmb_finish_outputs(pmb_handle* h, pmb_result* r, bool to_host);

@@ -467,6 +467,21 @@ static int check_device_pointer(pmb_handle* h, const void* p) {
   return pmb_fail(h, PMB_E_INVALID, "device column pointer is not CUDA memory (pageable host memory?)");
 }
 
+int pmb_check_output(pmb_handle* h, const void* p, bool* own) {
+  const uintptr_t a = (uintptr_t)p;
+  *own = true;
+  for (const auto& r : h->ptr_ok)
+    if (a >= r.first && a < r.second) return PMB_OK;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    at.type = cudaMemoryTypeUnregistered;
+  }
+  if (at.type == cudaMemoryTypeUnregistered) return pmb_fail(h, PMB_E_INVALID, "device output pointer is not CUDA memory");
+  *own = at.type != cudaMemoryTypeHost && at.device == h->device;
+  return PMB_OK;
+}
+
 int pmb_stage_column(pmb_handle* h, const pmb_column& c, int64_t n, DCol* out) {
   out->dtype = c.dtype;
   out->elem = pmb_dtype_bytes(c.dtype);

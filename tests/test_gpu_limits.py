@@ -142,3 +142,33 @@ def test_expression_behind_work_in_flight(n):
         g = N.groupby({"k": N.ColumnData(key), "x": N.ColumnData(x)}, ["k"], [("Sum", e, "s"), ("Count", e, "c")], sort={"by": "k"})
         assert [int(v) for v in g.data[1][: min(n, 3)]] == [int((2 * np.arange(n))[k == i].sum()) for i in range(min(n, 3))]
         assert [int(v) for v in g.data[2][: min(n, 3)]] == [int((k == i).sum()) for i in range(min(n, 3))]
+
+
+# device outputs of an expression: this GPU's memory in place, pinned host memory by a copy, pageable memory refused
+@pytest.mark.parametrize("jit", ["0", "1"])
+@pytest.mark.parametrize("kind", ["device", "pinned", "pageable", "pageable validity"])
+def test_expression_output_memory(kind, jit, monkeypatch):
+    import torch
+
+    monkeypatch.setenv("PMB_JIT", jit)
+    n = 5003
+    x = torch.arange(n, dtype=torch.int64, device="cuda")
+    abi, _keep = N._to_abi_columns([N.ColumnData(x)])
+    e, _k = N.compile_predicate({"kind": "Arith", "op": "Mul", "lhs": {"kind": "Column", "name": "x"},
+                                 "rhs": {"kind": "Column", "name": "x"}}, {"x": 0})
+
+    def memory(size, dtype, pageable):
+        return torch.zeros(size, dtype=dtype, device="cuda" if kind != "pinned" and not pageable else None, pin_memory=kind == "pinned")
+
+    data = memory(n, torch.int64, kind == "pageable")
+    valid = memory(N._bitmap_bytes(n), torch.uint8, kind.startswith("pageable"))
+    torch.cuda.synchronize()
+    h, dt = N.default_handle(), C.c_int32()
+    rc = h._lib.pmb_eval_expr(h.raw, C.byref(e), abi, 1, data.data_ptr(), valid.data_ptr(), 1, C.byref(dt))
+    if kind.startswith("pageable"):
+        with pytest.raises(ValueError, match="not CUDA memory"):
+            h.check(rc)
+        return
+    h.check(rc)
+    assert np.array_equal(data.cpu().numpy(), np.arange(n) ** 2)
+    assert np.unpackbits(valid.cpu().numpy(), bitorder="little")[:n].all()
