@@ -1323,7 +1323,7 @@ int recompile_dd(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int3
 extern "C" int pmb_groupby(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
                            pmb_result** out) {
   bool ordered;
-  return pmb_groupby_call(h, q, cols, n_cols, nullptr, &ordered, out);
+  return pmb_again_uncarried(h, [&] { return pmb_groupby_call(h, q, cols, n_cols, nullptr, &ordered, out); });
 }
 
 int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,

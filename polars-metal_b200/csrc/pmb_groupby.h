@@ -120,6 +120,20 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
 // already are the sorted slice
 int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
                      const pmb_sort_spec* spec, bool* ordered, pmb_result** out);
+// A whole group-by call. Values carried through the partition passes take up to 64 bytes a row that the rest
+// of the call may lack (its outputs, its groups, the sort of its result): out of memory with them, it
+// runs again without.
+template <typename Call>
+int pmb_again_uncarried(pmb_handle* h, const Call& call) {
+  if (!h) return call();
+  h->carried = false;
+  int rc = call();
+  if (rc != PMB_E_OOM || !h->carried) return rc;
+  h->no_carry = true;
+  rc = call();
+  h->no_carry = false;
+  return rc;
+}
 // learned selector (pmb_learned.cu): strategy and group count for AUTO; false when no selector is
 // installed or its output is unusable
 bool pmb_selector_pick(pmb_handle* h, const CompiledQuery& cq, int* strategy, int64_t* groups);

@@ -207,9 +207,12 @@ struct pmb_handle {
   float* selector = nullptr;
   int32_t launches = 0;
   int64_t h2d = 0, d2h = 0;
+  // the partition passes of this call carried values (or lacked the memory to); a call without: pmb_groupby.h
+  bool carried = false, no_carry = false;
   // failures made on the host for tests (pmb_debug_faults)
   int fault_jit = -1;       // run-time kernels that may still be compiled (-1: any number)
   bool fault_wait = false;  // sorts run as if a wait had given up
+  size_t fault_ws = 0;      // bytes that the workspace cannot grow beyond (0: the device's memory)
 };
 
 // status helpers (pmb_runtime.cu)

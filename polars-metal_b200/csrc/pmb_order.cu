@@ -1219,8 +1219,8 @@ extern "C" int pmb_sort_columns(pmb_handle* h, const pmb_column* cols, int32_t n
   return PMB_OK;
 }
 
-extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
-                                  const pmb_sort_spec* spec, pmb_result** out) {
+static int groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
+                          const pmb_sort_spec* spec, pmb_result** out) {
   if (!h) return PMB_E_INVALID;
   if (!out) return pmb_fail(h, PMB_E_INVALID, "out is NULL");
   *out = nullptr;
@@ -1271,4 +1271,9 @@ extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_c
   pmb_call_end(h);
   *out = r;
   return PMB_OK;
+}
+
+extern "C" int pmb_groupby_sorted(pmb_handle* h, const pmb_query* q, const pmb_column* cols, int32_t n_cols,
+                                  const pmb_sort_spec* spec, pmb_result** out) {
+  return pmb_again_uncarried(h, [&] { return groupby_sorted(h, q, cols, n_cols, spec, out); });
 }

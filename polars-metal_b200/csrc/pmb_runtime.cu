@@ -116,6 +116,12 @@ void* pmb_ws_alloc(pmb_handle* h, size_t bytes) {
   }
   size_t last = h->ws.empty() ? 0 : h->ws.back().cap;
   size_t want = std::max(std::max(bytes, (size_t)64 << 20), last);
+  if (h->fault_ws) {
+    size_t held = 0;
+    for (const auto& b : h->ws) held += b.cap;
+    if (held + bytes > h->fault_ws) return nullptr;
+    want = std::min(want, h->fault_ws - held);
+  }
   uint8_t* p = nullptr;
   if (cudaMalloc((void**)&p, want) != cudaSuccess) {
     cudaGetLastError();
@@ -818,10 +824,11 @@ int pmb_last_stats(const pmb_handle* h, pmb_stats* out) {
 
 // Internal check (not part of the C ABI in pmb.h): failures that the handle's next calls meet, made on the
 // host: at most `jit_kernels` more run-time compiled kernels (-1: any number); with `wait`, every sort starts
-// with the status of a bounded wait that gave up.
-void pmb_debug_faults(pmb_handle* h, int32_t jit_kernels, int32_t wait) {
+// with the status of a bounded wait that gave up; a workspace of at most `ws_bytes` (0: no limit).
+void pmb_debug_faults(pmb_handle* h, int32_t jit_kernels, int32_t wait, int64_t ws_bytes) {
   h->fault_jit = jit_kernels;
   h->fault_wait = wait != 0;
+  h->fault_ws = (size_t)ws_bytes;
 }
 
 void pmb_result_free(pmb_result* r) {

@@ -1705,11 +1705,12 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   // the partition passes carry the aggregated values when the run-time compiled aggregation can take
   // them and the buffers fit
   Payload pay;
-  bool carry = part_groups > 0 && m > 1 && plan_payload(q, &pay) && pmb_jit_enabled(1LL << 40);
+  bool carry = part_groups > 0 && m > 1 && !h->no_carry && plan_payload(q, &pay) && pmb_jit_enabled(1LL << 40);
   if (carry) {
     const std::string keep_err = h->err;
     pay.ctas = part_ctas(W, pay);
     carry = pmb_jit_part_kernel(h, cq, W, L.bits < 64, true, pay.ctas, &pay.plan, &pay.kernel) == PMB_OK;
+    h->carried = carry;
     const WsMark mark = pmb_ws_mark(h);
     for (int b = 0; carry && b < passes; b++)
       for (int e = 0; carry && e < pay.n; e++) {

@@ -14,9 +14,9 @@ from polars_b200 import _native as N
 pytestmark = pytest.mark.gpu
 
 
-def faults(h, jit_kernels=-1, wait=False):
+def faults(h, jit_kernels=-1, wait=False, workspace=0):
     """Failures that the calls of a handle meet from here on (pmb_debug_faults); no arguments: none."""
-    h._lib.pmb_debug_faults(h.raw, C.c_int32(jit_kernels), C.c_int32(wait))
+    h._lib.pmb_debug_faults(h.raw, C.c_int32(jit_kernels), C.c_int32(wait), C.c_int64(workspace))
 
 
 def device_bytes(ptr, nbytes):
@@ -172,3 +172,41 @@ def test_expression_output_memory(kind, jit, monkeypatch):
     h.check(rc)
     assert np.array_equal(data.cpu().numpy(), np.arange(n) ** 2)
     assert np.unpackbits(valid.cpu().numpy(), bitorder="little")[:n].all()
+
+
+# a workspace too small for the values that the partition passes would carry: the call runs without carrying them,
+# down to the least that it needs so, plain, sorted by a key and sorted by an aggregate
+@pytest.mark.parametrize("sort", [None, {"by": "k"}, {"by": ["m", "k"]}], ids=["plain", "key", "aggregate"])
+def test_workspace_without_carried_values(sort, monkeypatch):
+    import torch
+
+    monkeypatch.setenv("PMB_JIT", "1")
+    n, groups = 4_300_003, 400_000
+    rng = np.random.default_rng(3)
+    k = np.concatenate([np.arange(groups), rng.integers(0, groups, n - groups)])
+    cols = {"k": (k, None)} | {c: (rng.integers(-2**40, 2**40, n), None) for c in "xyz"}
+    aggs = [("Sum", "x", "s"), ("Max", "y", "m"), ("Min", "z", "l")]
+    want = pyoracle.groupby(cols, ["k"], aggs, None)
+    data = {c: N.ColumnData(torch.from_numpy(d).cuda()) for c, (d, _) in cols.items()}
+    torch.cuda.synchronize()
+
+    def run(workspace):
+        h = N.Handle(0)
+        faults(h, workspace=workspace)
+        try:
+            got = N.groupby(data, ["k"], aggs, strategy="partitioned", capacity_hint=groups, sort=sort, handle=h)
+        except MemoryError:
+            return False
+        finally:
+            h.close()
+        if sort:
+            assert (np.diff(got.data[0] if sort["by"] == "k" else got.data[2]) >= 0).all()
+        assert got.strategy == "partitioned"
+        assert_results_match(as_dict(got), want, 1, aggs, f"{workspace} bytes")
+        return True
+
+    MB = 1 << 20
+    assert run(0)
+    fits = [w for w in range(640, 159, -20) if run(w * MB)]
+    assert fits and fits == list(range(640, fits[-1] - 1, -20))  # whatever fits a workspace fits a larger one
+    assert fits[-1] * MB < 2 * n * (12 + 24), fits  # keys, row numbers and 24 bytes of values a row, twice each
