@@ -1577,17 +1577,23 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         F.grecs = grecs;
         F.gcap = (uint64_t)out_cap;
         if (ordered_by_keys(cq, L)) {
+          const WsMark order_mark = pmb_ws_mark(h);
           int64_t rows = 0;
           const int orc = ordered_finalize<W>(h, cq, F, (int64_t)ng, &rows);
-          if (orc) return orc;
-          ng = (unsigned long long)rows;
-          cq.ordered = true;
-        } else {
+          if (orc && orc != PMB_E_OOM) return orc;
+          if (orc) {  // the order keys do not fit: the columns are sorted, whose keys may be narrower
+            pmb_ws_release(h, order_mark);
+          } else {
+            ng = (unsigned long long)rows;
+            cq.ordered = true;
+          }
+        }
+        if (!cq.ordered) {
           const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)ng + ST_NT - 1) / ST_NT, (int64_t)h->sm_count * 16));
-        pmb_kernel_begin(h, "part_finalize");
-        k_part_finalize<W><<<blocks, ST_NT, 0, h->stream>>>(F);
-        pmb_kernel_end(h);
-        PMB_CUDA(h, cudaGetLastError());
+          pmb_kernel_begin(h, "part_finalize");
+          k_part_finalize<W><<<blocks, ST_NT, 0, h->stream>>>(F);
+          pmb_kernel_end(h);
+          PMB_CUDA(h, cudaGetLastError());
         }
       }
     }

@@ -210,3 +210,40 @@ def test_workspace_without_carried_values(sort, monkeypatch):
     fits = [w for w in range(640, 159, -20) if run(w * MB)]
     assert fits and fits == list(range(640, fits[-1] - 1, -20))  # whatever fits a workspace fits a larger one
     assert fits[-1] * MB < 2 * n * (12 + 24), fits  # keys, row numbers and 24 bytes of values a row, twice each
+
+
+# a workspace too small for the groups' order keys (two words each, the sort column's own key one): the finished
+# columns are sorted instead, down to what that needs
+def test_workspace_without_order_keys(monkeypatch):
+    import torch
+
+    monkeypatch.setenv("PMB_JIT", "1")
+    n = 2_000_003  # a group a row; too few values to carry
+    rng = np.random.default_rng(4)
+    k = rng.permutation(n)
+    cols = {"k": (k * (2**42 + 1), None), "j": (k.astype(np.int32), None), "x": (rng.integers(-2**40, 2**40, n), None)}
+    want = np.argsort(k)[-1000:][::-1]
+    data = {c: N.ColumnData(torch.from_numpy(d).cuda()) for c, (d, _) in cols.items()}
+    torch.cuda.synchronize()
+
+    def run(workspace):
+        h = N.Handle(0)
+        h.set_profiling(True)
+        faults(h, workspace=workspace)
+        try:
+            got = N.groupby(data, ["k", "j"], [("Sum", "x", "s")], strategy="partitioned", capacity_hint=n,
+                            sort={"by": "j", "descending": True, "limit": 1000}, handle=h)
+            kernels = h.last_stats()["kernels"]
+        except MemoryError:
+            return None
+        finally:
+            h.close()
+        assert got.strategy == "partitioned" and got.n_groups == 1000
+        for have, c in zip(got.data, ("k", "j", "x")):
+            assert np.array_equal(have, cols[c][0][want])
+        return "ordered" if "ordered_finalize" in kernels else "columns"
+
+    MB = 1 << 20
+    how = [run(w * MB) for w in range(600, 99, -4)]
+    assert how[0] == run(0) == "ordered" and how[-1] is None
+    assert "columns" in how and how == sorted(how, key=["ordered", "columns", None].index)
