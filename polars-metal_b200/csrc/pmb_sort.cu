@@ -1437,6 +1437,13 @@ bool plan_payload(const DQuery& q, Payload* p) {
 // their threads (pmb_jit_part.cuh has both sides' times), else one
 inline int part_ctas(int W, const Payload& pay) { return W == 1 && pay.row_bytes <= 24 ? 2 : 1; }
 
+// Partitions per work item: runs of them with half a table of rows on average (rows bound the groups; the
+// hash spreads them, so a run stays far from the whole table), at least one each. Not by the rows of a
+// partition rounded down: 1.9 of them as 1 would make runs of 0.95 of a table.
+inline int part_run(int slots, int64_t n_parts, int64_t m) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, slots / 2 * n_parts / std::max<int64_t>(1, m)));
+}
+
 // the aggregation of the partitioned strategy over keys / row indices sorted by partition
 template <int W>
 int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_result* r, const unsigned long long* keys,
@@ -1514,7 +1521,7 @@ int run_part_agg(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_r
         int jslots = slots, jrun = run;
         if (ctas == 2) {
           jslots = std::min(slots, (h->max_smem_optin / 2 - 1536) / (4 + 8 * W + J.srec + 2) & ~7);
-          jrun = (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, jslots / 2 / std::max<int64_t>(1, m / n_parts)));
+          jrun = part_run(jslots, n_parts, m);
         }
         const int64_t jitems = (n_parts + jrun - 1) / jrun;
         JPartH JA;
@@ -1792,11 +1799,7 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     k_part_starts<W><<<(unsigned)(n_parts / ST_NT + 1), ST_NT, 0, h->stream>>>(k0, cap, m, pb, pstart);
     pmb_kernel_end(h);
     PMB_CUDA(h, cudaGetLastError());
-    // work items: runs of partitions with half a table of rows on average (rows bound the groups; the
-    // hash spreads them, so a run stays far from the whole table), at least one partition each
-    const int64_t rows = std::max<int64_t>(1, m / n_parts);
-    const int run = (int)std::max<int64_t>(1, std::min<int64_t>(n_parts, slots / 2 / rows));
-    return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pstart, n_parts, run, slots, part_groups, ctr, status,
+    return run_part_agg<W>(h, cq, L, r, k0, i0, cap, m, pstart, n_parts, part_run(slots, n_parts, m), slots, part_groups, ctr, status,
                            PMB_STRATEGY_PARTITIONED, carry ? &pay : nullptr);
   }
   // segment starts

@@ -347,3 +347,24 @@ def test_ranked_sort_columns(case):
         by = ["v", "j", "w", "i"]
     got, want = _sorted_both(cols, by, [desc, not desc, desc, desc][: len(by)], **kw)
     assert_same_rows(got, want, f"{distinct} {kind}")
+
+
+# work items of the partitioned aggregation: a fraction of a row, and just below two and three rows, in each of
+# 65,536 partitions (by the hint's estimate), every row a group of its own: half a table an item, so that the
+# strategy holds; with a filter that leaves few of many rows, the values are carried
+@pytest.mark.parametrize("filtered", [False, True])
+@pytest.mark.parametrize("jit", ["0", "1"])
+@pytest.mark.parametrize("kept", [20_000, 65_535, 130_900, 196_400])
+def test_partition_runs(kept, jit, filtered, monkeypatch):
+    monkeypatch.setenv("PMB_JIT", jit)
+    n = 2_900_017 if filtered else kept
+    rng = np.random.default_rng(kept)
+    k = rng.permutation(n)
+    cols = {"k": (k * 8191, None), "f": (k.astype(np.int32), None), "x": (rng.integers(-2**40, 2**40, n), None),
+            "y": (rng.integers(-2**40, 2**40, n), None), "z": (rng.integers(-2**40, 2**40, n), None)}
+    pred = {"kind": "Compare", "op": "Lt", "lhs": {"kind": "Column", "name": "f"}, "rhs": {"kind": "LiteralI64", "value": kept}}
+    aggs = [("Max", "x", "s"), ("Min", "y", "l"), ("Max", "z", "h")]
+    got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, ["k"], aggs, pred if filtered else None,
+                    strategy="partitioned", capacity_hint=400_000)
+    assert got.strategy == "partitioned" and got.n_groups == kept
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, ["k"], aggs, pred if filtered else None), 1, aggs)
