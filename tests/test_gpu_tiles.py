@@ -368,3 +368,78 @@ def test_partition_runs(kept, jit, filtered, monkeypatch):
                     strategy="partitioned", capacity_hint=400_000)
     assert got.strategy == "partitioned" and got.n_groups == kept
     assert_results_match(as_dict(got), pyoracle.groupby(cols, ["k"], aggs, pred if filtered else None), 1, aggs)
+
+
+def _table(want):
+    return {nm: (d, v, dt, want["n_groups"]) for nm, d, v, dt in zip(want["names"], want["data"], want["validity"], want["dtypes"])}
+
+
+# slices of groups left in the wanted order, by all keys, so that order and slice are unique: every output column
+# of every row, so that a record taken from another place than its key shows
+@pytest.mark.parametrize("strategy", ["partitioned", "sort"])
+@pytest.mark.parametrize("order", [{"by": ["j", "k", "w"], "descending": [True, False, True], "offset": 5, "limit": 1000},
+                                   {"by": ["k", "w", "j"], "nulls_last": [False, False, True], "offset": -900},
+                                   {"by": ["w", "j", "k"], "descending": True, "offset": 2_000, "limit": 3}],
+                         ids=lambda o: "-".join(o["by"]))
+@pytest.mark.parametrize("kind", ["narrow", "wide"])
+def test_ordered_slices(kind, order, strategy):
+    rng = np.random.default_rng(len(kind))
+    n = 120_000
+    k = rng.integers(0, 3000, n)
+    k = np.where(k % 2 == 0, k, -k) * (3_000_000_000_000_000 if kind == "wide" else 1)
+    cols = {"k": (k, None), "j": (rng.integers(-20, 20, n).astype(np.int16), pack(rng.random(n) > 0.02)),
+            "w": ((rng.integers(0, 2, n) * 2**30).astype(np.int32), None), "v": (rng.standard_normal(n), pack(rng.random(n) > 0.1))}
+    keys, aggs = ["k", "j", "w"], [("Min", "v", "s"), ("Max", "v", "t"), ("Len", None, "c")]
+    got = as_dict(N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, keys, aggs, strategy=strategy, sort=order))
+    flags = lambda x: [bool(x)] * 3 if isinstance(x, bool) else list(x)  # noqa: E731
+    want = pyoracle.sort_table(_table(pyoracle.groupby(cols, keys, aggs, None)), order["by"], flags(order.get("descending", False)),
+                               flags(order.get("nulls_last", False)), False, order["offset"], order.get("limit", -1))
+    assert_same_rows(got, want, f"{kind} {strategy}")
+
+
+# the table of a learned estimate: three slots a predicted group (two made half of the tables too small)
+@pytest.mark.parametrize("card,width", [(3000, 4), (90_000, 8), (400_000, 8)])
+def test_slots_of_a_learned_estimate(card, width):
+    rng = np.random.default_rng(card)
+    n = 3_000_000
+    q = ({"k": rng.integers(0, card, n).astype(np.int32 if width == 4 else np.int64), "v": rng.standard_normal(n)}, ["k"],
+         [("Sum", "v", "s"), ("Len", None, "c")])
+    strategy, groups = N.selector_choose(*q)
+    got = N.groupby(*q)
+    assert got.strategy == strategy
+    if got.rehash_count == 0 and strategy.endswith("hash"):
+        slots = min(max(3 * groups, 1024), 2 * n)
+        assert got.capacity == (slots + 3) // 4 * 4
+
+
+# the group-by's passes over two-word keys: tiles of 3072, its edges and remainders, the sort's digits and the
+# partitions'; and with carried values (64 MB of them) over keys of one word (tiles of 3840) and of two
+@pytest.mark.parametrize("strategy", ["partitioned", "sort"])
+@pytest.mark.parametrize("n", [1, 2, 3071, 3072, 3073, 6143, 6144, 6145, 49_152])
+def test_two_word_passes(n, strategy):
+    rng = np.random.default_rng(n)
+    k = rng.integers(-2**62, 2**62, n)
+    cols = {"k": (k[rng.integers(0, max(1, n // 3), n)], None), "j": (rng.integers(-2**31, 2**31, n).astype(np.int32) >> 30, pack(rng.random(n) > 0.1)),
+            "v": (rng.integers(-2**40, 2**40, n), None)}
+    aggs = [("Sum", "v", "s"), ("Min", "v", "l"), ("Len", None, "c")]
+    got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, ["k", "j"], aggs, strategy=strategy)
+    assert got.strategy == strategy
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, ["k", "j"], aggs, None), 2, aggs)
+
+
+@pytest.mark.parametrize("hint", [20_000, 400_000])  # one pass, two passes
+@pytest.mark.parametrize("words,n", [(1, 729 * 3840 - 1), (1, 729 * 3840), (1, 729 * 3840 + 1), (2, 911 * 3072 - 1), (2, 911 * 3072),
+                                     (2, 911 * 3072 + 1)])
+def test_carried_tiles(words, n, hint):
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, 15_000, n)
+    cols = {"k": (k * (2**48 + 1 if words == 2 else 1), None), "x": (rng.integers(-2**40, 2**40, n), None),
+            "y": (rng.integers(-2**40, 2**40, n), None), "z": (rng.integers(-2**40, 2**40, n), pack(rng.random(n) > 0.1))}
+    keys = ["k"]
+    if words == 2:
+        cols["j"] = ((k % 5 * 2**29).astype(np.int32), None)
+        keys.append("j")
+    aggs = [("Sum", "x", "s"), ("Max", "y", "h"), ("Sum", "z", "t"), ("Count", "z", "c")]
+    got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, keys, aggs, strategy="partitioned", capacity_hint=hint)
+    assert got.strategy == "partitioned"
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, None), len(keys), aggs)
