@@ -1436,11 +1436,18 @@ int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, 
 }
 
 // Many groups and no heavy key: partition the rows by key hash and aggregate every partition in a
-// shared-memory table instead of a global table (or a full sort) that lives in HBM. Measured on
-// 100M uniform rows: 64-bit keys tie with the global table near 250K groups and win 2.3x from 1M
-// groups on; 96-bit keys (the prebuilt 128-bit hash kernel) win 2x from 2M groups and tie at
-// 200K. A heavy key would make its partition one CTA's serial work, so the most frequent sampled
-// key must stand for at most 256K rows.
+// shared-memory table instead of a global table (or a full sort) that lives in HBM. A heavy key would
+// make its partition one CTA's serial work, so the most frequent sampled key must stand for at most 256K
+// rows. Global table against partitions, ms, 100M uniform rows, Float64 values carried (pmb_sort.cu):
+//                                 200K groups    350K           500K           700K           2M
+//   64 key bits, sum and len      2.2 / 4.2      2.8 / 4.2      3.2 / 4.2      12.9 / 4.2     13.2 / 4.2
+//   64 key bits, 7 aggregates     13.7 / 5.6     14.8 / 5.5     15.2 / 5.5     26.1 / 5.5     26.3 / 5.6
+//   more bits, sum and len        3.4 / 6.4      3.8 / 6.4      4.1 / 6.4      13.6 / 6.4     13.9 / 6.5
+//   more bits, 7 aggregates       12.9 / 7.8     13.8 / 7.9     14.1 / 7.8     24.5 / 7.9     25.0 / 8.0
+// (keys that pack into 64 bits by their ranges within 0.4 of those that have 64; 20M rows of more bits, sum
+// and len: 0.9 / 1.5, 1.0 / 1.5, 1.0 / 1.5, 2.6 / 1.5, 2.6 / 1.6.) What decides is whether the table, four slots
+// of key and record a group, stays in L2: small records tie between 500K and 700K groups, seven aggregates below
+// 100K (64 bits) and at 100K (more). The limits, by the key alone, lie inside that span.
 bool pmb_heavy_key(const CompiledQuery& cq, const SketchOut& sk) {
   if (sk.samples <= 0) return false;
   int top = 0;
@@ -1457,8 +1464,10 @@ bool pmb_heavy_key(const CompiledQuery& cq, const SketchOut& sk) {
 // in the sample: over the 13,000 timed tables of the selector's training data, such queries never
 // ran faster than the run-time compiled hash kernel (vetoing them would have cost 22 ms of 1,520 ms
 // there), while a heavy key can make its segment one CTA's serial work (the hash workload: 27.8 ms
-// sorted against 2.0 ms hashed). Wider keys keep the network's pick: their hash path is the slower
-// prebuilt 128-bit kernel, and there the sort and partitioned strategies often win.
+// sorted against 2.0 ms hashed). Wider keys, those that do not pack into 64 bits by their ranges, keep the
+// network's pick: with a heavy key their hash path is the slower prebuilt 128-bit kernel, and there the
+// sort and partitioned strategies often win. (The tables were timed when the partition passes carried no
+// values and no key was packed: more queries are vetoed now than the training data's figures say.)
 bool pmb_selector_vetoed(const CompiledQuery& cq, const SketchOut& sk, int strategy) {
   return (strategy == PMB_STRATEGY_SORT || strategy == PMB_STRATEGY_PARTITIONED) && cq.dq.key_bits <= 64 &&
          pmb_heavy_key(cq, sk);

@@ -90,7 +90,7 @@ bool pmb_selector_vetoed(const CompiledQuery& cq, const SketchOut& sk, int strat
 int pmb_plan_hash(pmb_handle* h, int max_smem_optin, CompiledQuery& cq, int strategy, int64_t est, bool have_sketch,
                   HashParams& P, int& nt, int& smem);
 // est_learned: est is the larger of the sample estimate and the strategy selector's predicted
-// group count (two estimates, so the table is sized tighter: 2 slots per group instead of 4)
+// group count (two estimates, so the table is sized tighter: 3 slots per group instead of 4)
 int pmb_groupby_hash(pmb_handle* h, CompiledQuery& cq, const pmb_query* uq, int strategy, int64_t est,
                      const SketchOut* sk, pmb_result* r, bool est_learned = false);
 // Keys wider than 64 bits at their types' widths: reads the key columns' ranges and, when the values

@@ -186,7 +186,7 @@ struct pmb_handle {
   uint8_t* hstage = nullptr;
   size_t hstage_cap = 0, hstage_used = 0, hstage_want = 0;
   uint8_t* rstage = nullptr;  // pinned staging of small results (pmb_finish_outputs), allocated at first use
-  unsigned int* sort_status = nullptr;  // device status of the call's output sort (pmb_order_finish reads it)
+  unsigned int* sort_status = nullptr;  // device status of the call's output sort (its end reads it)
   pmb_h2d_pool* h2d_pool = nullptr;
   bool h2d_pool_failed = false;
   // profiling

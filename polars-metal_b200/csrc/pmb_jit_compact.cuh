@@ -12,8 +12,9 @@
 // output position that is a multiple of 32, so stores are whole aligned lines and a validity word is
 // one ballot and one plain store (only a tile's first and last word are shared with its neighbours).
 // What bounds it: DRAM and the tile's chain of round trips. With four rows per thread held in
-// registers from the verdict to the scatter: 1288 us for 100M rows of 28 bytes (63% kept), 849 us
-// here, against 695 us for the bytes alone. (Fetching the next tile ahead into a second stage was
+// registers from the verdict to the scatter: 1288 us for 100M rows of 28 bytes (54% kept), 808 us
+// here, against 666 us for the bytes alone at a copy's rate (20M rows under a profiler: DRAM 61% of its peak,
+// reads 1.01 of the columns' bytes, 86% of the warps active, waiting at the tile's barriers). (Fetching the next tile ahead into a second stage was
 // slower, 1.9 ms: a tile taken early publishes its count late, and every later look-back waits.)
 
 #define JC_NT 256

@@ -1099,8 +1099,8 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
       const int smem = L.dict_slots * 6;
       const auto encode = W == 1 ? k_order_encode<1, true> : k_order_encode<2, true>;
       PMB_CUDA(h, cudaFuncSetAttribute(encode, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      const int per_sm = smem <= 96 << 10 ? 2 : 1;
-      encode<<<h->sm_count * per_sm, DICT_NT, smem, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
+      static_assert(DICT_SLOTS * 6 <= 96 << 10, "two CTAs an SM");
+      encode<<<h->sm_count * 2, DICT_NT, smem, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
     } else if (W == 1) {
       k_order_encode<1, false><<<blocks_for(h, n), OR_NT, 0, h->stream>>>(L, n, perm, k0, cap, i0, passes, hist, h->sort_status);
     } else {

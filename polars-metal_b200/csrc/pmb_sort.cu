@@ -431,9 +431,11 @@ __device__ __forceinline__ unsigned long long digit_lookback(unsigned long long*
 // counts are published to the later tiles' look-backs before any ranking, and the counters, once
 // scanned, are the keys' running positions in the tile: a key goes straight to its place in shared
 // memory. The lanes of a round with the same digit find each other through a per-warp table of
-// lane masks (one atomicOr): __match_any_sync and eight ballots per key both cost more issue slots.
-// What bounds it: shared-memory atomics and accesses (about 50 cycles per 32 keys and SM; without
-// any output or look-back the ranking alone takes 60% of the time), not DRAM. 100M 64-bit keys:
+// lane masks (one atomicOr; the way CUB's block radix ranking has as its atomic-or match):
+// __match_any_sync and eight ballots per key both cost more issue slots.
+// What bounds it: shared-memory atomics and accesses (42 shared wavefronts per 32 keys, the LSU data pipe at 67%
+// of its peak over 20M pairs and DRAM at 27%; without any output or look-back the ranking alone takes 60% of
+// the time), then the loads and look-backs that 36 warps an SM wait for. 100M 64-bit keys:
 // 795 us (3.0 TB/s of the 6.4 a plain copy reaches); 256 threads x 16 keys with match_any, ranks
 // held to the end and a look-back of one state per step took 1020 us. 128-bit keys, 20M: 259 us,
 // against 552 us. Prefetching the next tile with bulk copies (persistent CTAs) took 900-960 us.
@@ -1735,7 +1737,6 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
   }
   const auto pass = part_groups > 0 ? k_sort_pass<W, true> : k_sort_pass<W, false>;
   PMB_CUDA(h, cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem));
-  int done = 0;
   if (h->fault_wait) PMB_CUDA(h, cudaMemsetAsync(status, PMB_ST_TIMEOUT, 1, h->stream));
   for (int p = 0; p < passes && m > 1; p++) {
     bool constant = false;
@@ -1792,7 +1793,6 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     PMB_CUDA(h, cudaGetLastError());
     std::swap(k0, k1);
     std::swap(i0, i1);
-    done++;
   }
   if (part_groups > 0) {
     pmb_kernel_begin(h, "part_starts");
@@ -1918,7 +1918,6 @@ int run_sort(pmb_handle* h, CompiledQuery& cq, const SortKeyLayout& L, pmb_resul
     r->columns[c].data = R.out_data[c];
     r->columns[c].validity = R.out_valid[c];
   }
-  (void)done;
   return PMB_OK;
 }
 
