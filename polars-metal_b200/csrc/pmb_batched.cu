@@ -264,6 +264,8 @@ __global__ void __launch_bounds__(FIN_NT) k_batch_finalize(const __grid_constant
       uint64_t bits = 0;
       finalize_agg(q, A, rec, valid, bits);
       store_out(F.out_base + oo[2 * oc], pmb_dtype_bytes(A.out_dtype), p, bits);
+      if (A.out_dtype == PMB_BOOL && valid && bits)
+        atomicOr(reinterpret_cast<unsigned*>(F.out_base + oo[2 * oc]) + (p >> 5), 1u << (p & 31));
       if (valid) atomicOr(&s_vb[oc][r >> 5], 1u << (r & 31));
     }
   }

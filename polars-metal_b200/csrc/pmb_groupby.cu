@@ -784,6 +784,7 @@ __global__ void __launch_bounds__(NT) k_finalize(const __grid_constant__ FinPara
         finalize_agg(q, A, rec, valid, bits);
         store(F.out_data[oc], pmb_dtype_bytes(A.out_dtype), bits);
       }
+      if (A.out_dtype == PMB_BOOL) word(F.out_data[oc], in && valid && bits);
       word(F.out_valid[oc], in && valid);
     }
   }

@@ -742,6 +742,7 @@ __device__ __forceinline__ void write_group(const ReduceParams& R, int64_t p, in
     uint64_t bits = 0;
     if (have) finalize_agg(q, A, rec, valid, bits);
     if (have) store_bits(R.out_data[oc], pmb_dtype_bytes(A.out_dtype), p, bits);
+    if (A.out_dtype == PMB_BOOL) setbit(R.out_data[oc], have && valid && bits);
     setbit(R.out_valid[oc], have && valid);
   }
 }
@@ -1054,6 +1055,8 @@ __global__ void __launch_bounds__(PA_NT, 1) k_part_agg(const __grid_constant__ P
           uint64_t bits = 0;
           finalize_agg(A.q, Ag, rec, valid, bits);
           store_bits(A.out_data[oc], pmb_dtype_bytes(Ag.out_dtype), (int64_t)p, bits);
+          if (Ag.out_dtype == PMB_BOOL && valid && bits)
+            atomicOr(reinterpret_cast<unsigned int*>(A.out_data[oc]) + (p >> 5), 1u << (p & 31));
           if (valid) atomicOr(&vb[oc * nwords + (rbit >> 5)], 1u << (rbit & 31));
         }
       }

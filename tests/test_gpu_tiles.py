@@ -443,3 +443,36 @@ def test_carried_tiles(words, n, hint):
     got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, keys, aggs, strategy="partitioned", capacity_hint=hint)
     assert got.strategy == "partitioned"
     assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, None), len(keys), aggs)
+
+
+# minima and maxima of Bool columns: bits, like the keys', in every strategy's last step, ordered by keys and by
+# the aggregate itself
+@pytest.mark.parametrize("jit", ["0", "1"])
+@pytest.mark.parametrize("sort", [None, {"by": ["k"]}, {"by": ["lo", "k"]}], ids=["plain", "key", "aggregate"])
+@pytest.mark.parametrize("strategy", ["smem_hash", "global_hash", "sort", "partitioned"])
+@pytest.mark.parametrize("n,groups", [(1, 1), (40, 7), (5003, 1000), (60_000, 20_000)])
+def test_bool_extremes(n, groups, strategy, sort, jit, monkeypatch):
+    monkeypatch.setenv("PMB_JIT", jit)
+    rng = np.random.default_rng(n)
+    cols = {"k": (rng.integers(0, groups, n), None, A.I64, n), "b": (pack(rng.random(n) > 0.4), None, A.BOOL, n),
+            "c": (pack(rng.random(n) > 0.6), pack(rng.random(n) > 0.3), A.BOOL, n)}
+    aggs = [("Min", "b", "lo"), ("Max", "b", "hi"), ("Min", "c", "c_lo"), ("Max", "c", "c_hi"), ("Sum", "c", "s"), ("Len", None, "n")]
+    got = as_dict(N.groupby({c: N.ColumnData(d, v, dtype=t, length=m) for c, (d, v, t, m) in cols.items()}, ["k"], aggs,
+                            strategy=strategy, sort=sort))
+    want = pyoracle.groupby(cols, ["k"], aggs, None)
+    assert_results_match(got, want, 1, aggs, strategy)
+    if sort:
+        assert_same_rows(got, pyoracle.sort_table(_table(want), sort["by"], [False] * len(sort["by"]), [False] * len(sort["by"])), strategy)
+
+
+def test_bool_extremes_in_a_batch():
+    rng = np.random.default_rng(1)
+    queries, wants = [], []
+    aggs = [("Min", "b", "lo"), ("Max", "b", "hi"), ("Max", "c", "c_hi"), ("Len", None, "n")]
+    for n in (1, 33, 2000, 70_000, 3, 9000):
+        cols = {"k": (rng.integers(0, max(1, n // 4), n), None, A.I64, n), "b": (pack(rng.random(n) > 0.4), None, A.BOOL, n),
+                "c": (pack(rng.random(n) > 0.6), pack(rng.random(n) > 0.3), A.BOOL, n)}
+        queries.append(({c: N.ColumnData(d, v, dtype=t, length=m) for c, (d, v, t, m) in cols.items()}, ["k"], aggs, None))
+        wants.append(pyoracle.groupby(cols, ["k"], aggs, None))
+    for got, want in zip(N.groupby_batched(queries), wants):
+        assert_results_match(as_dict(got), want, 1, aggs)
