@@ -657,6 +657,8 @@ extern "C" int pmb_groupby_batched(pmb_handle* h, const pmb_query* qs, const pmb
     rc = pmb_ws_begin(h);
     if (rc) return fail_all(rc);
     pmb_call_begin(h);
+    for (int i : batch)
+      for (int c = 0; c < cqs[i].dq.n_cols; c++) pmb_expect_column(h, cols[i][cqs[i].map.user[c]], cqs[i].dq.n_rows);
     for (int i : batch) {
       outs[i] = pmb_result_new(cqs[i].dq.n_keys + cqs[i].dq.n_aggs);
       if (!outs[i]) return fail_all(pmb_fail(h, PMB_E_OOM, "host allocation failed"));

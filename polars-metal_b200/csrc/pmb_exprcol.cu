@@ -550,6 +550,7 @@ extern "C" int pmb_eval_expr(pmb_handle* h, const pmb_expr* expr, const pmb_colu
   if (rc) return rc;
   pmb_call_begin(h);
   P.n_cols = (int)F.user_of.size();
+  for (int s = 0; s < P.n_cols; s++) pmb_expect_column(h, cols[F.user_of[s]], n);
   for (int s = 0; s < P.n_cols; s++) {
     DCol d;
     memset(&d, 0, sizeof(d));

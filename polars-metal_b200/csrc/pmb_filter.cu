@@ -439,6 +439,7 @@ int pmb_compare(pmb_handle* h, const pmb_column* lhs, const pmb_column* rhs, int
   const int64_t n = lhs->length;
   cq.dq.n_cols = (int)cq.map.user.size();
   cq.dq.n_rows = n;
+  for (int c = 0; c < cq.dq.n_cols; c++) pmb_expect_column(h, cols[cq.map.user[c]], n);
   for (int c = 0; c < cq.dq.n_cols; c++) {
     rc = pmb_stage_column(h, cols[cq.map.user[c]], n, &cq.dq.col[c]);
     if (rc) return rc;
@@ -541,6 +542,7 @@ static int compact_common(pmb_handle* h, const pmb_expr* pred, const uint8_t* pd
   rc = pmb_ws_begin(h);
   if (rc) return rc;
   pmb_call_begin(h);
+  for (int c = 0; c < cq.dq.n_cols; c++) pmb_expect_column(h, cols[cq.map.user[c]], n_rows);
   for (int c = 0; c < cq.dq.n_cols; c++) {
     rc = pmb_stage_column(h, cols[cq.map.user[c]], n_rows, &cq.dq.col[c]);
     if (rc) return rc;

@@ -1352,6 +1352,7 @@ int pmb_groupby_call(pmb_handle* h, const pmb_query* q, const pmb_column* cols, 
     return code;
   };
   // stage the touched columns
+  for (int c = 0; c < cq.dq.n_cols; c++) pmb_expect_column(h, cols[cq.map.user[c]], cq.dq.n_rows);
   for (int c = 0; c < cq.dq.n_cols; c++) {
     rc = pmb_stage_column(h, cols[cq.map.user[c]], cq.dq.n_rows, &cq.dq.col[c]);
     if (rc) return bail(rc);

@@ -188,6 +188,7 @@ struct pmb_handle {
   uint8_t* rstage = nullptr;  // pinned staging of small results (pmb_finish_outputs), allocated at first use
   unsigned int* sort_status = nullptr;  // device status of the call's output sort (its end reads it)
   pmb_h2d_pool* h2d_pool = nullptr;
+  size_t host_bytes = 0;  // of the call's host columns that the pool would take (pmb_expect_column)
   bool h2d_pool_failed = false;
   // profiling
   bool profiling = false;
@@ -256,6 +257,8 @@ pmb_result* pmb_result_new(int32_t n_columns);
 // column staging (pmb_runtime.cu): makes a device view of a column, copying host data in
 // and realigning device data whose offset breaks 16-byte alignment.
 int pmb_stage_column(pmb_handle* h, const pmb_column& c, int64_t n_rows, DCol* out);
+// a column that the call is going to stage: how much the host columns come to decides how they are copied
+void pmb_expect_column(pmb_handle* h, const pmb_column& c, int64_t n_rows);
 // *own: a device output pointer is memory of the handle's GPU, which kernels may store to (pinned host memory
 // and other GPUs' are copied to); PMB_E_INVALID when it is neither
 int pmb_check_output(pmb_handle* h, const void* p, bool* own);

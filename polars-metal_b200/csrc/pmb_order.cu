@@ -1201,6 +1201,7 @@ extern "C" int pmb_sort_columns(pmb_handle* h, const pmb_column* cols, int32_t n
   pmb_call_begin(h);
   DCol d[PMB_MAX_COLS];
   memset(d, 0, sizeof(d));
+  for (int c = 0; c < n_cols; c++) pmb_expect_column(h, cols[c], n);
   for (int c = 0; c < n_cols; c++) {
     rc = pmb_stage_column(h, cols[c], n, &d[c]);
     if (rc) return rc;

@@ -247,3 +247,21 @@ def test_workspace_without_order_keys(monkeypatch):
     how = [run(w * MB) for w in range(600, 99, -4)]
     assert how[0] == run(0) == "ordered" and how[-1] is None
     assert "columns" in how and how == sorted(how, key=["ordered", "columns", None].index)
+
+
+# pageable columns around what the staging threads take (columns of 4 MB, calls of 20 MB of them) and their chunks: one
+# column or several, sizes that no chunk divides, the values and their places right
+@pytest.mark.parametrize("cols,n", [(1, 524_287), (1, 524_288), (1, 2_621_439), (1, 2_621_440), (1, 2_621_441), (1, 5_000_011),
+                                    (3, 524_288), (3, 873_813), (3, 873_815), (5, 524_287), (5, 524_288), (2, 4_194_305)])
+def test_staged_column_sizes(cols, n):
+    rng = np.random.default_rng(n)
+    data = {f"c{i}": rng.integers(-2**62, 2**62, n) for i in range(cols)}
+    data["c0"][0] = -2**62  # the one row that goes
+    for _ in range(2):
+        got = N.filter_columns(data, {"kind": "Compare", "op": "Gt", "lhs": {"kind": "Column", "name": "c0"},
+                                      "rhs": {"kind": "LiteralI64", "value": -2**62}})
+        keep = data["c0"] > -2**62
+        m = int(keep.sum())
+        assert got.n_groups == m
+        for have, d in zip(got.data, data.values()):
+            assert np.array_equal(have[:m], d[keep])
