@@ -669,9 +669,8 @@ __global__ void __launch_bounds__(OR_NT) k_order_gather(const __grid_constant__ 
 
 // ---------------------------------------------------------------- small tables in one launch
 // Up to SMALL_ROWS rows whose sort columns fit 128 key bits at their full widths: one CTA packs the
-// keys, sorts them in shared memory and gathers the slice, in one launch without a read-back. The
-// general path's launches (ranges, null flags, encode, a pass per digit, gather) and its two
-// read-backs cost 340 us of a 1000-group call whatever the size.
+// keys, sorts them in shared memory and gathers the slice, in one launch without a read-back, where that is less
+// than the general path's launches (ranges, encode, a pass per digit, gather) and its read-back (small_pays).
 constexpr int SMALL_ROWS = 8192;
 constexpr int SMALL_NT = 1024;
 
@@ -862,6 +861,23 @@ double sampled_distinct(const OrderRange& g, int k) {
   return f1 == 0 ? g.distinct[k] : g.distinct[k] + f1 * f1 / (2 * std::max(f2, 0.5));
 }
 
+// Whether k_order_small beats the general path, whose time goes by its passes. Measured for sort_columns of three
+// columns, us: k_order_small of one- / two-word keys 38 / 51 up to 1024 rows, 50 / 78 to 2048, 80 / 140 to 4096,
+// 146 / 280 to 8192, whatever the values; the general path 44 where all rows have one key, 73 with one pass, 85 with
+// two, 106 with four, 146 with eight, 165 with nine of two-word keys. The passes follow from the values'
+// ranges, which only the general path reads: floats are taken to fill their types, integers 16 bits of them.
+bool small_pays(const DCol* cols, const pmb_sort_spec& s, int64_t n, int full_bits) {
+  if (n <= 1 || n > SMALL_ROWS || full_bits > 128) return false;
+  static constexpr int us[4][2] = {{38, 51}, {50, 78}, {80, 140}, {146, 280}};
+  int size = 0, bits = 0;
+  while ((1024 << size) < n) size++;
+  for (int k = 0; k < s.n_by; k++) {
+    const DCol& d = cols[s.by[k]];
+    bits += (pmb_is_float(d.dtype) ? pmb_dtype_bits(d.dtype) : std::min(pmb_dtype_bits(d.dtype), 16)) + (d.valid != nullptr);
+  }
+  return us[size][full_bits > 64] <= 62 + 11 * ((bits + 7) / 8);
+}
+
 // pmb_order_columns for a table that k_order_small takes
 int order_small(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, const pmb_sort_spec& s, const int* desc,
                 const int* nlast, pmb_result* r) {
@@ -961,7 +977,7 @@ int pmb_order_columns(pmb_handle* h, const DCol* cols, int n_cols, int64_t n, co
     const DCol& d = cols[s.by[k]];
     full_bits += pmb_dtype_bits(d.dtype) + (d.valid != nullptr);
   }
-  if (n > 1 && n <= SMALL_ROWS && full_bits <= 128) return order_small(h, cols, n_cols, n, s, desc, nlast, r);
+  if (small_pays(cols, s, n, full_bits)) return order_small(h, cols, n_cols, n, s, desc, nlast, r);
   // ranges and null counts of the sort columns
   SortCols C;
   memset(&C, 0, sizeof(C));

@@ -476,3 +476,22 @@ def test_bool_extremes_in_a_batch():
         wants.append(pyoracle.groupby(cols, ["k"], aggs, None))
     for got, want in zip(N.groupby_batched(queries), wants):
         assert_results_match(as_dict(got), want, 1, aggs)
+
+
+# which sorts go in one launch: up to 2048 rows all, up to 4096 those of one-word keys with two digits and more, up to
+# 8192 those of a float of 64 bits alone (the passes of the others take less); the orders are right on both sides
+@pytest.mark.parametrize("n", [2, 1024, 1025, 2048, 2049, 4096, 4097, 8192, 8193])
+@pytest.mark.parametrize("case", [("int8", False, 2048), ("int16", False, 4096), ("int64", False, 4096), ("int64", True, 2048),
+                                  ("float32", False, 4096), ("float64", False, 8192), ("float64", True, 4096)],
+                         ids=lambda c: f"{c[0]}{'-null' * c[1]}")
+def test_small_sort_rule(case, n):
+    kind, nulls, largest = case
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal(n).astype(kind) if kind[0] == "f" else rng.integers(-100, 100, n).astype(kind)
+    cols = {"a": (a, pack(rng.random(n) > 0.2) if nulls else None), "row": (np.arange(n), None)}
+    h = N.Handle(0)
+    h.set_profiling(True)
+    got = N.sort_columns({k: N.ColumnData(d, v) for k, (d, v) in cols.items()}, ["a"], [True], handle=h)
+    assert ("order_small" in h.last_stats()["kernels"]) == (n <= largest)
+    assert_same_rows(as_dict(got), pyoracle.sort_table(cols, ["a"], [True], [False]), f"{n} rows of {kind}")
+    h.close()
