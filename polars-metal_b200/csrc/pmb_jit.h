@@ -91,6 +91,7 @@ struct JPartH {
   long long n_items;
   int slots;
   int run;
+  unsigned probes;
   unsigned long long* ticket;
   unsigned long long* gkeys;
   unsigned char* grecs;

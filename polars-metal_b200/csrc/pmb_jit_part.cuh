@@ -29,6 +29,7 @@ struct JPart {
   long long n_items;
   int slots;                          // table slots
   int run;                            // partitions per work item
+  unsigned probes;                    // slots that a row tries before its item counts as one of too many groups
   unsigned long long* ticket;
   unsigned long long* gkeys;          // dense groups: packed keys, word-major (stride gcap)
   unsigned char* grecs;               // and their records, J_REC bytes each
@@ -45,6 +46,7 @@ struct JPart {
 // two rows and the ticket taken between the items, 6.46 ms with three and the next ticket early, 5.95 ms
 // as two CTAs of 512 threads and two rows, 5.47 ms so; 12M rows in 3.8M groups 652, 596, 535 and 496 us.
 #define JP_R (JP_CTAS == 2 ? 1 : 3)
+
 
 __device__ __forceinline__ unsigned long long jp_hash(const unsigned long long* k) {
   unsigned long long h = pmb_fmix64(k[0]);
@@ -143,7 +145,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, JP_CTAS) pmb_jit_part_agg(con
             break;
           }
           slot[r] = sl + 1 == (unsigned)S ? 0u : sl + 1;
-          if (++probes[r] >= (unsigned)S) {
+          if (++probes[r] >= A.probes) {
             atomicOr(P.status, PMB_ST_OVERFLOW);  // the item has more groups than the table
             pending[r] = false;
           }
@@ -181,7 +183,7 @@ extern "C" __global__ void __launch_bounds__(J_NT, JP_CTAS) pmb_jit_part_agg(con
               break;
             }
             slot[r] = sl + 1 == (unsigned)S ? 0u : sl + 1;
-            if (++probes[r] >= (unsigned)S) {
+            if (++probes[r] >= A.probes) {
               atomicOr(P.status, PMB_ST_OVERFLOW);  // the item has more groups than the table
               pending[r] = false;
             }

@@ -495,3 +495,28 @@ def test_small_sort_rule(case, n):
     assert ("order_small" in h.last_stats()["kernels"]) == (n <= largest)
     assert_same_rows(as_dict(got), pyoracle.sort_table(cols, ["a"], [True], [False]), f"{n} rows of {kind}")
     h.close()
+
+
+# partitions with more groups than their table: the attempt ends at its first rows that find no slot, whatever
+# the number of rows, and the sort strategy gives the result; one-word keys of fewer and of all 64 bits, two words
+@pytest.mark.parametrize("kind", ["one word", "64 bits", "two words"])
+def test_overflowing_partitions(kind):
+    rng = np.random.default_rng(6)
+    n = 1_500_000
+    k = rng.permutation(n)
+    cols = {"k": (k * 8191, None), "v": (rng.integers(0, 1000, n).astype(np.int32), None)}
+    if kind == "64 bits":
+        cols["k"] = (rng.integers(-2**63, 2**63 - 1, n), None)
+    keys = ["k"]
+    if kind == "two words":
+        cols["k"] = (rng.integers(-2**63, 2**63 - 1, n), None)
+        cols["j"] = ((k % 3).astype(np.int16), None)
+        keys.append("j")
+    aggs = [("Sum", "v", "s"), ("Max", "v", "m"), ("Len", None, "c")]
+    h = N.Handle(0)
+    h.set_profiling(True)
+    data = {c: N.ColumnData(*d) for c, d in cols.items()}
+    got = N.groupby(data, keys, aggs, strategy="partitioned", capacity_hint=5000, handle=h)
+    assert got.strategy == "sort"
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, None), len(keys), aggs)
+    h.close()
