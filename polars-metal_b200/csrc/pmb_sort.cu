@@ -2030,9 +2030,14 @@ bool pmb_apply_packed_keys(CompiledQuery& cq) {
 // A nullable Int64 key is 65 bits wide by its type, two key columns 96 or more; their values mostly
 // need far fewer. Packed into 64 bits they take the run-time compiled hash kernel, its sampled-key
 // tables and the CTA-shared tier instead of the prebuilt 128-bit kernel, which has none of them
-// (10M rows, nullable Int64 keys, 200K groups: 2524 us there).
+// (10M rows, nullable Int64 keys, 200K groups: 2524 us there). Below the run-time kernel's 2M rows the 64-bit
+// prebuilt kernels have the sampled-key tables, which pay for the ranges (a pass and a wait, 20 to 60 us) where some
+// key is frequent. Packed / not, us, one key, Zipf(1.0) and a quarter of the rows' number of groups: 20K rows 219 / 141,
+// 193 / 126, 136 / 108; 60K 226 / 217, 201 / 167, 141 / 116; 200K 244 / 501, 217 / 317, 167 / 139; 1.9M 777 / 3971,
+// 608 / 2080, 421 / 424. Hence PACK_ROWS.
+constexpr int64_t PACK_ROWS = 100000;
 int pmb_pack_wide_keys(pmb_handle* h, CompiledQuery& cq) {
-  if (cq.dq.key_bits <= 64 || cq.dq.n_rows == 0) return PMB_OK;
+  if (cq.dq.key_bits <= 64 || (cq.dq.n_rows < PACK_ROWS && !pmb_jit_enabled(cq.dq.n_rows)) || cq.dq.n_rows == 0) return PMB_OK;
   SortKeyLayout L;
   key_columns(cq.dq, L);
   const int rc = read_key_ranges(h, cq, L);

@@ -520,3 +520,21 @@ def test_overflowing_partitions(kind):
     assert got.strategy == "sort"
     assert_results_match(as_dict(got), pyoracle.groupby(cols, keys, aggs, None), len(keys), aggs)
     h.close()
+
+
+# wide keys are packed from 100,000 rows on (their ranges are read), and where kernels are compiled at every size;
+# on both sides one key, few and many, nulls among them
+@pytest.mark.parametrize("jit", [None, "1"])
+@pytest.mark.parametrize("groups", [1, 50, 20_000])
+@pytest.mark.parametrize("n", [1, 500, 99_999, 100_000])
+def test_packing_rule(n, groups, jit, monkeypatch):
+    monkeypatch.setenv("PMB_JIT", jit) if jit else monkeypatch.delenv("PMB_JIT", raising=False)
+    rng = np.random.default_rng(n + groups)
+    cols = {"k": (rng.integers(0, groups, n) * 4099 - 7, pack(rng.random(n) > 0.1)), "v": (rng.standard_normal(n), None)}
+    aggs = [("Sum", "v", "s"), ("Min", "v", "l"), ("Len", None, "c")]
+    h = N.Handle(0)
+    h.set_profiling(True)
+    got = N.groupby({c: N.ColumnData(*d) for c, d in cols.items()}, ["k"], aggs, strategy="global_hash", handle=h)
+    assert ("key_range" in h.last_stats()["kernels"]) == (n >= 100_000 or jit == "1")
+    assert_results_match(as_dict(got), pyoracle.groupby(cols, ["k"], aggs, None), 1, aggs)
+    h.close()
