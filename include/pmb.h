@@ -256,7 +256,7 @@ const char* pmb_last_error(const pmb_handle* h);
 int pmb_set_stream(pmb_handle* h, void* cuda_stream);
 /* The handle's later launches come after the work that is on `cuda_stream` (of the same GPU; NULL = the
  * legacy default stream) at the time of this call: for device buffers that it still fills or reads. The
- * host does not wait. */
+ * host does not wait. Work that a stream is capturing is not waited for. */
 int pmb_wait_for_stream(pmb_handle* h, void* cuda_stream);
 /* 1 = record per-kernel CUDA-event timings of every call (readable with pmb_last_stats). */
 int pmb_set_profiling(pmb_handle* h, int32_t enabled);

@@ -812,6 +812,13 @@ int pmb_wait_for_stream(pmb_handle* h, void* stream) {
   if (!h) return PMB_E_INVALID;
   if ((cudaStream_t)stream == h->stream) return PMB_OK;
   PMB_CUDA(h, cudaSetDevice(h->device));
+  // a stream that is being captured runs nothing yet, and waiting for it would draw this call into the capture
+  cudaStreamCaptureStatus capturing;
+  if (cudaStreamIsCapturing((cudaStream_t)stream, &capturing) != cudaSuccess) {
+    cudaGetLastError();
+    return PMB_OK;
+  }
+  if (capturing != cudaStreamCaptureStatusNone) return PMB_OK;
   if (!h->other_stream) PMB_CUDA(h, cudaEventCreateWithFlags(&h->other_stream, cudaEventDisableTiming));
   PMB_CUDA(h, cudaEventRecord(h->other_stream, (cudaStream_t)stream));
   PMB_CUDA(h, cudaStreamWaitEvent(h->stream, h->other_stream, 0));

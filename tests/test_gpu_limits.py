@@ -265,3 +265,23 @@ def test_staged_column_sizes(cols, n):
         assert got.n_groups == m
         for have, d in zip(got.data, data.values()):
             assert np.array_equal(have[:m], d[keep])
+
+
+# a stream that torch is capturing into a graph (relaxed, so that other streams may run): the expression is evaluated
+# at once, on the library's stream, and neither joins the capture nor ends it
+def test_expression_beside_a_capture():
+    import torch
+
+    x = torch.arange(1000, dtype=torch.int64, device="cuda")
+    e = {"kind": "Arith", "op": "Add", "lhs": {"kind": "Column", "name": "x"}, "rhs": {"kind": "Column", "name": "x"}}
+    N.eval_expr({"x": N.ColumnData(x)}, e)  # (a capture allocates from a pool of its own, the library not at all)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="relaxed"):
+        y = x + 1
+        got = N.eval_expr({"x": N.ColumnData(x)}, e)
+    for _ in range(2):
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, x + 1) and torch.equal(got.data[:1000], 2 * x)
+        assert np.unpackbits(got.validity.cpu().numpy(), bitorder="little")[:1000].all()
