@@ -256,7 +256,7 @@ static int launch_shift(pmb_handle* h, const uint8_t* in, uint8_t* out, int64_t 
 // driver's own staging of a pageable copy is one thread's memcpy (4.0 ms for 61 MB, 2.1 ms so;
 // the link alone 1.1 ms). Every thread owns two chunks: it fills one while the other's copy is in
 // flight, and queues its copies on the handle's stream itself (their destinations are disjoint).
-// The threads are started with the handle's first large pageable copy and end with the handle.
+// The threads are started with the first copy that they take and end with the handle.
 struct pmb_h2d_pool {
   static constexpr size_t CHUNK = (size_t)1 << 20;
   int n_threads = 0;  // the caller's among them
